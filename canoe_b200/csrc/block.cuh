@@ -45,6 +45,9 @@ struct Geom {
   // (the six panels of a cubed-sphere shell share one geometry)
   int npanel = 1;
   int64_t pstride = 0;
+  // scratch of the column march (march.cuh), march_doubles() long; null: the
+  // fused x1 stage runs one CTA per column (column.cuh)
+  double *march = nullptr;
 };
 
 // geometry tables of a cubed-sphere panel (gnomonic_equiangle.cpp:140-222)
@@ -90,6 +93,9 @@ int launch_x1col(const Geom &g, const canoe_thermo_t &th, int recon, int rs,
                  int implicit_flag, int precision, int mode, const double *w, double *du, double *u,
                  double *u1, const double *dtp, const Stage &s, int stage,
                  double *flx_out, cudaStream_t st);
+// scratch of the column march of a block's fused x1 stage (march.cuh) in
+// doubles; 0 when the block keeps the CTA-per-column kernel
+size_t march_doubles(const Geom &g, const canoe_thermo_t &th, int implicit_flag, int precision);
 // implicit solves along x2 (dir 1) and x3 (dir 2) of a dry block (lines.cu):
 // whether the flag asks for one in a direction the block has, the doubles
 // of each of the two line-major scratch arrays, and the solve of du in place

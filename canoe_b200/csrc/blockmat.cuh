@@ -189,8 +189,8 @@ __device__ __forceinline__ constexpr int sel(int r) {
 // FluxJacobian (flux_decomposition.hpp:102-120), reduced to N x N, evaluated
 // in T (double; float for the FP32 flux path, whose implicit blocks are
 // formed from FP32 coefficients and eliminated in FP64)
-template <int N, int NY, typename T = double>
-__device__ __forceinline__ void jacobian(M<N> &d, double gm1_, const double *w) {
+template <int N, int NY, typename T = double, typename W = double>
+__device__ __forceinline__ void jacobian(M<N> &d, double gm1_, const W *w) {
   using S = Slots<NY>;
   const T gm1 = T(gm1_);
   T v1 = T(w[S::IVX]), v2 = T(w[S::IVY]), v3 = T(w[S::IVZ]);
@@ -212,10 +212,9 @@ __device__ __forceinline__ void jacobian(M<N> &d, double gm1_, const double *w) 
 // |A| = R |Lambda| R^-1 at the face between cells with primitive states wl,
 // wr: RoeAverage (:34-67), SoundSpeed, Eigenvalue (:70-75), Eigenvector
 // (:78-99); only the N x N reduced block is formed, in T as jacobian.
-template <int N, int NY, typename T = double>
-__device__ __forceinline__ void abs_jacobian(M<N> &A, const canoe_thermo_t &th,
-                                             double gm1_, const double *wl_,
-                                             const double *wr_) {
+template <int N, int NY, typename T = double, typename W = double, class TH>
+__device__ __forceinline__ void abs_jacobian(M<N> &A, const TH &th,
+                                             double gm1_, const W *wl_, const W *wr_) {
   using S = Slots<NY>;
   const T gm1 = T(gm1_);
   T wl[S::NV], wr[S::NV], prim[S::NV];

@@ -141,6 +141,7 @@ struct canoe_block {
   // x2 / x3 implicit solves: line-major scratch of w and du, line spacings
   // (nx2 + 2 NG entries of dx2, then nx3 + 2 NG of dx3)
   double *d_wt = nullptr, *d_dut = nullptr, *d_dxl = nullptr;
+  double *d_march = nullptr;  // scratch of the column march (Geom::march)
   bool lines = false;
   cudaStream_t st = nullptr;
   bool own_stream = false;
@@ -236,7 +237,7 @@ static int block_free(canoe_block *b) {
                   (void *)b->d_x1f, (void *)b->d_x1v, (void *)b->d_dx1f,
                   (void *)b->d_scr, (void *)b->d_dt, (void *)b->d_pref, (void *)b->d_dtacc,
                   (void *)b->d_err, (void *)b->d_sat, (void *)b->d_wt, (void *)b->d_dut,
-                  (void *)b->d_dxl})
+                  (void *)b->d_dxl, (void *)b->d_march})
     if (p) cudaFree(p);
   if (b->own_stream && b->st) cudaStreamDestroy(b->st);
   delete b;
@@ -485,6 +486,14 @@ int canoe_block_create(const canoe_block_config_t *cfg, canoe_block_t *out) {
     if ((e = cudaMemcpy(b->d_dxl, dl.data(), dl.size() * sizeof(double), cudaMemcpyHostToDevice)))
       return fail(e, "copy");
   }
+  // without memory for the march's scratch the block keeps the kernel that
+  // needs none
+  if (const size_t nm = march_doubles(g, b->th, cfg->implicit_flag, cfg->precision))
+    if (cudaMalloc(&b->d_march, nm * sizeof(double))) {
+      b->d_march = nullptr;
+      cudaGetLastError();
+    }
+  g.march = b->d_march;
   if ((e = cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking))) return fail(e, "stream");
   b->own_stream = true;
   g.x1f = b->d_x1f;

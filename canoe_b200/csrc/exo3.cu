@@ -881,6 +881,7 @@ struct canoe_shell {
   canoe_thermo_t th;
   Geom g;
   int64_t pvals = 0;  // values per panel
+  double *d_march = nullptr;  // scratch of the column march (Geom::march)
   double *d_u = nullptr, *d_w = nullptr, *d_u1 = nullptr, *d_du = nullptr;
   double *d_x1f = nullptr, *d_x1v = nullptr, *d_dx1f = nullptr, *d_dt = nullptr;
   double *d_tabs = nullptr, *d_lr = nullptr, *d_pref = nullptr;
@@ -895,7 +896,7 @@ struct canoe_shell {
 
 static int shell_free(canoe_shell *s) {
   if (!s) return 0;
-  for (void *p : {(void *)s->d_u, (void *)s->d_w, (void *)s->d_u1, (void *)s->d_du,
+  for (void *p : {(void *)s->d_u, (void *)s->d_w, (void *)s->d_u1, (void *)s->d_du, (void *)s->d_march,
                   (void *)s->d_x1f, (void *)s->d_x1v, (void *)s->d_dx1f, (void *)s->d_dt,
                   (void *)s->d_tabs, (void *)s->d_lr, (void *)s->d_pref, (void *)s->d_dtacc,
                   (void *)s->d_err,
@@ -1088,6 +1089,16 @@ int canoe_shell_create(const canoe_shell_config_t *cfg, canoe_shell_t *out) {
              {s->d_edge, er.data(), er.size() * sizeof(EdgeRow)}};
   for (auto &c : cps)
     if ((e = cudaMemcpy(c.d, c.h, c.n, cudaMemcpyHostToDevice))) return fail(e, "copy tables");
+  {  // scratch of the column march, all panels in one launch; optional
+    Geom g6 = g;
+    g6.npanel = 6;
+    if (const size_t nm = march_doubles(g6, s->th, cfg->implicit_flag, cfg->precision))
+      if (cudaMalloc(&s->d_march, nm * sizeof(double))) {
+        s->d_march = nullptr;
+        cudaGetLastError();
+      }
+    g.march = s->d_march;
+  }
   if ((e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking))) return fail(e, "stream");
   s->own_stream = true;
   g.x1f = s->d_x1f;

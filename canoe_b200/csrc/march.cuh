@@ -1,0 +1,1010 @@
+// march.cuh -- the fused x1 stage of a block of many columns: a CTA takes a
+// tile of 32 neighbouring columns, a lane per column, and marches from the top
+// level to the bottom in chunks of C levels, then back up.
+//
+// The CTA-per-column kernel (column.cuh) pays for parallelism inside a column:
+// cyclic and parallel cyclic reduction instead of one elimination, a serial
+// hydrostatic scan on one lane, phases that leave most lanes of the CTA idle.
+// With thousands of columns the columns themselves are the parallelism, and
+// the block elimination runs serially in a lane:
+//   warps 0 .. C-1 share the levels of a chunk, in four phases:
+//     1. the hydrostatic scan down to a level and its decomposition
+//     2. reconstruction, two levels up: four cells of one variable at a time,
+//        so that every limited slope and interface value is computed once
+//     3. the Riemann problem at a face, three levels up
+//     4. four levels up: flux divergence and sources added to du, |A| at the
+//        cell's lower face and the Jacobian of the cell below
+//     (column.cuh P1-P5a, the same expressions)
+//   warps C and C + 1 eliminate the rows of the previous chunk downwards
+//     (forward_backward.hpp:15-91 with the sweep reversed), a row each in
+//     turn, so that one forms its row while the other finishes the row above:
+//     with the rows
+//     scaled by twice the cell's volume over its lower face area,
+//     b' = A_i + J_{i-1} = -b, c' = A_{i+1} - J_{i+1} = -c,
+//     D_i = a_i - c'_i H_{i+1}, H_i = D_i^-1 b'_i,
+//     g_i = D_i^-1 (r_i + c'_i g_{i+1}).
+// H, g and what the update needs of du go to a scratch array laid out
+// [tile][level][component][lane]; on the way up x_i = g_i + H_i x_{i-1}, then
+// the species correction and the register update (forward_backward.hpp:93-137,
+// implicit_hydro_tasks.cpp:152-160, 283).
+//
+// Rows of the block arrays run along x1, so the columns of a tile are strided
+// in memory.  TMA moves them: a box of C levels x 32 columns x NV variables
+// per request (a probe of the access pattern on w of 128x256x256: 5.9 TB/s,
+// 3.0 TB/s with cp.async, 4.5 TB/s with loads and shared-memory stores).  A
+// tensor map needs rows of a multiple of 16 bytes, so columns of an odd
+// number of levels go through registers instead (g.bulk = 0).
+//
+// Measured against the CTA-per-column kernel (one launch, 128x256x256 moist,
+// PPM + HLLC): FP32 fluxes 2.52 -> 1.27 ms, FP64 3.05 -> 2.01 ms.  What bounds
+// it: a chunk is a chain of four barrier-separated phases of dependent FP64
+// and FP32 arithmetic (about 10k cycles for eight levels) that two CTAs per SM
+// (shared memory) overlap; its traffic is the algorithmic bytes and 2 x 136 B
+// per cell of scratch.
+#pragma once
+
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
+#include <type_traits>
+
+#include "column.cuh"
+
+namespace cb {
+
+constexpr int kMarchCols = 32;  // columns per CTA
+constexpr int kMarchUp = 4;     // levels per chunk of the way back up
+// Fewest columns that march.  A tile takes the same time alone on an SM as
+// beside another, so up to 148 tiles (4736 columns) the march takes as long as
+// for one: 128 levels 135 us in FP32, 250 us in FP64, where the CTA-per-column
+// kernel takes 38 and 46 ns a column.
+constexpr int kMarchMinCols32 = 3800, kMarchMinCols64 = 6000;
+
+// scratch per level of a tile: H and g (12 components, a tile's levels
+// contiguous); then du of the species, of the two transverse momenta, and
+// (with species) the sum of the density increments, and the RK register u1
+constexpr int kMarchH = 12;
+__host__ __device__ constexpr int march_nd(int ny) { return 2 + ny + (ny > 0 ? 1 : 0); }
+__host__ __device__ constexpr int march_comp(int ny) { return march_nd(ny) + 5 + ny; }
+
+// tiles of bj x bk = 32 columns that cover nx2 x nx3 with the fewest tiles
+struct MarchTile {
+  int bj, bk, nj, nk;
+};
+inline MarchTile march_tile(int nx2, int nx3) {
+  MarchTile best{0, 0, 0, 0};
+  for (int bj = 32; bj >= 1; bj /= 2) {
+    const int bk = kMarchCols / bj;
+    const MarchTile t{bj, bk, (nx2 + bj - 1) / bj, (nx3 + bk - 1) / bk};
+    if (!best.bj || (int64_t)t.nj * t.nk < (int64_t)best.nj * best.nk) best = t;
+  }
+  return best;
+}
+
+inline size_t march_scratch_doubles(int ny, int nx1, int nx2, int nx3, int npanel) {
+  const MarchTile t = march_tile(nx2, nx3);
+  return (size_t)t.nj * t.nk * npanel * nx1 * (kMarchH + march_comp(ny)) * kMarchCols;
+}
+
+// Shared memory of a tile, in doubles.  Levels are counted from the top (t = 0
+// is the highest ghost cell).  w and du hold the chunk in hand; rings of a
+// chunk and four levels hold the decomposed state q, the FP64 values that
+// later phases need beside it (raw), and the face states wL, overwritten by
+// the fluxes.
+template <int NV, int C, typename R, int GEO>
+struct MarchSmem {
+  static constexpr int RQ = C + 4, RP = 16, NC = kMarchCols, ny = NV - 5;
+  // rows in the ring of |A|, J and the right-hand side: a chunk's, and the two
+  // that the elimination still works on while the next chunk's are formed with
+  // the two above them
+  static constexpr int RR = C + 4, NRH = GEO ? 5 : 4;
+  // raw: rho, p and, where q is rounded to FP32, v1 (GEO: all velocities)
+  static constexpr int NR = sizeof(R) == 8 ? 2 : (GEO ? 5 : 3);
+  static constexpr int rsz(int n) { return (n * (int)sizeof(R) + 7) / 8; }
+  static constexpr int w = 0;                        // [NV][32][C], swizzled;
+  static constexpr int wr = w;                       // in phases 2, 3: wR, [C][NV][32] R
+  static constexpr int d = w + C * NV * NC;          // [NV][32][C], swizzled
+  static constexpr int q = d + C * NV * NC;          // [RQ][NV][32] R
+  static constexpr int raw = q + rsz(RQ * NV * NC);  // [RQ][NR][32]
+  static constexpr int f = raw + RQ * NR * NC;       // [RQ][NV][32] R: wL, then F
+  static constexpr int ps = f + rsz(RQ * NV * NC);   // [RP][32] face pressure
+  static constexpr int gm = ps + RP * NC;            // [RQ][32] RovRd
+  static constexpr int r = gm + RQ * NC;             // [RR][NRH][32] rhs, row geometry
+  static constexpr int aj = r + RR * NRH * NC;       // [RR][15][32] R: |A|, J
+  static constexpr int hg = aj + rsz(RR * 15 * NC);  // [12][32] H, g of the last row
+  static constexpr int total1 = hg + 12 * NC;
+  // way back up, chunks q & 3: u, species of w, H and g, and x of two chunks
+  static constexpr int UP = kMarchUp;
+  static constexpr int u = 0;                    // [4][NV][32][UP], swizzled
+  static constexpr int sp = u + 4 * UP * NV * NC;  // [4][ny][32][UP], swizzled
+  static constexpr int h = sp + 4 * UP * ny * NC;  // [4][UP][12][32]
+  static constexpr int x = h + 4 * UP * 12 * NC;   // [2][UP][3][32]
+  static constexpr int total2 = x + 2 * UP * 3 * NC;
+  static constexpr int total = total1 > total2 ? total1 : total2;
+  // the levels' dx follow at `total`
+  static constexpr size_t bytes(int nc1) { return sizeof(double) * ((size_t)total + nc1); }
+};
+
+// levels per chunk
+template <typename R>
+constexpr int march_chunk(int ny) {
+  return sizeof(R) == 4 && ny <= 3 ? 8 : 4;
+}
+
+// barriers reached from the level warps' and the elimination warp's own loops
+template <int ID, int NT>
+__device__ __forceinline__ void march_sync() {
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(NT) : "memory");
+}
+
+template <int ID, int NT>
+__device__ __forceinline__ void march_arrive() {
+  asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(NT) : "memory");
+}
+
+struct MarchMaps {
+  CUtensorMap w, du, u, sp;
+};
+
+__device__ __forceinline__ void march_tma_load(double *dst, const CUtensorMap *map, int x, int j,
+                                               int k, int n, int pan, uint64_t *m) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(smem_addr(dst)),
+      "l"(map), "r"(x), "r"(j), "r"(k), "r"(n), "r"(pan), "r"(smem_addr(m))
+      : "memory");
+}
+__device__ __forceinline__ void march_tma_store(const CUtensorMap *map, int x, int j, int k, int n,
+                                                int pan, const double *src) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.global.shared::cta.tile.bulk_group "
+      "[%0, {%1, %2, %3, %4, %5}], [%6];" ::"l"(map),
+      "r"(x), "r"(j), "r"(k), "r"(n), "r"(pan), "r"(smem_addr(src))
+      : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+
+// place of (variable, column, level) in a box of 8 or 4 levels as TMA lays it
+// out with the 64- or 32-byte swizzle: 16-byte pieces permuted so that a
+// warp's reads of one level spread over the banks
+template <int C>
+__device__ __forceinline__ int march_box(int n, int c, int o) {
+  if constexpr (C == 8) return (n * kMarchCols + c) * 8 + ((((o >> 1) ^ (c >> 1)) & 3) << 1) + (o & 1);
+  else return (n * kMarchCols + c) * 4 + ((((o >> 1) ^ (c >> 2)) & 1) << 1) + (o & 1);
+}
+
+// reciprocal by two Newton-Raphson steps on the hardware's approximation
+// (relative error 2^-20 -> 2^-40 -> below one ulp for normal numbers): no
+// branch for the rare ranges, so that a row's elimination schedules as one
+// block of instructions
+__device__ __forceinline__ double march_rcp(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  r = fma(r, fma(-d, r, 1.), r);
+  return fma(r, fma(-d, r, 1.), r);
+}
+
+template <int NY, int RECON, int RS, typename R, int GEO, int C>
+__global__ void __launch_bounds__((C + 2) * 32, 2)
+    k_x1march(Geom g, canoe_thermo_t th, Mix<R> mx, MarchTile tl,
+              const __grid_constant__ MarchMaps maps,
+              const double *__restrict__ w, const double *__restrict__ du, double *u, double *scr,
+              const double *__restrict__ dtp, Stage st, int stage) {
+  using S = Slots<NY>;
+  using P = MarchSmem<5 + NY, C, R, GEO>;
+  constexpr int NV = S::NV, NC = kMarchCols, N = 3, UP = kMarchUp;
+  constexpr int ND = march_nd(NY), NCOMP = march_comp(NY);
+  constexpr int RQ = P::RQ, RP = P::RP, NR = P::NR, RR = P::RR, NRH = P::NRH;
+  constexpr bool PERT = sizeof(R) == 4;
+  constexpr int NTP = C * 32, NTA = NTP + 64;
+  extern __shared__ __align__(1024) double sm[];
+  __shared__ __align__(8) uint64_t mbar[6];  // w, du, four chunks of the way up
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nc1 = g.nc1, is = g.is, ie = g.ie;
+  const bool bulk = g.bulk != 0;
+  const bool leader = threadIdx.x == 0;
+
+  // the tile's first column, and this lane's column within it: columns past
+  // the block's edge repeat the last one inside and write nothing to u (their
+  // scratch is their own)
+  const int tj = blockIdx.x % tl.nj, tkp = blockIdx.x / tl.nj;
+  const int pan = tkp / tl.nk;
+  const int j0 = g.js + tj * tl.bj, k0 = g.ks + (tkp - pan * tl.nk) * tl.bk;
+  auto column = [&](int c, int &j, int &k) {  // nearest column of the block
+    j = min(j0 + c % tl.bj, g.je);
+    k = min(k0 + c / tl.bj, g.ke);
+  };
+  int j, k;
+  column(lane, j, k);
+  const int lc = (k - k0) * tl.bj + (j - j0);
+  const bool on = lc == lane;
+  const int64_t pbase = g.npanel > 1 ? (int64_t)pan * g.pstride : 0;
+  const int64_t base = pbase + (int64_t)k * g.sk + (int64_t)j * nc1;
+  double *scrh = scr + (int64_t)blockIdx.x * g.nx1 * kMarchH * NC;  // H, g of the tile
+  scr += (int64_t)gridDim.x * g.nx1 * kMarchH * NC + (int64_t)blockIdx.x * g.nx1 * NCOMP * NC;
+  const double grav = th.grav;
+  const double wght = st.beta * dtp[0], idt = 1. / wght;
+  double *wb = sm + P::w, *db = sm + P::d, *rb = sm + P::r + lane;
+  double *psr = sm + P::ps + lane, *gmr = sm + P::gm + lane, *rawb = sm + P::raw + lane;
+  R *qb = reinterpret_cast<R *>(sm + P::q) + lane;
+  R *fb = reinterpret_cast<R *>(sm + P::f) + lane;
+  R *wrb = reinterpret_cast<R *>(sm + P::wr) + lane;
+  R *ajb = reinterpret_cast<R *>(sm + P::aj) + lane;
+  double *sdx = sm + P::total;  // dx1f
+  const int last_m = nc1 / C;  // rows lag the levels by four: t = nc1 ends them
+
+  // a bounded wait that gave up is reported once; the tile then runs on
+  // without waiting (its values are lost, nothing hangs)
+  bool ok = true;
+  auto wait = [&](int q, uint32_t parity) {
+    if (ok && !mbar_wait(mbar + q, parity)) {
+      ok = false;
+      if (g.err) atomicOr(g.err, (uint32_t)CANOE_EBIT_TIMEOUT);
+    }
+  };
+  constexpr uint32_t kBoxBytes = C * NV * NC * 8;
+  if (leader) {
+    for (int q = 0; q < 6; ++q) mbar_init(mbar + q, 1);
+    fence_mbar_init();
+  }
+  for (int i = threadIdx.x; i < nc1; i += NTA) sdx[i] = g.dx1f[i];
+  __syncthreads();
+
+  if (warp < C) {
+    const int64_t nkj = (int64_t)g.nc3 * g.nc2;
+    auto tab = [&](int t, int kk, int jj) { return g.shell[t * nkj + (int64_t)kk * g.nc2 + jj]; };
+    double cosc = 0., sinc = 1., cth1 = 0.;
+    if constexpr (GEO) {
+      cosc = tab(kTabCosC, k, j);
+      sinc = tab(kTabSinC, k, j);
+      cth1 = tab(kTabCth1, k, j);
+    }
+    // without TMA: this warp's variables of a box through registers, lanes
+    // along the levels of 32 / C columns at a time
+    constexpr int NPW = (NV + C - 1) / C;  // variables per warp
+    constexpr int CPI = 32 / C;            // columns per load
+    double ld[NPW][C];
+    auto reg_load = [&](const double *arr, int lo) {
+      const int l = lo + lane % C;
+#pragma unroll
+      for (int q = 0; q < C; ++q) {
+        int cj, ck;
+        column(q * CPI + lane / C, cj, ck);
+        const double *src = arr + pbase + (int64_t)ck * g.sk + (int64_t)cj * nc1 + l;
+#pragma unroll
+        for (int v = 0; v < NPW; ++v) {
+          const int n = warp + v * C;
+          ld[v][q] = n < NV && l >= 0 && l < nc1 ? src[n * g.sv] : 0.;
+        }
+      }
+    };
+    auto reg_store = [&](double *dst) {
+#pragma unroll
+      for (int q = 0; q < C; ++q)
+#pragma unroll
+        for (int v = 0; v < NPW; ++v) {
+          const int n = warp + v * C;
+          if (n < NV) dst[march_box<C>(n, q * CPI + lane / C, lane % C)] = ld[v][q];
+        }
+    };
+    // chunk m: w of levels lo .. lo + C - 1; du of the rows it completes, four
+    // levels up
+    auto chunk_lo = [&](int m) { return nc1 - C * (m + 1); };
+    auto tma_w = [&](int m) {
+      if (leader && m <= last_m) {
+        mbar_expect_tx(mbar, kBoxBytes);
+        march_tma_load(wb, &maps.w, chunk_lo(m), j0, k0, 0, pan, mbar);
+      }
+    };
+    auto wrap = [](int s) { return s < 0 ? s + RQ : (s >= RQ ? s - RQ : s); };
+    static_assert(RR == RQ, "rows and levels share their ring places");
+    int bq = 0;  // ring place of the chunk's first level and row
+    if (bulk) {
+      tma_w(0);
+    } else {
+      reg_load(w, chunk_lo(0));
+      reg_store(wb);
+    }
+    if (warp == 0) {
+      // face pressures from the top of the column up through the ghosts
+      // (t = 2 is the face ie + 1)
+      const double *w0 = w + base, *wp_ = w0 + S::IPR * g.sv;
+      const double RdTv = wp_[ie] / w0[ie];
+      double p = wp_[ie] * exp(grav * sdx[ie] / (2 * RdTv));
+      const double gt = g.bc[1] == CANOE_BC_REFLECT ? -grav : grav;
+      psr[2 * NC] = p;
+#pragma unroll
+      for (int t = 1; t <= NG; ++t) {
+        p = p + gt * w0[ie + t] * sdx[ie + t];
+        psr[((2 - t) & (RP - 1)) * NC] = p;
+      }
+    }
+    march_sync<0, NTA>();
+    for (int m = 0; m <= last_m; ++m) {
+      const int t = m * C + warp;
+      // ---- phase 1
+      if (bulk) {
+        if (leader) {
+          mbar_expect_tx(mbar + 1, kBoxBytes);
+          march_tma_load(db, &maps.du, chunk_lo(m) + 4, j0, k0, 0, pan, mbar + 1);
+        }
+        wait(0, m & 1);
+      }
+      if (t < nc1) {
+        double wv[NV];
+#pragma unroll
+        for (int n = 0; n < NV; ++n) wv[n] = wb[march_box<C>(n, lc, C - 1 - warp)];
+        double a, b;  // psf(l), psf(l + 1)
+        if (t <= 2) {
+          a = psr[t * NC];
+          b = psr[((t - 1) & (RP - 1)) * NC];
+        } else {
+          // psf(i) = psf(i+1) - grav rho(i) dx(i) from the top, in the
+          // reference's order; every warp sums down from the last level of
+          // the previous chunk
+          const int t0 = m == 0 ? 2 : m * C - 1;
+          a = psr[(t0 & (RP - 1)) * NC];
+          b = a;
+          for (int s = t0 + 1; s <= t; ++s) {
+            const int i = nc1 - 1 - s;
+            const double gg = i < is && g.bc[0] == CANOE_BC_REFLECT ? -grav : grav;
+            const double x = gg * wb[march_box<C>(0, lc, C - 1 - (s - m * C))];
+            b = a;
+            a = a - x * sdx[i];
+          }
+          psr[(t & (RP - 1)) * NC] = a;
+        }
+        const double pv = fabs(a - b) < 1.E-6 ? 0.5 * (a + b) : (a - b) / log(a / b);
+        double feps = 1.;
+#pragma unroll
+        for (int n = 1; n <= NY; ++n)
+          if (n <= th.nvapor) feps += wv[n] * th.inv_mu_ratio_m1[n - 1];
+        const double gmv = th.rd * feps;
+        gmr[wrap(bq + warp) * NC] = gmv;
+        R *qo = qb + wrap(bq + warp) * NV * NC;
+        qo[0] = R(wv[S::IPR] / (wv[0] * gmv));
+        qo[S::IPR * NC] = R(wv[S::IPR] - pv);
+#pragma unroll
+        for (int n = 1; n < NV - 1; ++n) qo[n * NC] = R(wv[n]);
+        double *ro = rawb + wrap(bq + warp) * NR * NC;
+        ro[0] = wv[0];
+        ro[NC] = wv[S::IPR];
+        if constexpr (NR > 2) ro[2 * NC] = wv[S::IVX];
+        if constexpr (NR > 3) {
+          ro[3 * NC] = wv[S::IVY];
+          ro[4 * NC] = wv[S::IVZ];
+        }
+      }
+      march_sync<1, NTP>();
+      // ---- phase 2: cells t - 2, by (variable, group of four cells)
+      if (!bulk) reg_load(du, chunk_lo(m) + 4);
+      {
+      // the warp's group of four cells and its first variable; its next ones
+      // are four apart
+      constexpr int SG = C / 4;
+      const int e0 = 4 * (warp % SG), n0 = warp / SG;
+      // q of the levels from two below the group's last cell to two above its
+      // first
+      const R *qp[8];
+      R *fp[4];
+#pragma unroll
+      for (int y = 0; y < 8; ++y) qp[y] = qb + (wrap(bq + e0 - 4 + y) * NV + n0) * NC;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) fp[e] = fb + (wrap(bq + e0 + e - 2) * NV + n0) * NC;
+      R *hp = wrb + (e0 * NV + n0) * NC;
+      const bool outflow = g.bc[0] == CANOE_BC_OUTFLOW || g.bc[1] == CANOE_BC_OUTFLOW;
+#pragma unroll
+      for (int it = 0; it < (NV + 3) / 4; ++it) {
+        const int n = n0 + 4 * it;
+        if (n >= NV) break;
+        R qv[8];
+#pragma unroll
+        for (int y = 0; y < 8; ++y) qv[y] = qp[y][4 * it * NC];
+        if (outflow && (n == 0 || n == S::IPR)) {
+          // density and pressure of outflow ghosts take the transformed
+          // values of the first / last interior cell
+          // (change_to_temperature.cpp:114-127)
+          for (int y = 0; y < 8; ++y) {
+            int d = e0 - 4 + y;
+            if (g.bc[0] == CANOE_BC_OUTFLOW) d = min(d, nc1 - 4 - m * C);
+            if (g.bc[1] == CANOE_BC_OUTFLOW) d = max(d, 3 - m * C);
+            if (d != e0 - 4 + y && d >= -4 && d < C) {
+              const R v = qb[(wrap(bq + d) * NV + n) * NC];
+#pragma unroll
+              for (int z = 0; z < 8; ++z)
+                if (z == y) qv[z] = v;
+            }
+          }
+        }
+        R lo[4], hi[4];
+        if constexpr (RECON == CANOE_RECON_PPM) {
+          R sl[6], fc[5];  // slopes of qv[1 .. 6]; faces below qv[1 .. 5]
+#pragma unroll
+          for (int y = 0; y < 6; ++y) sl[y] = ppm_slope(qv[y + 2], qv[y + 1], qv[y]);
+#pragma unroll
+          for (int y = 0; y < 5; ++y) fc[y] = ppm_face(qv[y + 2], qv[y + 1], sl[y + 1], sl[y]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            lo[e] = fc[e + 1];
+            hi[e] = fc[e];
+            ppm_limit(qv[e + 2], lo[e], hi[e]);
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            // cell of the group, kept inside is - 1 .. ie + 1
+            const int c = max(min(nc1 - 1 - (m * C + e0 + e - 2), ie + 1), is - 1);
+            plm_cell_nu(qv[e + 3], qv[e + 2], qv[e + 1], R(g.x1v[c - 1]), R(g.x1v[c]),
+                        R(g.x1v[c + 1]), R(g.x1f[c]), R(g.x1f[c + 1]), lo[e], hi[e]);
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          fp[e][4 * it * NC] = lo[e];
+          hp[(e * NV + 4 * it) * NC] = hi[e];
+        }
+      }
+      }
+      if (!bulk) reg_store(db);
+      march_sync<1, NTP>();
+      // ---- phase 3: face t - 3, between the cells t - 2 (left) and t - 3
+      if (t >= 5 && t < nc1) {
+        R *fo = fb + wrap(bq + warp - 3) * NV * NC;
+        R wl[NV], wr[NV], fx[NV];
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+          wl[n] = wrb[(warp * NV + n) * NC];
+          wr[n] = fo[n * NC];
+        }
+        const double pf = psr[((t - 3) & (RP - 1)) * NC];
+        const double gamma = sqrt(gmr[wrap(bq + warp - 3) * NC] * gmr[wrap(bq + warp - 2) * NC]);
+        if constexpr (PERT) {
+          R pr = wr[S::IPR], pl = wl[S::IPR];
+          if (R(pf) + pr < R(0)) pr = R(0);
+          if (R(pf) + pl < R(0)) pl = R(0);
+          wr[S::IPR] = pr;
+          wl[S::IPR] = pl;
+          wr[0] = (R(pf) + pr) / (wr[0] * R(gamma));
+          wl[0] = (R(pf) + pl) / (wl[0] * R(gamma));
+        } else {
+          double pr = wr[S::IPR] + pf;
+          if (pr < 0.) pr = pf;
+          wr[S::IPR] = pr;
+          wr[0] = pr / (wr[0] * gamma);
+          double pl = wl[S::IPR] + pf;
+          if (pl < 0.) pl = pf;
+          wl[S::IPR] = pl;
+          wl[0] = pl / (wl[0] * gamma);
+        }
+        if constexpr (GEO) {
+          if constexpr (PERT) hllc_pert<R, NY, 0, true>(mx, wl, wr, R(pf), fx, R(cosc));
+          else hllc<R, NY, 0, true>(mx, wl, wr, fx, R(cosc));
+          const R ty = fx[S::IVY], tz = fx[S::IVZ];
+          fx[S::IVY] = ty + tz * R(cth1);
+          fx[S::IVZ] = tz + ty * R(cth1);
+        } else if constexpr (PERT) {
+          riemann_pert<R, NY, RS, 0>(mx, wl, wr, R(pf), fx);
+        } else {
+          riemann<R, NY, RS, 0>(mx, wl, wr, fx);
+        }
+#pragma unroll
+        for (int n = 0; n < NV; ++n) fo[n * NC] = fx[n];
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // wR's place takes w
+      march_sync<0, NTA>();
+      // ---- phase 4: row i, level t - 4
+      if (bulk) {
+        tma_w(m + 1);
+        wait(1, m & 1);
+      } else {
+        reg_load(w, chunk_lo(m + 1));
+      }
+      if (t >= 5 && t <= nc1) {
+        const int i = nc1 - 1 - (t - 4);
+        const double *rd = rawb + wrap(bq + warp - 3) * NR * NC;  // cell i - 1
+        const double *ru = rawb + wrap(bq + warp - 4) * NR * NC;  // cell i
+        const R *qd = qb + wrap(bq + warp - 3) * NV * NC, *qu = qb + wrap(bq + warp - 4) * NV * NC;
+        if (i <= ie) {
+          const R *flo = fb + wrap(bq + warp - 4) * NV * NC;
+          const R *fhi = fb + wrap(bq + warp - 5) * NV * NC;
+          const double rho = ru[0], v1 = NR > 2 ? ru[2 * NC] : (double)qu[S::IVX * NC];
+          const double gsrc = wght * rho * grav;
+          const double plo = psr[((t - 4) & (RP - 1)) * NC], phi = psr[((t - 5) & (RP - 1)) * NC];
+          double dv[NV], dd, ra = 1.;  // diagonal of the scaled row, its area ratio
+          if constexpr (GEO) {
+            const double d2 = tab(kTabDx2A, k, j), d3 = tab(kTabDx3A, k, j);
+            const double sc = sinc, cs = cosc;
+            const double xv = g.x1v[i], df = sdx[i];
+            const double a1m = d2 * d3 * g.x1f[i] * g.x1f[i] * sc;
+            const double a1p = d2 * d3 * g.x1f[i + 1] * g.x1f[i + 1] * sc;
+            const double vol = df * d2 * d3 * xv * xv * sc;
+            const double a2m = xv * tab(kTabDx3AF2, k, j) * df;
+            const double a2p = xv * tab(kTabDx3AF2, k, j + 1) * df;
+            const double a3m = xv * tab(kTabDx2AF3, k, j) * df;
+            const double a3p = xv * tab(kTabDx2AF3, k + 1, j) * df;
+            const double v2 = NR > 3 ? ru[3 * NC] : (double)qu[S::IVY * NC];
+            const double v3 = NR > 3 ? ru[4 * NC] : (double)qu[S::IVZ * NC];
+            const double pr = ru[NC];
+            const double v_2 = v2 + v3 * cs, v_3 = v3 + v2 * cs, sine2 = sc * sc;
+            const double x_ov_rD =
+                (a2m * tab(kTabSinF2, k, j) - a2p * tab(kTabSinF2, k, j + 1)) / vol;
+            const double y_ov_rC =
+                (a3m * tab(kTabSinF3, k, j) - a3p * tab(kTabSinF3, k + 1, j)) / vol;
+            double csrc[3];
+            csrc[0] = wght * ((2.0 * pr + rho * (v2 * v_2 + v3 * v_3)) / xv);
+            csrc[1] = wght * (-x_ov_rD * (pr + rho * v3 * v3 * sine2) - rho * v1 * v_2 / xv);
+            csrc[2] = wght * (-y_ov_rC * (pr + rho * v2 * v2 * sine2) - rho * v1 * v_3 / xv);
+#pragma unroll
+            for (int n = 0; n < NV; ++n) {
+              double dfl = a1p * (double)fhi[n * NC] - a1m * (double)flo[n * NC];
+              if (PERT && n == S::IVX) dfl += a1p * phi - a1m * plo;
+              double v = -(wght * dfl / vol);
+              if (n == S::IVX) v += csrc[0];
+              if (n == S::IVY) v += csrc[1];
+              if (n == S::IVZ) v += csrc[2];
+              if (n == S::IVX) v += gsrc;
+              if (n == S::IPR) v += gsrc * v1;
+              dv[n] = v;
+            }
+            dd = idt * (2. * vol / a1m);
+            ra = a1p / a1m;
+          } else {
+            const double idx = 1. / sdx[i];
+#pragma unroll
+            for (int n = 0; n < NV; ++n) {
+              double d = ((double)fhi[n * NC] - (double)flo[n * NC]) * idx;
+              if (PERT && n == S::IVX) d += (phi - plo) * idx;
+              double v = -(wght * d);
+              if (n == S::IVX) v += gsrc;
+              if (n == S::IPR) v += gsrc * v1;
+              dv[n] = v;
+            }
+            dd = idt * (2. * sdx[i]);
+          }
+#pragma unroll
+          for (int n = 0; n < NV; ++n) dv[n] = db[march_box<C>(n, lc, C - 1 - warp)] + dv[n];
+          double dsum = dv[0];
+#pragma unroll
+          for (int n = 1; n <= NY; ++n) dsum += dv[n];
+          double *ro = rb + wrap(bq + warp) * NRH * NC;
+          ro[0] = dsum * dd;
+          ro[NC] = dv[S::IVX] * dd;
+          ro[2 * NC] = dv[S::IPR] * dd;
+          ro[3 * NC] = dd;
+          if constexpr (GEO) ro[4 * NC] = ra;
+          double *so = scr + (int64_t)(i - is) * NCOMP * NC + lane;
+#pragma unroll
+          for (int n = 1; n <= NY; ++n) so[(1 + n) * NC] = dv[n];
+          so[0] = dv[S::IVY];
+          so[NC] = dv[S::IVZ];
+          if constexpr (NY > 0) so[(2 + NY) * NC] = dsum;
+        }
+        // |A| at face i and J of cell i - 1
+        {
+          const double gm1 = mx.gm1;
+          // the FP32 path evaluates them in FP32: its velocities and mass
+          // fractions are rounded in q already
+          using W = typename std::conditional<GEO, double, R>::type;
+          W wu[NV], wd[NV];
+#pragma unroll
+          for (int n = 1; n < NV - 1; ++n) {
+            wd[n] = qd[n * NC];
+            wu[n] = qu[n * NC];
+          }
+          wd[0] = W(rd[0]);
+          wu[0] = W(ru[0]);
+          wd[S::IPR] = W(rd[NC]);
+          wu[S::IPR] = W(ru[NC]);
+          if constexpr (GEO) {
+            // velocities projected to the local frame, in FP64
+            if constexpr (NR > 3) {
+#pragma unroll
+              for (int n = 0; n < 3; ++n) {
+                wd[S::IVX + n] = rd[(2 + n) * NC];
+                wu[S::IVX + n] = ru[(2 + n) * NC];
+              }
+            }
+            wd[S::IVY] += wd[S::IVZ] * cosc;
+            wu[S::IVY] += wu[S::IVZ] * cosc;
+            wd[S::IVZ] *= sinc;
+            wu[S::IVZ] *= sinc;
+          }
+          R *ao = ajb + wrap(bq + warp) * 15 * NC;
+          M<N> mt;
+          jacobian<N, NY, R>(mt, gm1, wd);  // its first row is 0 1 0
+#pragma unroll
+          for (int e = 0; e < 6; ++e) ao[(9 + e) * NC] = R(mt.a[1 + e / 3][e % 3]);
+          abs_jacobian<N, NY, R>(mt, mx, gm1, wd, wu);
+#pragma unroll
+          for (int e = 0; e < 9; ++e) ao[e * NC] = R(mt.a[e / 3][e % 3]);
+        }
+      }
+      if (!bulk) reg_store(wb);
+      bq = wrap(bq + C);
+      march_sync<0, NTA>();
+    }
+  } else {
+    // ---- elimination of the rows of chunk m, while the level warps work on
+    // chunk m + 1; this warp takes every second row
+    const int e2 = warp - C;
+    double *hg = sm + P::hg + lane;
+    auto row = [&](int t) {
+      if (t < 7 || t > nc1) return;  // rows ie .. is
+      const int i = nc1 - 1 - (t - 4);
+      // |A| at faces i and i + 1; J of cells i - 1, i and i + 1 (rows 1, 2)
+      const R *ai = ajb + (t % RR) * 15 * NC, *ap = ajb + ((t - 1) % RR) * 15 * NC;
+      const R *jm = ai + 9 * NC, *jc = ap + 9 * NC, *jp = ajb + ((t - 2) % RR) * 15 * NC + 9 * NC;
+      auto jrow = [](const R *j6, int x, int y) {
+        return x == 0 ? (y == 1 ? 1. : 0.) : (double)j6[((x - 1) * 3 + y) * NC];
+      };
+      const double *ri = rb + (t % RR) * NRH * NC;
+      const double dd = ri[3 * NC];
+      const double ra = GEO ? ri[4 * NC] : 1.;
+      double D[3][3], b[3][3], c[3][3], v[3];
+#pragma unroll
+      for (int x = 0; x < 3; ++x) {
+        v[x] = ri[x * NC];
+#pragma unroll
+        for (int y = 0; y < 3; ++y) {
+          const double am = ai[(3 * x + y) * NC], au = ap[(3 * x + y) * NC];
+          if constexpr (GEO) {
+            D[x][y] = am + au * ra + (ra - 1.) * jrow(jc, x, y);
+            c[x][y] = (au - jrow(jp, x, y)) * ra;
+          } else {
+            D[x][y] = am + au;
+            c[x][y] = x == 0 && y != 1 ? au : au - jrow(jp, x, y);
+          }
+          b[x][y] = x == 0 && y != 1 ? am : am + jrow(jm, x, y);
+        }
+      }
+      const double ph = grav * wght * dd;  // gravity over the row's scale
+      D[0][0] += dd;
+      D[1][1] += dd;
+      D[2][2] += dd;
+      D[1][0] -= ph;
+      D[2][1] -= ph;
+      if (i == is) {  // walls: the ghost cell mirrors the boundary cell
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+#pragma unroll
+          for (int y = 0; y < 3; ++y) {
+            D[x][y] += y == 1 ? b[x][y] : -b[x][y];
+            b[x][y] = 0.;
+          }
+      }
+      if (i == ie) {
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+#pragma unroll
+          for (int y = 0; y < 3; ++y) D[x][y] += y == 1 ? c[x][y] : -c[x][y];
+      } else {
+        // H, g of the row above, from the other warp
+        if (e2 == 0) march_sync<2, 64>();
+        else march_sync<3, 64>();
+#pragma unroll
+        for (int z = 0; z < 3; ++z) {
+          const double h0 = hg[3 * z * NC], h1 = hg[(3 * z + 1) * NC], h2 = hg[(3 * z + 2) * NC];
+          const double gz = hg[(9 + z) * NC];
+#pragma unroll
+          for (int x = 0; x < 3; ++x) {
+            D[x][0] -= c[x][z] * h0;
+            D[x][1] -= c[x][z] * h1;
+            D[x][2] -= c[x][z] * h2;
+            v[x] += c[x][z] * gz;
+          }
+        }
+      }
+      // adjugate over the determinant, as inv(M<3>)
+      double K[3][3];
+      K[0][0] = D[1][1] * D[2][2] - D[1][2] * D[2][1];
+      K[1][0] = D[1][2] * D[2][0] - D[1][0] * D[2][2];
+      K[2][0] = D[1][0] * D[2][1] - D[1][1] * D[2][0];
+      K[0][1] = D[0][2] * D[2][1] - D[0][1] * D[2][2];
+      K[1][1] = D[0][0] * D[2][2] - D[0][2] * D[2][0];
+      K[2][1] = D[0][1] * D[2][0] - D[0][0] * D[2][1];
+      K[0][2] = D[0][1] * D[1][2] - D[0][2] * D[1][1];
+      K[1][2] = D[0][2] * D[1][0] - D[0][0] * D[1][2];
+      K[2][2] = D[0][0] * D[1][1] - D[0][1] * D[1][0];
+      const double id = march_rcp(D[0][0] * K[0][0] + D[0][1] * K[1][0] + D[0][2] * K[2][0]);
+      double h[kMarchH];
+#pragma unroll
+      for (int x = 0; x < 3; ++x) {
+#pragma unroll
+        for (int y = 0; y < 3; ++y)
+          h[3 * x + y] = (K[x][0] * b[0][y] + K[x][1] * b[1][y] + K[x][2] * b[2][y]) * id;
+        h[9 + x] = (K[x][0] * v[0] + K[x][1] * v[1] + K[x][2] * v[2]) * id;
+      }
+#pragma unroll
+      for (int e = 0; e < kMarchH; ++e) hg[e * NC] = h[e];
+      if (t < nc1) {
+        if (e2 == 0) march_arrive<3, 64>();
+        else march_arrive<2, 64>();
+      }
+      double *so = scrh + (int64_t)(i - is) * kMarchH * NC + lane;
+#pragma unroll
+      for (int e = 0; e < kMarchH; ++e) so[e * NC] = h[e];
+    };
+    march_sync<0, NTA>();
+    march_sync<0, NTA>();  // phase 3 of chunk 0
+    march_sync<0, NTA>();  // phase 4 of chunk 0
+    for (int m = 0; m <= last_m; ++m) {
+      for (int p = e2; p < C - 2; p += 2) row(m * C + p);
+      // all but the chunk's last two rows are done before the next chunk's
+      // rows are formed in their places
+      if (m < last_m) march_sync<0, NTA>();  // phase 3 of chunk m + 1
+      row(m * C + C - 2 + e2);
+      if (m < last_m) march_sync<0, NTA>();  // phase 4 of chunk m + 1
+    }
+  }
+
+  // ---- way back up in chunks of four levels from 2 + 4 q (the first starts
+  // in the ghost level is - 1: boxes start at even levels).  Phase q: the
+  // elimination warp finds x of chunk q + 1, the level warps update chunk q,
+  // chunk q - 1 is written out and chunk q + 2 fetched.
+  asm volatile("fence.proxy.async;" ::: "memory");  // H, g and the buffers, before bulk copies
+  march_sync<0, NTA>();
+  const int nq = (ie - 2) / UP + 1;
+  double *ub = sm + P::u, *spb = sm + P::sp, *hb = sm + P::h, *xs = sm + P::x + lane;
+  constexpr int UC = UP * NV * NC, SC = UP * NY * NC, HC = UP * kMarchH * NC;
+  auto fetch_up = [&](int q) {  // by one lane
+    if (q >= nq) return;
+    uint64_t *mb = mbar + 2 + (q & 3);
+    const int lo = 2 + UP * q, i0 = max(lo, is), i1 = min(lo + UP - 1, ie);
+    const uint32_t hbytes = (i1 - i0 + 1) * kMarchH * NC * 8;
+    mbar_expect_tx(mb, hbytes + (bulk ? (UC + SC) * 8 : 0));
+    bulk_g2s(hb + (q & 3) * HC + (i0 - lo) * kMarchH * NC, scrh + (int64_t)(i0 - is) * kMarchH * NC,
+             hbytes, mb);
+    if (bulk) {
+      march_tma_load(ub + (q & 3) * UC, &maps.u, lo, j0, k0, 0, pan, mb);
+      if constexpr (NY > 0) march_tma_load(spb + (q & 3) * SC, &maps.sp, lo, j0, k0, 1, pan, mb);
+    }
+  };
+  if (warp < C) {
+    // C = 8: two warps per level, one for the densities, one for momenta and
+    // energy; C = 4: a warp does both
+    constexpr int HALVES = C / UP;
+    const int lev = warp / HALVES, half = HALVES == 2 ? warp % 2 : -1;
+    constexpr int N0 = NY > 0 ? 2 * NY + 2 : 1;  // values of the densities' half
+    constexpr int NL = HALVES == 2 ? (N0 > 6 ? N0 : 6) : N0 + 6;
+    double cur[NL], nxt[NL];
+    // scratch of the update: du and the sum of the densities, then u1
+    auto load_scr = [&](int q, double *v) {
+      const int i = 2 + UP * q + lev;
+      if (q >= nq || i < is || i > ie) return;
+      const double *si = scr + (int64_t)(i - is) * NCOMP * NC + lane;
+      int x = 0;
+      if (half != 1) {
+#pragma unroll
+        for (int n = 1; n <= NY; ++n) v[x++] = si[(1 + n) * NC];
+        if constexpr (NY > 0) v[x++] = si[(2 + NY) * NC];
+        if (stage != 0)
+#pragma unroll
+          for (int n = 0; n <= NY; ++n) v[x + n] = si[(ND + n) * NC];
+        x += NY + 1;
+      }
+      if (half != 0) {
+        v[x++] = si[0];
+        v[x++] = si[NC];
+        if (stage != 0)
+#pragma unroll
+          for (int n = 0; n < 4; ++n) v[x + n] = si[(ND + S::IVX + n) * NC];
+      }
+    };
+    // without TMA, u and the species of w through registers
+    constexpr int NE = (NV + NY) * UP * NC, NLD = (NE + NTP - 1) / NTP;
+    double rg[NLD];
+    auto reg_up = [&](int q, bool put) {
+#pragma unroll
+      for (int z = 0; z < NLD; ++z) {
+        const int e = threadIdx.x + z * NTP;
+        const int o = e % UP, c = e / UP % NC, n = e / (UP * NC);
+        const int l = 2 + UP * q + o;
+        if (e >= NE || q >= nq || l >= nc1) continue;
+        if (put) {
+          if (n < NV) ub[(q & 3) * UC + march_box<UP>(n, c, o)] = rg[z];
+          else spb[(q & 3) * SC + march_box<UP>(n - NV, c, o)] = rg[z];
+        } else {
+          int cj, ck;
+          column(c, cj, ck);
+          const int64_t at = pbase + (int64_t)ck * g.sk + (int64_t)cj * nc1 + l;
+          rg[z] = n < NV ? u[n * g.sv + at] : w[(n - NV + 1) * g.sv + at];
+        }
+      }
+    };
+    if (!bulk) {
+      reg_up(0, false);
+      reg_up(0, true);
+    }
+    load_scr(0, cur);
+    for (int q = -1; q <= nq; ++q) {
+      if (!bulk) {
+        if (q >= 1) {
+          const double *src = ub + ((q - 1) & 3) * UC;
+          for (int e = threadIdx.x; e < UC; e += NTP) {
+            const int o = e % UP, c = e / UP % NC, n = e / (UP * NC), l = 2 + UP * (q - 1) + o;
+            int cj, ck;
+            column(c, cj, ck);
+            if ((ck - k0) * tl.bj + cj - j0 == c && l >= is && l <= ie)
+              u[n * g.sv + pbase + (int64_t)ck * g.sk + (int64_t)cj * nc1 + l] =
+                  src[march_box<UP>(n, c, o)];
+          }
+        }
+        reg_up(q + 2, false);
+      }
+      if (q >= 0) load_scr(q + 1, nxt);
+      const int i = 2 + UP * q + lev;
+      if (q >= 0 && q < nq && i >= is && i <= ie) {
+        if (bulk) wait(2 + (q & 3), (q >> 2) & 1);
+        double *uc = ub + (q & 3) * UC;
+        const double *xi = xs + (q & 1) * UP * 3 * NC + lev * 3 * NC;
+        double *s1 = scr + (int64_t)(i - is) * NCOMP * NC + ND * NC + lane;
+        // slots n0 .. n0 + NN - 1: their increments dv, and u1 as loaded
+        auto update = [&](auto nn, int n0, const double *dv, const double *u1) {
+          constexpr int NN = decltype(nn)::value;
+          double uo[NN];
+#pragma unroll
+          for (int n = 0; n < NN; ++n) uo[n] = uc[march_box<UP>(n0 + n, lane, lev)];
+#pragma unroll
+          for (int n = 0; n < NN; ++n) {
+            if (stage == 0) s1[(n0 + n) * NC] = uo[n];
+            const double s = st.g1 * uo[n] + st.g2 * (stage == 0 ? uo[n] : u1[n]);
+            if (on) uc[march_box<UP>(n0 + n, lane, lev)] = s + dv[n];
+          }
+        };
+        if (half != 1) {
+          // species correction (forward_backward.hpp:101-124)
+          double dv[NY + 1];
+          const double x0 = xi[0];
+          dv[0] = x0;
+          if constexpr (NY > 0) {
+            const double dens = x0 - cur[NY];
+            const double *wc = spb + (q & 3) * SC;
+#pragma unroll
+            for (int n = 1; n <= NY; ++n) dv[n] = wc[march_box<UP>(n - 1, lc, lev)];
+#pragma unroll
+            for (int n = 1; n <= NY; ++n) {
+              dv[n] = cur[n - 1] + dens * dv[n];
+              dv[0] -= dv[n];
+            }
+          }
+          update(std::integral_constant<int, NY + 1>(), 0, dv, cur + (NY > 0 ? NY + 1 : 0));
+        }
+        if (half != 0) {
+          const double *cm = cur + (half == 1 ? 0 : NL - 6);
+          const double dv[4] = {xi[NC], cm[0], cm[1], xi[2 * NC]};
+          update(std::integral_constant<int, 4>(), S::IVX, dv, cm + 2);
+        }
+      }
+      if (q >= 0) {
+#pragma unroll
+        for (int z = 0; z < NL; ++z) cur[z] = nxt[z];
+      }
+      if (!bulk) reg_up(q + 2, true);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      march_sync<0, NTA>();
+    }
+  } else if (warp == C + 1) {
+    // the copies
+    if (lane == 0) fetch_up(0);
+    for (int q = -1; q <= nq; ++q) {
+      if (lane == 0) {
+        if (bulk && q >= 1)
+          march_tma_store(&maps.u, 2 + UP * (q - 1), j0, k0, 0, pan, ub + ((q - 1) & 3) * UC);
+        // chunk q - 2 has been read out: its place takes chunk q + 2
+        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        fetch_up(q + 2);
+      }
+      __syncwarp();
+      march_sync<0, NTA>();
+    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  } else {
+    double x[3] = {0., 0., 0.};
+    for (int q = -1; q <= nq; ++q) {
+      if (q + 1 < nq) {
+        wait(2 + ((q + 1) & 3), ((q + 1) >> 2) & 1);
+        double *xo = xs + ((q + 1) & 1) * UP * 3 * NC;
+        const double *hc = hb + ((q + 1) & 3) * HC + lane;
+#pragma unroll
+        for (int o = 0; o < UP; ++o) {
+          const int i = 2 + UP * (q + 1) + o;
+          if (i < is || i > ie) continue;
+          double y[3];
+#pragma unroll
+          for (int a = 0; a < 3; ++a)
+            y[a] = hc[(o * kMarchH + 9 + a) * NC] + (hc[(o * kMarchH + 3 * a) * NC] * x[0] +
+                                                     hc[(o * kMarchH + 3 * a + 1) * NC] * x[1] +
+                                                     hc[(o * kMarchH + 3 * a + 2) * NC] * x[2]);
+#pragma unroll
+          for (int a = 0; a < 3; ++a) xo[(o * 3 + a) * NC] = x[a] = y[a];
+        }
+      }
+      march_sync<0, NTA>();
+    }
+  }
+  if (!ok)  // copies still in flight get a second bounded wait
+    for (int q = 0; q < 6; ++q) mbar_wait(mbar + q, 0);
+}
+
+// the tensor map encoder of the driver (null where there is none)
+inline PFN_cuTensorMapEncodeTiled march_encoder() {
+  static const PFN_cuTensorMapEncodeTiled f = [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault,
+                                         &r) != cudaSuccess ||
+        r != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+    return (PFN_cuTensorMapEncodeTiled)p;
+  }();
+  return f;
+}
+
+// launcher for one NY (instantiated in march_ny*.cu)
+template <int NY>
+int run_x1march(const Geom &g, const canoe_thermo_t &th, int recon, int rs, int prec,
+                const double *w, const double *du, double *u, const double *dtp, const Stage &s,
+                int stage, cudaStream_t st) {
+  const bool ppm = recon == CANOE_RECON_PPM, hllc = rs == CANOE_RSOLVER_HLLC;
+  const bool f32 = prec == CANOE_FP32_PERTURBATION;
+  const int npan = g.npanel > 1 ? g.npanel : 1;
+  const MarchTile tl = march_tile(g.nx2, g.nx3);
+  Geom gg = g;
+  MarchMaps maps{};
+  auto al16 = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
+  gg.bulk = g.nc1 % 2 == 0 && al16(w) && al16(du) && al16(u) && march_encoder() ? 1 : 0;
+  // box of `lev` levels x the tile's columns x nn variables
+  auto encode = [&](CUtensorMap &m, const double *p, int lev, int nn) {
+    const cuuint64_t dim[5] = {(cuuint64_t)g.nc1, (cuuint64_t)g.nc2, (cuuint64_t)g.nc3,
+                               (cuuint64_t)(5 + NY), (cuuint64_t)npan};
+    const cuuint64_t pst = npan > 1 ? (cuuint64_t)g.pstride : (cuuint64_t)((5 + NY) * g.sv);
+    const cuuint64_t str[4] = {(cuuint64_t)g.nc1 * 8, (cuuint64_t)g.sk * 8, (cuuint64_t)g.sv * 8,
+                               pst * 8};
+    const cuuint32_t box[5] = {(cuuint32_t)lev, (cuuint32_t)tl.bj, (cuuint32_t)tl.bk,
+                               (cuuint32_t)nn, 1};
+    const cuuint32_t one[5] = {1, 1, 1, 1, 1};
+    return march_encoder()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, const_cast<double *>(p), dim,
+                           str, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           lev == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  auto go = [&](auto kern, const auto &mx, int C, size_t smem) -> int {
+    if (gg.bulk && !(encode(maps.w, w, C, 5 + NY) && encode(maps.du, du, C, 5 + NY) &&
+                     encode(maps.u, u, kMarchUp, 5 + NY) &&
+                     encode(maps.sp, w, kMarchUp, NY > 0 ? NY : 1)))
+      gg.bulk = 0;
+    if (int rc = ensure_smem((const void *)kern, smem)) return rc;
+    kern<<<(unsigned)(tl.nj * tl.nk * npan), (C + 2) * 32, smem, st>>>(
+        gg, th, mx, tl, maps, w, du, u, g.march, dtp, s, stage);
+    CB_CUDA(cudaGetLastError());
+    return 0;
+  };
+#define CB_MK(RC, RSV, R, GEO)                                                               \
+  go(k_x1march<NY, RC, RSV, R, GEO, march_chunk<R>(NY)>, make_mix<R>(th), march_chunk<R>(NY), \
+     MarchSmem<5 + NY, march_chunk<R>(NY), R, GEO>::bytes(g.nc1))
+  if (g.shell) {
+    if constexpr (NY == 0) {
+      if (!hllc) {
+        set_error("the cubed-sphere panel uses the HLLC solver");
+        return CANOE_ERR_UNSUPPORTED;
+      }
+      if (ppm) return f32 ? CB_MK(3, 1, float, 1) : CB_MK(3, 1, double, 1);
+      return f32 ? CB_MK(2, 1, float, 1) : CB_MK(2, 1, double, 1);
+    } else {
+      set_error("the cubed-sphere panel is dry");
+      return CANOE_ERR_UNSUPPORTED;
+    }
+  }
+  if (ppm) {
+    if (hllc) return f32 ? CB_MK(3, 1, float, 0) : CB_MK(3, 1, double, 0);
+    return f32 ? CB_MK(3, 0, float, 0) : CB_MK(3, 0, double, 0);
+  }
+  if (hllc) return f32 ? CB_MK(2, 1, float, 0) : CB_MK(2, 1, double, 0);
+  return f32 ? CB_MK(2, 0, float, 0) : CB_MK(2, 0, double, 0);
+#undef CB_MK
+}
+
+}  // namespace cb

@@ -32,10 +32,36 @@ __device__ __forceinline__ R pdiv(R a, R b) {
   else return a / b;
 }
 
+// The mixture constants of canoe_thermo_t in the arithmetic type, converted
+// once on the host: as a kernel parameter they are operands of the FP32
+// arithmetic, where canoe_thermo_t costs a conversion from FP64 at each use
+// that the registers do not let the compiler keep.
+template <typename R>
+struct Mix {
+  int nvapor;
+  R gm1;  // gammad - 1
+  R cv_ratio_m1[CANOE_MAX_NY], inv_mu_ratio_m1[CANOE_MAX_NY];
+};
+template <typename R>
+inline Mix<R> make_mix(const canoe_thermo_t &th) {
+  Mix<R> m{};
+  m.nvapor = th.nvapor;
+  m.gm1 = R(th.gammad - 1.);
+  for (int n = 0; n < CANOE_MAX_NY; ++n) {
+    m.cv_ratio_m1[n] = R(th.cv_ratio_m1[n]);
+    m.inv_mu_ratio_m1[n] = R(th.inv_mu_ratio_m1[n]);
+  }
+  return m;
+}
+template <typename R>
+__device__ __forceinline__ R mix_gm1(const canoe_thermo_t &th) { return R(th.gammad - 1.); }
+template <typename R>
+__device__ __forceinline__ R mix_gm1(const Mix<R> &th) { return th.gm1; }
+
 // Mixture adiabatic index from mass fractions w[1..NY]
 // (canoe src/interface/eos.hpp:48-67, rho = 1).
-template <typename R, int NY>
-__device__ __forceinline__ R get_gamma(const canoe_thermo_t &th, const R *w) {
+template <typename R, int NY, class TH>
+__device__ __forceinline__ R get_gamma(const TH &th, const R *w) {
   R fsig = R(1), feps = R(1);
 #pragma unroll
   for (int n = 1; n <= NY; ++n) {
@@ -45,12 +71,12 @@ __device__ __forceinline__ R get_gamma(const canoe_thermo_t &th, const R *w) {
     else
       feps -= w[n];
   }
-  return R(1) + R(th.gammad - 1.) * feps / fsig;
+  return R(1) + mix_gm1<R>(th) * feps / fsig;
 }
 
 // EquationOfState::SoundSpeed (canoe src/snap/eos/ideal_moist_hydro.cpp:87-91)
-template <typename R, int NY>
-__device__ __forceinline__ R sound_speed(const canoe_thermo_t &th, const R *w) {
+template <typename R, int NY, class TH>
+__device__ __forceinline__ R sound_speed(const TH &th, const R *w) {
   R gamma = get_gamma<R, NY>(th, w);
   return sqrt(gamma * w[Slots<NY>::IPR] / w[0]);
 }
@@ -136,8 +162,8 @@ __device__ __forceinline__ void plm_cell_nu(R qm, R q0, R qp, R xvm, R xv0,
 // LMARS (Chen et al. 2013): canoe src/snap/riemann/lmars.cpp:19-85.  The
 // kinetic term uses the identity lowering of Cartesian coordinates (the
 // reference indexes vec_lower's 3-element result with the variable slot).
-template <typename R, int NY, int DIR>
-__device__ __forceinline__ void lmars(const canoe_thermo_t &th, const R *wli,
+template <typename R, int NY, int DIR, class TH>
+__device__ __forceinline__ void lmars(const TH &th, const R *wli,
                                       const R *wri, R *flx) {
   using S = Slots<NY>;
   constexpr int ivx = S::IVX + DIR;
@@ -183,8 +209,8 @@ __device__ __forceinline__ void lmars(const canoe_thermo_t &th, const R *wli,
 // 25-233.  COVKE: the x1 problem on a cubed-sphere panel, whose kinetic
 // energy is contravariant . covariant velocity with the cell's cosine
 // ke_cth (hllc_transform.cpp:92-101); the Cartesian branch otherwise.
-template <typename R, int NY, int DIR, bool COVKE = false>
-__device__ __forceinline__ void hllc(const canoe_thermo_t &th, const R *wl,
+template <typename R, int NY, int DIR, bool COVKE = false, class TH>
+__device__ __forceinline__ void hllc(const TH &th, const R *wl,
                                      const R *wr, R *flx, R ke_cth = R(0)) {
   using S = Slots<NY>;
   constexpr int IVX = S::IVX, IVY = S::IVY, IVZ = S::IVZ, IPR = S::IPR;
@@ -289,8 +315,8 @@ __device__ __forceinline__ void hllc(const canoe_thermo_t &th, const R *wl,
   flx[IPR] = f[IPR];
 }
 
-template <typename R, int NY, int RS, int DIR>
-__device__ __forceinline__ void riemann(const canoe_thermo_t &th, const R *wl,
+template <typename R, int NY, int RS, int DIR, class TH>
+__device__ __forceinline__ void riemann(const TH &th, const R *wl,
                                         const R *wr, R *flx) {
   if constexpr (RS == CANOE_RSOLVER_LMARS)
     lmars<R, NY, DIR>(th, wl, wr, flx);
@@ -307,8 +333,8 @@ __device__ __forceinline__ void riemann(const canoe_thermo_t &th, const R *wl,
 // LMARS and, since sl + sr + sm = 1, for HLLC.  Absolute pressure enters only
 // where the solvers need it in relative terms (sound speeds, enthalpy).
 
-template <typename R, int NY, int DIR>
-__device__ __forceinline__ void lmars_pert(const canoe_thermo_t &th, const R *wli,
+template <typename R, int NY, int DIR, class TH>
+__device__ __forceinline__ void lmars_pert(const TH &th, const R *wli,
                                            const R *wri, R pref, R *flx) {
   using S = Slots<NY>;
   constexpr int ivx = S::IVX + DIR;
@@ -350,8 +376,8 @@ __device__ __forceinline__ void lmars_pert(const canoe_thermo_t &th, const R *wl
 
 // COVKE: the covariant kinetic energy of the x1 problem on a cubed-sphere
 // panel, as in hllc()
-template <typename R, int NY, int DIR, bool COVKE = false>
-__device__ __forceinline__ void hllc_pert(const canoe_thermo_t &th, const R *wl, const R *wr,
+template <typename R, int NY, int DIR, bool COVKE = false, class TH>
+__device__ __forceinline__ void hllc_pert(const TH &th, const R *wl, const R *wr,
                                           R pref, R *flx, R ke_cth = R(0)) {
   using S = Slots<NY>;
   constexpr int IVX = S::IVX, IVY = S::IVY, IVZ = S::IVZ, IPR = S::IPR;
@@ -449,8 +475,8 @@ __device__ __forceinline__ void hllc_pert(const canoe_thermo_t &th, const R *wl,
   flx[IPR] = f[IPR];
 }
 
-template <typename R, int NY, int RS, int DIR>
-__device__ __forceinline__ void riemann_pert(const canoe_thermo_t &th, const R *wl,
+template <typename R, int NY, int RS, int DIR, class TH>
+__device__ __forceinline__ void riemann_pert(const TH &th, const R *wl,
                                              const R *wr, R pref, R *flx) {
   if constexpr (RS == CANOE_RSOLVER_LMARS)
     lmars_pert<R, NY, DIR>(th, wl, wr, pref, flx);
