@@ -15,40 +15,44 @@ CB_DECL(2)
 CB_DECL(3)
 CB_DECL(6)
 #undef CB_DECL
-#define CB_DECL(NY)                                                                       \
-  extern template int run_x1march<NY>(const Geom &, const canoe_thermo_t &, int, int, int, \
-                                      const double *, const double *, double *,           \
-                                      const double *, const Stage &, int, cudaStream_t);
-CB_DECL(0)
-CB_DECL(1)
-CB_DECL(2)
-CB_DECL(3)
-CB_DECL(6)
+#define CB_DECL(NY, N)                                                                \
+  extern template int run_x1march<NY, N>(const Geom &, const canoe_thermo_t &, int, int, \
+                                         int, const double *, const double *, double *, \
+                                         const double *, const Stage &, int, cudaStream_t);
+#define CB_DECL2(NY) CB_DECL(NY, 3) CB_DECL(NY, 5)
+CB_DECL2(0)
+CB_DECL2(1)
+CB_DECL2(2)
+CB_DECL2(3)
+CB_DECL2(6)
+#undef CB_DECL2
 #undef CB_DECL
 
 size_t march_doubles(const Geom &g, const canoe_thermo_t &th, int flag, int prec) {
   const int64_t ncol = (int64_t)g.nx2 * g.nx3 * (g.npanel > 1 ? g.npanel : 1);
   const bool lines = line_solve_on(g, flag, 1) || line_solve_on(g, flag, 2);
-  // what the march provides: the 3x3 solve between walls, on the hydrostatic
+  // what the march provides: the x1 solve between walls, on the hydrostatic
   // decomposition, with du initialised by an x2 pass
-  if (!(flag & 1) || (flag & 8) || lines || g.bc[0] == CANOE_BC_PERIODIC || th.grav == 0. ||
-      !g.f2)
-    return 0;
-  if (ncol < (prec == CANOE_FP32_PERTURBATION ? kMarchMinCols32 : kMarchMinCols64)) return 0;
+  if (!(flag & 1) || lines || g.bc[0] == CANOE_BC_PERIODIC || th.grav == 0. || !g.f2) return 0;
+  const int n = flag & 8 ? 5 : 3;
+  const int least = n == 5 ? kMarchMinCols5
+                           : (prec == CANOE_FP32_PERTURBATION ? kMarchMinCols32 : kMarchMinCols64);
+  if (ncol < least) return 0;
   // columns too long for the CTA-per-column kernel stay refused there
-  if (sizeof(double) * col_smem(g.nv, g.nc1, g.nx1, 3, 0, 1).total > 227 * 1024) return 0;
-  return march_scratch_doubles(th.ny, g.nx1, g.nx2, g.nx3, g.npanel > 1 ? g.npanel : 1);
+  if (sizeof(double) * col_smem(g.nv, g.nc1, g.nx1, n, 0, 1).total > 227 * 1024) return 0;
+  return march_scratch_doubles(th.ny, n, g.nx1, g.nx2, g.nx3, g.npanel > 1 ? g.npanel : 1);
 }
 
+template <int N>
 static int launch_x1march(const Geom &g, const canoe_thermo_t &th, int recon, int rs, int prec,
                           const double *w, const double *du, double *u, const double *dtp,
                           const Stage &s, int stage, cudaStream_t st) {
   switch (th.ny) {
-    case 0: return run_x1march<0>(g, th, recon, rs, prec, w, du, u, dtp, s, stage, st);
-    case 1: return run_x1march<1>(g, th, recon, rs, prec, w, du, u, dtp, s, stage, st);
-    case 2: return run_x1march<2>(g, th, recon, rs, prec, w, du, u, dtp, s, stage, st);
-    case 3: return run_x1march<3>(g, th, recon, rs, prec, w, du, u, dtp, s, stage, st);
-    case 6: return run_x1march<6>(g, th, recon, rs, prec, w, du, u, dtp, s, stage, st);
+    case 0: return run_x1march<0, N>(g, th, recon, rs, prec, w, du, u, dtp, s, stage, st);
+    case 1: return run_x1march<1, N>(g, th, recon, rs, prec, w, du, u, dtp, s, stage, st);
+    case 2: return run_x1march<2, N>(g, th, recon, rs, prec, w, du, u, dtp, s, stage, st);
+    case 3: return run_x1march<3, N>(g, th, recon, rs, prec, w, du, u, dtp, s, stage, st);
+    case 6: return run_x1march<6, N>(g, th, recon, rs, prec, w, du, u, dtp, s, stage, st);
     default:
       set_error("unsupported number of mass-fraction slots");
       return CANOE_ERR_UNSUPPORTED;
@@ -71,7 +75,8 @@ int launch_x1col(const Geom &g, const canoe_thermo_t &th, int recon, int rs, int
     }
   }
   if (mode == kColStep && g.march)
-    return launch_x1march(g, th, recon, rs, prec, w, du, u, dtp, s, stage, st);
+    return flag & 8 ? launch_x1march<5>(g, th, recon, rs, prec, w, du, u, dtp, s, stage, st)
+                    : launch_x1march<3>(g, th, recon, rs, prec, w, du, u, dtp, s, stage, st);
   switch (th.ny) {
     case 0: return run_x1col<0>(g, th, recon, rs, flag, prec, mode, w, du, u, u1, dtp, s, stage, fo, st);
     case 1: return run_x1col<1>(g, th, recon, rs, flag, prec, mode, w, du, u, u1, dtp, s, stage, fo, st);

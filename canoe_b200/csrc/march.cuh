@@ -59,13 +59,20 @@ constexpr int kMarchUp = 4;     // levels per chunk of the way back up
 // for one: 128 levels 135 us in FP32, 250 us in FP64, where the CTA-per-column
 // kernel takes 38 and 46 ns a column.
 constexpr int kMarchMinCols32 = 3800, kMarchMinCols64 = 6000;
+// with 5x5 blocks one tile fills an SM: 134 us a round of 148 tiles at 64 levels
+// against 127 ns a column
+constexpr int kMarchMinCols5 = 1100;
 
-// scratch per level of a tile: H and g (12 components, a tile's levels
-// contiguous); then du of the species, of the two transverse momenta, and
-// (with species) the sum of the density increments, and the RK register u1
-constexpr int kMarchH = 12;
-__host__ __device__ constexpr int march_nd(int ny) { return 2 + ny + (ny > 0 ? 1 : 0); }
-__host__ __device__ constexpr int march_comp(int ny) { return march_nd(ny) + 5 + ny; }
+// scratch per level of a tile with N x N blocks: H and g (a tile's levels
+// contiguous); then du of the two transverse momenta (N = 3, whose solve
+// leaves them), of the species, and (with species) the sum of the density
+// increments, and the RK register u1
+__host__ __device__ constexpr int march_h(int n) { return n * n + n; }
+__host__ __device__ constexpr int march_nt(int n) { return n == 3 ? 2 : 0; }
+__host__ __device__ constexpr int march_nd(int ny, int n) {
+  return march_nt(n) + ny + (ny > 0 ? 1 : 0);
+}
+__host__ __device__ constexpr int march_comp(int ny, int n) { return march_nd(ny, n) + 5 + ny; }
 
 // tiles of bj x bk = 32 columns that cover nx2 x nx3 with the fewest tiles
 struct MarchTile {
@@ -81,9 +88,9 @@ inline MarchTile march_tile(int nx2, int nx3) {
   return best;
 }
 
-inline size_t march_scratch_doubles(int ny, int nx1, int nx2, int nx3, int npanel) {
+inline size_t march_scratch_doubles(int ny, int n, int nx1, int nx2, int nx3, int npanel) {
   const MarchTile t = march_tile(nx2, nx3);
-  return (size_t)t.nj * t.nk * npanel * nx1 * (kMarchH + march_comp(ny)) * kMarchCols;
+  return (size_t)t.nj * t.nk * npanel * nx1 * (march_h(n) + march_comp(ny, n)) * kMarchCols;
 }
 
 // Shared memory of a tile, in doubles.  Levels are counted from the top (t = 0
@@ -91,13 +98,13 @@ inline size_t march_scratch_doubles(int ny, int nx1, int nx2, int nx3, int npane
 // chunk and four levels hold the decomposed state q, the FP64 values that
 // later phases need beside it (raw), and the face states wL, overwritten by
 // the fluxes.
-template <int NV, int C, typename R, int GEO>
+template <int NV, int C, typename R, int GEO, int N>
 struct MarchSmem {
   static constexpr int RQ = C + 4, RP = 16, NC = kMarchCols, ny = NV - 5;
   // rows in the ring of |A|, J and the right-hand side: a chunk's, and the two
   // that the elimination still works on while the next chunk's are formed with
   // the two above them
-  static constexpr int RR = C + 4, NRH = GEO ? 5 : 4;
+  static constexpr int RR = C + 4, NRH = N + (GEO ? 2 : 1), NAJ = N * N + N * (N - 1);
   // raw: rho, p and, where q is rounded to FP32, v1 (GEO: all velocities)
   static constexpr int NR = sizeof(R) == 8 ? 2 : (GEO ? 5 : 3);
   static constexpr int rsz(int n) { return (n * (int)sizeof(R) + 7) / 8; }
@@ -110,16 +117,17 @@ struct MarchSmem {
   static constexpr int ps = f + rsz(RQ * NV * NC);   // [RP][32] face pressure
   static constexpr int gm = ps + RP * NC;            // [RQ][32] RovRd
   static constexpr int r = gm + RQ * NC;             // [RR][NRH][32] rhs, row geometry
-  static constexpr int aj = r + RR * NRH * NC;       // [RR][15][32] R: |A|, J
-  static constexpr int hg = aj + rsz(RR * 15 * NC);  // [12][32] H, g of the last row
-  static constexpr int total1 = hg + 12 * NC;
+  static constexpr int aj = r + RR * NRH * NC;       // [RR][NAJ][32] R: |A|, J
+  static constexpr int hg = aj + rsz(RR * NAJ * NC);  // [NH][32] H, g of the last row
+  static constexpr int NH = march_h(N);
+  static constexpr int total1 = hg + NH * NC;
   // way back up, chunks q & 3: u, species of w, H and g, and x of two chunks
   static constexpr int UP = kMarchUp;
   static constexpr int u = 0;                    // [4][NV][32][UP], swizzled
   static constexpr int sp = u + 4 * UP * NV * NC;  // [4][ny][32][UP], swizzled
-  static constexpr int h = sp + 4 * UP * ny * NC;  // [4][UP][12][32]
-  static constexpr int x = h + 4 * UP * 12 * NC;   // [2][UP][3][32]
-  static constexpr int total2 = x + 2 * UP * 3 * NC;
+  static constexpr int h = sp + 4 * UP * ny * NC;  // [4][UP][NH][32]
+  static constexpr int x = h + 4 * UP * NH * NC;   // [2][UP][N][32]
+  static constexpr int total2 = x + 2 * UP * N * NC;
   static constexpr int total = total1 > total2 ? total1 : total2;
   // the levels' dx follow at `total`
   static constexpr size_t bytes(int nc1) { return sizeof(double) * ((size_t)total + nc1); }
@@ -184,17 +192,18 @@ __device__ __forceinline__ double march_rcp(double d) {
   return fma(r, fma(-d, r, 1.), r);
 }
 
-template <int NY, int RECON, int RS, typename R, int GEO, int C>
-__global__ void __launch_bounds__((C + 2) * 32, 2)
+template <int NY, int RECON, int RS, typename R, int GEO, int C, int N>
+__global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     k_x1march(Geom g, canoe_thermo_t th, Mix<R> mx, MarchTile tl,
               const __grid_constant__ MarchMaps maps,
               const double *__restrict__ w, const double *__restrict__ du, double *u, double *scr,
               const double *__restrict__ dtp, Stage st, int stage) {
   using S = Slots<NY>;
-  using P = MarchSmem<5 + NY, C, R, GEO>;
-  constexpr int NV = S::NV, NC = kMarchCols, N = 3, UP = kMarchUp;
-  constexpr int ND = march_nd(NY), NCOMP = march_comp(NY);
-  constexpr int RQ = P::RQ, RP = P::RP, NR = P::NR, RR = P::RR, NRH = P::NRH;
+  using P = MarchSmem<5 + NY, C, R, GEO, N>;
+  constexpr int NV = S::NV, NC = kMarchCols, UP = kMarchUp;
+  constexpr int ND = march_nd(NY, N), NT = march_nt(N), NCOMP = march_comp(NY, N), NH = P::NH;
+  constexpr int RQ = P::RQ, RP = P::RP, NR = P::NR, RR = P::RR, NRH = P::NRH,
+                NAJ = P::NAJ;
   constexpr bool PERT = sizeof(R) == 4;
   constexpr int NTP = C * 32, NTA = NTP + 64;
   extern __shared__ __align__(1024) double sm[];
@@ -220,8 +229,8 @@ __global__ void __launch_bounds__((C + 2) * 32, 2)
   const bool on = lc == lane;
   const int64_t pbase = g.npanel > 1 ? (int64_t)pan * g.pstride : 0;
   const int64_t base = pbase + (int64_t)k * g.sk + (int64_t)j * nc1;
-  double *scrh = scr + (int64_t)blockIdx.x * g.nx1 * kMarchH * NC;  // H, g of the tile
-  scr += (int64_t)gridDim.x * g.nx1 * kMarchH * NC + (int64_t)blockIdx.x * g.nx1 * NCOMP * NC;
+  double *scrh = scr + (int64_t)blockIdx.x * g.nx1 * NH * NC;  // H, g of the tile
+  scr += (int64_t)gridDim.x * g.nx1 * NH * NC + (int64_t)blockIdx.x * g.nx1 * NCOMP * NC;
   const double grav = th.grav;
   const double wght = st.beta * dtp[0], idt = 1. / wght;
   double *wb = sm + P::w, *db = sm + P::d, *rb = sm + P::r + lane;
@@ -569,15 +578,21 @@ __global__ void __launch_bounds__((C + 2) * 32, 2)
           double *ro = rb + wrap(bq + warp) * NRH * NC;
           ro[0] = dsum * dd;
           ro[NC] = dv[S::IVX] * dd;
-          ro[2 * NC] = dv[S::IPR] * dd;
-          ro[3 * NC] = dd;
-          if constexpr (GEO) ro[4 * NC] = ra;
+          if constexpr (N == 5) {
+            ro[2 * NC] = dv[S::IVY] * dd;
+            ro[3 * NC] = dv[S::IVZ] * dd;
+          }
+          ro[(N - 1) * NC] = dv[S::IPR] * dd;
+          ro[N * NC] = dd;
+          if constexpr (GEO) ro[(N + 1) * NC] = ra;
           double *so = scr + (int64_t)(i - is) * NCOMP * NC + lane;
 #pragma unroll
-          for (int n = 1; n <= NY; ++n) so[(1 + n) * NC] = dv[n];
-          so[0] = dv[S::IVY];
-          so[NC] = dv[S::IVZ];
-          if constexpr (NY > 0) so[(2 + NY) * NC] = dsum;
+          for (int n = 1; n <= NY; ++n) so[(NT + n - 1) * NC] = dv[n];
+          if constexpr (NT > 0) {
+            so[0] = dv[S::IVY];
+            so[NC] = dv[S::IVZ];
+          }
+          if constexpr (NY > 0) so[(NT + NY) * NC] = dsum;
         }
         // |A| at face i and J of cell i - 1
         {
@@ -609,14 +624,14 @@ __global__ void __launch_bounds__((C + 2) * 32, 2)
             wd[S::IVZ] *= sinc;
             wu[S::IVZ] *= sinc;
           }
-          R *ao = ajb + wrap(bq + warp) * 15 * NC;
+          R *ao = ajb + wrap(bq + warp) * NAJ * NC;
           M<N> mt;
-          jacobian<N, NY, R>(mt, gm1, wd);  // its first row is 0 1 0
+          jacobian<N, NY, R>(mt, gm1, wd);  // its first row is 0 1 0 ..
 #pragma unroll
-          for (int e = 0; e < 6; ++e) ao[(9 + e) * NC] = R(mt.a[1 + e / 3][e % 3]);
+          for (int e = 0; e < N * (N - 1); ++e) ao[(N * N + e) * NC] = R(mt.a[1 + e / N][e % N]);
           abs_jacobian<N, NY, R>(mt, mx, gm1, wd, wu);
 #pragma unroll
-          for (int e = 0; e < 9; ++e) ao[e * NC] = R(mt.a[e / 3][e % 3]);
+          for (int e = 0; e < N * N; ++e) ao[e * NC] = R(mt.a[e / N][e % N]);
         }
       }
       if (!bulk) reg_store(wb);
@@ -631,22 +646,23 @@ __global__ void __launch_bounds__((C + 2) * 32, 2)
     auto row = [&](int t) {
       if (t < 7 || t > nc1) return;  // rows ie .. is
       const int i = nc1 - 1 - (t - 4);
-      // |A| at faces i and i + 1; J of cells i - 1, i and i + 1 (rows 1, 2)
-      const R *ai = ajb + (t % RR) * 15 * NC, *ap = ajb + ((t - 1) % RR) * 15 * NC;
-      const R *jm = ai + 9 * NC, *jc = ap + 9 * NC, *jp = ajb + ((t - 2) % RR) * 15 * NC + 9 * NC;
-      auto jrow = [](const R *j6, int x, int y) {
-        return x == 0 ? (y == 1 ? 1. : 0.) : (double)j6[((x - 1) * 3 + y) * NC];
+      // |A| at faces i and i + 1; J of cells i - 1, i and i + 1 (rows 1 ..)
+      const R *ai = ajb + (t % RR) * NAJ * NC, *ap = ajb + ((t - 1) % RR) * NAJ * NC;
+      const R *jm = ai + N * N * NC, *jc = ap + N * N * NC,
+              *jp = ajb + ((t - 2) % RR) * NAJ * NC + N * N * NC;
+      auto jrow = [](const R *j, int x, int y) {
+        return x == 0 ? (y == 1 ? 1. : 0.) : (double)j[((x - 1) * N + y) * NC];
       };
       const double *ri = rb + (t % RR) * NRH * NC;
-      const double dd = ri[3 * NC];
-      const double ra = GEO ? ri[4 * NC] : 1.;
-      double D[3][3], b[3][3], c[3][3], v[3];
+      const double dd = ri[N * NC];
+      const double ra = GEO ? ri[(N + 1) * NC] : 1.;
+      double D[N][N], b[N][N], c[N][N], v[N];
 #pragma unroll
-      for (int x = 0; x < 3; ++x) {
+      for (int x = 0; x < N; ++x) {
         v[x] = ri[x * NC];
 #pragma unroll
-        for (int y = 0; y < 3; ++y) {
-          const double am = ai[(3 * x + y) * NC], au = ap[(3 * x + y) * NC];
+        for (int y = 0; y < N; ++y) {
+          const double am = ai[(N * x + y) * NC], au = ap[(N * x + y) * NC];
           if constexpr (GEO) {
             D[x][y] = am + au * ra + (ra - 1.) * jrow(jc, x, y);
             c[x][y] = (au - jrow(jp, x, y)) * ra;
@@ -656,73 +672,108 @@ __global__ void __launch_bounds__((C + 2) * 32, 2)
           }
           b[x][y] = x == 0 && y != 1 ? am : am + jrow(jm, x, y);
         }
+        D[x][x] += dd;
       }
       const double ph = grav * wght * dd;  // gravity over the row's scale
-      D[0][0] += dd;
-      D[1][1] += dd;
-      D[2][2] += dd;
       D[1][0] -= ph;
-      D[2][1] -= ph;
+      D[N - 1][1] -= ph;
       if (i == is) {  // walls: the ghost cell mirrors the boundary cell
 #pragma unroll
-        for (int x = 0; x < 3; ++x)
+        for (int x = 0; x < N; ++x)
 #pragma unroll
-          for (int y = 0; y < 3; ++y) {
+          for (int y = 0; y < N; ++y) {
             D[x][y] += y == 1 ? b[x][y] : -b[x][y];
             b[x][y] = 0.;
           }
       }
       if (i == ie) {
 #pragma unroll
-        for (int x = 0; x < 3; ++x)
+        for (int x = 0; x < N; ++x)
 #pragma unroll
-          for (int y = 0; y < 3; ++y) D[x][y] += y == 1 ? c[x][y] : -c[x][y];
+          for (int y = 0; y < N; ++y) D[x][y] += y == 1 ? c[x][y] : -c[x][y];
       } else {
         // H, g of the row above, from the other warp
         if (e2 == 0) march_sync<2, 64>();
         else march_sync<3, 64>();
 #pragma unroll
-        for (int z = 0; z < 3; ++z) {
-          const double h0 = hg[3 * z * NC], h1 = hg[(3 * z + 1) * NC], h2 = hg[(3 * z + 2) * NC];
-          const double gz = hg[(9 + z) * NC];
+        for (int z = 0; z < N; ++z) {
+          double hz[N];
 #pragma unroll
-          for (int x = 0; x < 3; ++x) {
-            D[x][0] -= c[x][z] * h0;
-            D[x][1] -= c[x][z] * h1;
-            D[x][2] -= c[x][z] * h2;
+          for (int y = 0; y < N; ++y) hz[y] = hg[(N * z + y) * NC];
+          const double gz = hg[(N * N + z) * NC];
+#pragma unroll
+          for (int x = 0; x < N; ++x) {
+#pragma unroll
+            for (int y = 0; y < N; ++y) D[x][y] -= c[x][z] * hz[y];
             v[x] += c[x][z] * gz;
           }
         }
       }
-      // adjugate over the determinant, as inv(M<3>)
-      double K[3][3];
-      K[0][0] = D[1][1] * D[2][2] - D[1][2] * D[2][1];
-      K[1][0] = D[1][2] * D[2][0] - D[1][0] * D[2][2];
-      K[2][0] = D[1][0] * D[2][1] - D[1][1] * D[2][0];
-      K[0][1] = D[0][2] * D[2][1] - D[0][1] * D[2][2];
-      K[1][1] = D[0][0] * D[2][2] - D[0][2] * D[2][0];
-      K[2][1] = D[0][1] * D[2][0] - D[0][0] * D[2][1];
-      K[0][2] = D[0][1] * D[1][2] - D[0][2] * D[1][1];
-      K[1][2] = D[0][2] * D[1][0] - D[0][0] * D[1][2];
-      K[2][2] = D[0][0] * D[1][1] - D[0][1] * D[1][0];
-      const double id = march_rcp(D[0][0] * K[0][0] + D[0][1] * K[1][0] + D[0][2] * K[2][0]);
-      double h[kMarchH];
+      double h[NH];
+      if constexpr (N == 3) {
+        // adjugate over the determinant, as inv(M<3>)
+        double K[3][3];
+        K[0][0] = D[1][1] * D[2][2] - D[1][2] * D[2][1];
+        K[1][0] = D[1][2] * D[2][0] - D[1][0] * D[2][2];
+        K[2][0] = D[1][0] * D[2][1] - D[1][1] * D[2][0];
+        K[0][1] = D[0][2] * D[2][1] - D[0][1] * D[2][2];
+        K[1][1] = D[0][0] * D[2][2] - D[0][2] * D[2][0];
+        K[2][1] = D[0][1] * D[2][0] - D[0][0] * D[2][1];
+        K[0][2] = D[0][1] * D[1][2] - D[0][2] * D[1][1];
+        K[1][2] = D[0][2] * D[1][0] - D[0][0] * D[1][2];
+        K[2][2] = D[0][0] * D[1][1] - D[0][1] * D[1][0];
+        const double id = march_rcp(D[0][0] * K[0][0] + D[0][1] * K[1][0] + D[0][2] * K[2][0]);
 #pragma unroll
-      for (int x = 0; x < 3; ++x) {
+        for (int x = 0; x < 3; ++x) {
 #pragma unroll
-        for (int y = 0; y < 3; ++y)
-          h[3 * x + y] = (K[x][0] * b[0][y] + K[x][1] * b[1][y] + K[x][2] * b[2][y]) * id;
-        h[9 + x] = (K[x][0] * v[0] + K[x][1] * v[1] + K[x][2] * v[2]) * id;
+          for (int y = 0; y < 3; ++y)
+            h[3 * x + y] = (K[x][0] * b[0][y] + K[x][1] * b[1][y] + K[x][2] * b[2][y]) * id;
+          h[9 + x] = (K[x][0] * v[0] + K[x][1] * v[1] + K[x][2] * v[2]) * id;
+        }
+      } else {
+        // D = L U in place, then the N columns of b' and v through L and U.
+        // No pivoting: up to a diagonal scaling, which elimination does not
+        // feel, D is a multiple of the identity plus |A| (no negative
+        // eigenvalue) plus the antisymmetric part of the flux differences, so
+        // its pivots do not vanish
+        double rp[N];
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+          rp[q] = march_rcp(D[q][q]);
+#pragma unroll
+          for (int x = q + 1; x < N; ++x) {
+            D[x][q] *= rp[q];
+#pragma unroll
+            for (int y = q + 1; y < N; ++y) D[x][y] -= D[x][q] * D[q][y];
+          }
+        }
+#pragma unroll
+        for (int y = 0; y <= N; ++y) {
+          double r[N];
+#pragma unroll
+          for (int x = 0; x < N; ++x) {
+            r[x] = y < N ? b[x][y < N ? y : 0] : v[x];
+#pragma unroll
+            for (int q = 0; q < x; ++q) r[x] -= D[x][q] * r[q];
+          }
+#pragma unroll
+          for (int x = N - 1; x >= 0; --x) {
+#pragma unroll
+            for (int q = x + 1; q < N; ++q) r[x] -= D[x][q] * r[q];
+            r[x] *= rp[x];
+            h[y < N ? N * x + y : N * N + x] = r[x];
+          }
+        }
       }
 #pragma unroll
-      for (int e = 0; e < kMarchH; ++e) hg[e * NC] = h[e];
+      for (int e = 0; e < NH; ++e) hg[e * NC] = h[e];
       if (t < nc1) {
         if (e2 == 0) march_arrive<3, 64>();
         else march_arrive<2, 64>();
       }
-      double *so = scrh + (int64_t)(i - is) * kMarchH * NC + lane;
+      double *so = scrh + (int64_t)(i - is) * NH * NC + lane;
 #pragma unroll
-      for (int e = 0; e < kMarchH; ++e) so[e * NC] = h[e];
+      for (int e = 0; e < NH; ++e) so[e * NC] = h[e];
     };
     march_sync<0, NTA>();
     march_sync<0, NTA>();  // phase 3 of chunk 0
@@ -745,14 +796,14 @@ __global__ void __launch_bounds__((C + 2) * 32, 2)
   march_sync<0, NTA>();
   const int nq = (ie - 2) / UP + 1;
   double *ub = sm + P::u, *spb = sm + P::sp, *hb = sm + P::h, *xs = sm + P::x + lane;
-  constexpr int UC = UP * NV * NC, SC = UP * NY * NC, HC = UP * kMarchH * NC;
+  constexpr int UC = UP * NV * NC, SC = UP * NY * NC, HC = UP * NH * NC;
   auto fetch_up = [&](int q) {  // by one lane
     if (q >= nq) return;
     uint64_t *mb = mbar + 2 + (q & 3);
     const int lo = 2 + UP * q, i0 = max(lo, is), i1 = min(lo + UP - 1, ie);
-    const uint32_t hbytes = (i1 - i0 + 1) * kMarchH * NC * 8;
+    const uint32_t hbytes = (i1 - i0 + 1) * NH * NC * 8;
     mbar_expect_tx(mb, hbytes + (bulk ? (UC + SC) * 8 : 0));
-    bulk_g2s(hb + (q & 3) * HC + (i0 - lo) * kMarchH * NC, scrh + (int64_t)(i0 - is) * kMarchH * NC,
+    bulk_g2s(hb + (q & 3) * HC + (i0 - lo) * NH * NC, scrh + (int64_t)(i0 - is) * NH * NC,
              hbytes, mb);
     if (bulk) {
       march_tma_load(ub + (q & 3) * UC, &maps.u, lo, j0, k0, 0, pan, mb);
@@ -765,7 +816,8 @@ __global__ void __launch_bounds__((C + 2) * 32, 2)
     constexpr int HALVES = C / UP;
     const int lev = warp / HALVES, half = HALVES == 2 ? warp % 2 : -1;
     constexpr int N0 = NY > 0 ? 2 * NY + 2 : 1;  // values of the densities' half
-    constexpr int NL = HALVES == 2 ? (N0 > 6 ? N0 : 6) : N0 + 6;
+    constexpr int N1 = NT + 4;                        // and of the momenta and energy
+    constexpr int NL = HALVES == 2 ? (N0 > N1 ? N0 : N1) : N0 + N1;
     double cur[NL], nxt[NL];
     // scratch of the update: du and the sum of the densities, then u1
     auto load_scr = [&](int q, double *v) {
@@ -775,16 +827,15 @@ __global__ void __launch_bounds__((C + 2) * 32, 2)
       int x = 0;
       if (half != 1) {
 #pragma unroll
-        for (int n = 1; n <= NY; ++n) v[x++] = si[(1 + n) * NC];
-        if constexpr (NY > 0) v[x++] = si[(2 + NY) * NC];
+        for (int n = 0; n <= NY - (NY > 0 ? 0 : 1); ++n) v[x++] = si[(NT + n) * NC];
         if (stage != 0)
 #pragma unroll
           for (int n = 0; n <= NY; ++n) v[x + n] = si[(ND + n) * NC];
         x += NY + 1;
       }
       if (half != 0) {
-        v[x++] = si[0];
-        v[x++] = si[NC];
+#pragma unroll
+        for (int n = 0; n < NT; ++n) v[x++] = si[n * NC];
         if (stage != 0)
 #pragma unroll
           for (int n = 0; n < 4; ++n) v[x + n] = si[(ND + S::IVX + n) * NC];
@@ -836,7 +887,7 @@ __global__ void __launch_bounds__((C + 2) * 32, 2)
       if (q >= 0 && q < nq && i >= is && i <= ie) {
         if (bulk) wait(2 + (q & 3), (q >> 2) & 1);
         double *uc = ub + (q & 3) * UC;
-        const double *xi = xs + (q & 1) * UP * 3 * NC + lev * 3 * NC;
+        const double *xi = xs + (q & 1) * UP * N * NC + lev * N * NC;
         double *s1 = scr + (int64_t)(i - is) * NCOMP * NC + ND * NC + lane;
         // slots n0 .. n0 + NN - 1: their increments dv, and u1 as loaded
         auto update = [&](auto nn, int n0, const double *dv, const double *u1) {
@@ -870,9 +921,10 @@ __global__ void __launch_bounds__((C + 2) * 32, 2)
           update(std::integral_constant<int, NY + 1>(), 0, dv, cur + (NY > 0 ? NY + 1 : 0));
         }
         if (half != 0) {
-          const double *cm = cur + (half == 1 ? 0 : NL - 6);
-          const double dv[4] = {xi[NC], cm[0], cm[1], xi[2 * NC]};
-          update(std::integral_constant<int, 4>(), S::IVX, dv, cm + 2);
+          const double *cm = cur + (HALVES == 2 ? 0 : NL - N1);
+          const double dv[4] = {xi[NC], NT ? cm[0] : xi[2 * NC], NT ? cm[1] : xi[3 * NC],
+                                xi[(N - 1) * NC]};
+          update(std::integral_constant<int, 4>(), S::IVX, dv, cm + NT);
         }
       }
       if (q >= 0) {
@@ -899,24 +951,28 @@ __global__ void __launch_bounds__((C + 2) * 32, 2)
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   } else {
-    double x[3] = {0., 0., 0.};
+    double x[N];
+#pragma unroll
+    for (int a = 0; a < N; ++a) x[a] = 0.;
     for (int q = -1; q <= nq; ++q) {
       if (q + 1 < nq) {
         wait(2 + ((q + 1) & 3), ((q + 1) >> 2) & 1);
-        double *xo = xs + ((q + 1) & 1) * UP * 3 * NC;
+        double *xo = xs + ((q + 1) & 1) * UP * N * NC;
         const double *hc = hb + ((q + 1) & 3) * HC + lane;
 #pragma unroll
         for (int o = 0; o < UP; ++o) {
           const int i = 2 + UP * (q + 1) + o;
           if (i < is || i > ie) continue;
-          double y[3];
+          double y[N];
 #pragma unroll
-          for (int a = 0; a < 3; ++a)
-            y[a] = hc[(o * kMarchH + 9 + a) * NC] + (hc[(o * kMarchH + 3 * a) * NC] * x[0] +
-                                                     hc[(o * kMarchH + 3 * a + 1) * NC] * x[1] +
-                                                     hc[(o * kMarchH + 3 * a + 2) * NC] * x[2]);
+          for (int a = 0; a < N; ++a) {
+            y[a] = 0.;
 #pragma unroll
-          for (int a = 0; a < 3; ++a) xo[(o * 3 + a) * NC] = x[a] = y[a];
+            for (int e = 0; e < N; ++e) y[a] += hc[(o * NH + N * a + e) * NC] * x[e];
+            y[a] += hc[(o * NH + N * N + a) * NC];
+          }
+#pragma unroll
+          for (int a = 0; a < N; ++a) xo[(o * N + a) * NC] = x[a] = y[a];
         }
       }
       march_sync<0, NTA>();
@@ -943,7 +999,7 @@ inline PFN_cuTensorMapEncodeTiled march_encoder() {
 }
 
 // launcher for one NY (instantiated in march_ny*.cu)
-template <int NY>
+template <int NY, int N>
 int run_x1march(const Geom &g, const canoe_thermo_t &th, int recon, int rs, int prec,
                 const double *w, const double *du, double *u, const double *dtp, const Stage &s,
                 int stage, cudaStream_t st) {
@@ -982,9 +1038,9 @@ int run_x1march(const Geom &g, const canoe_thermo_t &th, int recon, int rs, int 
     CB_CUDA(cudaGetLastError());
     return 0;
   };
-#define CB_MK(RC, RSV, R, GEO)                                                               \
-  go(k_x1march<NY, RC, RSV, R, GEO, march_chunk<R>(NY)>, make_mix<R>(th), march_chunk<R>(NY), \
-     MarchSmem<5 + NY, march_chunk<R>(NY), R, GEO>::bytes(g.nc1))
+#define CB_MK(RC, RSV, R, GEO)                                            \
+  go(k_x1march<NY, RC, RSV, R, GEO, march_chunk<R>(NY), N>, make_mix<R>(th), \
+     march_chunk<R>(NY), MarchSmem<5 + NY, march_chunk<R>(NY), R, GEO, N>::bytes(g.nc1))
   if (g.shell) {
     if constexpr (NY == 0) {
       if (!hllc) {

@@ -1,8 +1,8 @@
-// march_ny0.cu -- instantiation of the column march for NY = 0
+// march_ny0.cu -- instantiation of the column march for NY = 0, 3x3 blocks
 #include "march.cuh"
 
 namespace cb {
-template int run_x1march<0>(const Geom &, const canoe_thermo_t &, int, int, int, const double *,
-                            const double *, double *, const double *, const Stage &, int,
-                            cudaStream_t);
+template int run_x1march<0, 3>(const Geom &, const canoe_thermo_t &, int, int, int,
+                               const double *, const double *, double *, const double *,
+                               const Stage &, int, cudaStream_t);
 }  // namespace cb

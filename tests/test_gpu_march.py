@@ -63,6 +63,27 @@ def test_march_step_matches_oracle(nx1, nx2, nx3, recon, rs, ny):
     assert g.error_word() == 0
 
 
+# the 5x5 correction: 1e-10 as its pin to the reference's own code (tests/test_ref_pin.py), whose
+# two Gauss-Jordan inverses already differ by 1e-11
+@pytest.mark.parametrize("nx1,nx2,nx3", [(4, 32, 33), (7, 35, 30), (34, 33, 34), (61, 1031, 1)])
+@pytest.mark.parametrize("recon,rs,ny", [(RECON_PPM, RS_HLLC, 3), (RECON_PLM, RS_LMARS, 0)])
+def test_march_full_correction_matches_oracle(nx1, nx2, nx3, recon, rs, ny):
+    from oracle import oracle
+    th = thermo.earth_moist() if ny else thermo.dry()
+    p = problems.moist3d(nx1=nx1, nx2=nx2, nx3=nx3, x1max=250.0 * nx1, x2max=250.0 * nx2,
+                         x3max=250.0 * nx3, th=th, recon=recon, rsolver=rs, satadj=0,
+                         implicit_flag=9)
+    _perturbed(p, 8)
+    g, o = MeshBlock(p), oracle.OracleBlock(p, roundtrip=False)
+    g.step(0.2)
+    o.step(0.2)
+    assert _rel(p, g.conserved(), o.conserved(), 0.2) < 1e-10
+    p.cfg.precision = FP32_PERTURBATION
+    m = MeshBlock(p)
+    m.step(0.2)
+    assert _rel(p, m.conserved(), o.conserved(), 0.2) < 1e-5
+
+
 @pytest.mark.parametrize("bc", [(BC_OUTFLOW, BC_OUTFLOW), (BC_REFLECT, BC_OUTFLOW),
                                 (BC_OUTFLOW, BC_REFLECT)])
 def test_march_outflow_walls(bc):
@@ -110,10 +131,10 @@ def test_march_by_stages_on_a_stream_and_by_graph():
     assert np.array_equal(a.conserved(), b.conserved())
 
 
-@pytest.mark.parametrize("nx1,nside", [(10, 32), (13, 34)])
-def test_march_shell_matches_oracle(nx1, nside):
+@pytest.mark.parametrize("nx1,nside,flag", [(10, 32, 1), (13, 34, 1), (12, 16, 9), (15, 14, 9)])
+def test_march_shell_matches_oracle(nx1, nside, flag):
     from oracle import oracle
-    p = problems.shell_c3(nx1=nx1, nside=nside)
+    p = problems.shell_c3(nx1=nx1, nside=nside, implicit_flag=flag)
     g, o = Shell(p), oracle.OracleShell(p)
     g.step(30.0)
     o.step(30.0)
@@ -122,4 +143,4 @@ def test_march_shell_matches_oracle(nx1, nside):
         s = np.linalg.norm(b[:, n])
         if 1 <= n <= 3:
             s = max(s, 30.0 * 24.79 * np.linalg.norm(b[:, 0]))
-        assert np.linalg.norm(a[:, n] - b[:, n]) <= 5e-11 * s
+        assert np.linalg.norm(a[:, n] - b[:, n]) <= (5e-11 if flag == 1 else 1e-10) * s
