@@ -56,12 +56,12 @@ constexpr int kMarchCols = 32;  // columns per CTA
 constexpr int kMarchUp = 4;     // levels per chunk of the way back up
 // Fewest columns that march.  A tile takes the same time alone on an SM as
 // beside another, so up to 148 tiles (4736 columns) the march takes as long as
-// for one: 128 levels 135 us in FP32, 250 us in FP64, where the CTA-per-column
+// for one: 128 levels 126 us in FP32, 236 us in FP64, where the CTA-per-column
 // kernel takes 38 and 46 ns a column.
-constexpr int kMarchMinCols32 = 3800, kMarchMinCols64 = 6000;
-// with 5x5 blocks one tile fills an SM: 134 us a round of 148 tiles at 64 levels
-// against 127 ns a column
-constexpr int kMarchMinCols5 = 1100;
+constexpr int kMarchMinCols32 = 3500, kMarchMinCols64 = 5500;
+// with 5x5 blocks one tile fills an SM: 128 levels 227 us a round of 148 tiles
+// against 188 ns a column
+constexpr int kMarchMinCols5 = 1200;
 
 // scratch per level of a tile with N x N blocks: H and g (a tile's levels
 // contiguous); then du of the two transverse momenta (N = 3, whose solve
@@ -121,12 +121,13 @@ struct MarchSmem {
   static constexpr int hg = aj + rsz(RR * NAJ * NC);  // [NH][32] H, g of the last row
   static constexpr int NH = march_h(N);
   static constexpr int total1 = hg + NH * NC;
-  // way back up, chunks q & 3: u, species of w, H and g, and x of two chunks
+  // way back up: u and the species of w of four chunks, H and g of five, and x
+  // of two
   static constexpr int UP = kMarchUp;
   static constexpr int u = 0;                    // [4][NV][32][UP], swizzled
   static constexpr int sp = u + 4 * UP * NV * NC;  // [4][ny][32][UP], swizzled
-  static constexpr int h = sp + 4 * UP * ny * NC;  // [4][UP][NH][32]
-  static constexpr int x = h + 4 * UP * NH * NC;   // [2][UP][N][32]
+  static constexpr int h = sp + 4 * UP * ny * NC;  // [5][UP][NH][32]
+  static constexpr int x = h + 5 * UP * NH * NC;   // [2][UP][N][32]
   static constexpr int total2 = x + 2 * UP * N * NC;
   static constexpr int total = total1 > total2 ? total1 : total2;
   // the levels' dx follow at `total`
@@ -207,7 +208,9 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
   constexpr bool PERT = sizeof(R) == 4;
   constexpr int NTP = C * 32, NTA = NTP + 64;
   extern __shared__ __align__(1024) double sm[];
-  __shared__ __align__(8) uint64_t mbar[6];  // w, du, four chunks of the way up
+  // w, du; of the way back up u and species (4 chunks), H and g (5)
+  constexpr int MU = 2, MH = 6, NMB = 11;
+  __shared__ __align__(8) uint64_t mbar[NMB];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nc1 = g.nc1, is = g.is, ie = g.ie;
   const bool bulk = g.bulk != 0;
@@ -242,8 +245,10 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
   double *sdx = sm + P::total;  // dx1f
   const int last_m = nc1 / C;  // rows lag the levels by four: t = nc1 ends them
 
-  // a bounded wait that gave up is reported once; the tile then runs on
-  // without waiting (its values are lost, nothing hangs)
+  // The elimination warps, which have time to spare, wait for the copies; the
+  // barrier that they then join hands the data to the level warps.  A bounded
+  // wait that gave up is reported once; the tile then runs on without waiting
+  // (its values are lost, nothing hangs).
   bool ok = true;
   auto wait = [&](int q, uint32_t parity) {
     if (ok && !mbar_wait(mbar + q, parity)) {
@@ -253,7 +258,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
   };
   constexpr uint32_t kBoxBytes = C * NV * NC * 8;
   if (leader) {
-    for (int q = 0; q < 6; ++q) mbar_init(mbar + q, 1);
+    for (int q = 0; q < NMB; ++q) mbar_init(mbar + q, 1);
     fence_mbar_init();
   }
   for (int i = threadIdx.x; i < nc1; i += NTA) sdx[i] = g.dx1f[i];
@@ -337,7 +342,6 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
           mbar_expect_tx(mbar + 1, kBoxBytes);
           march_tma_load(db, &maps.du, chunk_lo(m) + 4, j0, k0, 0, pan, mbar + 1);
         }
-        wait(0, m & 1);
       }
       if (t < nc1) {
         double wv[NV];
@@ -502,12 +506,8 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // wR's place takes w
       march_sync<0, NTA>();
       // ---- phase 4: row i, level t - 4
-      if (bulk) {
-        tma_w(m + 1);
-        wait(1, m & 1);
-      } else {
-        reg_load(w, chunk_lo(m + 1));
-      }
+      if (bulk) tma_w(m + 1);
+      else reg_load(w, chunk_lo(m + 1));
       if (t >= 5 && t <= nc1) {
         const int i = nc1 - 1 - (t - 4);
         const double *rd = rawb + wrap(bq + warp - 3) * NR * NC;  // cell i - 1
@@ -775,16 +775,25 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
 #pragma unroll
       for (int e = 0; e < NH; ++e) so[e * NC] = h[e];
     };
+    auto arrived = [&](int q, int m) {  // w (q = 0) or du (1) of chunk m
+      if (bulk && e2 == q) wait(q, m & 1);
+    };
+    arrived(0, 0);
     march_sync<0, NTA>();
-    march_sync<0, NTA>();  // phase 3 of chunk 0
-    march_sync<0, NTA>();  // phase 4 of chunk 0
-    for (int m = 0; m <= last_m; ++m) {
-      for (int p = e2; p < C - 2; p += 2) row(m * C + p);
+    for (int m = -1; m <= last_m; ++m) {
+      if (m >= 0)
+        for (int p = e2; p < C - 2; p += 2) row(m * C + p);
       // all but the chunk's last two rows are done before the next chunk's
       // rows are formed in their places
-      if (m < last_m) march_sync<0, NTA>();  // phase 3 of chunk m + 1
-      row(m * C + C - 2 + e2);
-      if (m < last_m) march_sync<0, NTA>();  // phase 4 of chunk m + 1
+      if (m < last_m) {
+        arrived(1, m + 1);
+        march_sync<0, NTA>();  // phase 3 of chunk m + 1
+      }
+      if (m >= 0) row(m * C + C - 2 + e2);
+      if (m < last_m) {
+        if (m + 2 <= last_m) arrived(0, m + 2);
+        march_sync<0, NTA>();  // phase 4 of chunk m + 1
+      }
     }
   }
 
@@ -797,18 +806,26 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
   const int nq = (ie - 2) / UP + 1;
   double *ub = sm + P::u, *spb = sm + P::sp, *hb = sm + P::h, *xs = sm + P::x + lane;
   constexpr int UC = UP * NV * NC, SC = UP * NY * NC, HC = UP * NH * NC;
-  auto fetch_up = [&](int q) {  // by one lane
+  // by one lane: H and g of chunk q, used first, and the rest of it; what the
+  // level warps read from scratch themselves starts towards L2
+  auto fetch_h = [&](int q) {
     if (q >= nq) return;
-    uint64_t *mb = mbar + 2 + (q & 3);
-    const int lo = 2 + UP * q, i0 = max(lo, is), i1 = min(lo + UP - 1, ie);
-    const uint32_t hbytes = (i1 - i0 + 1) * NH * NC * 8;
-    mbar_expect_tx(mb, hbytes + (bulk ? (UC + SC) * 8 : 0));
-    bulk_g2s(hb + (q & 3) * HC + (i0 - lo) * NH * NC, scrh + (int64_t)(i0 - is) * NH * NC,
-             hbytes, mb);
+    const int lo = 2 + UP * q, i0 = max(lo, is), n = min(lo + UP - 1, ie) - i0 + 1;
+    uint64_t *mb = mbar + MH + q % 5;
+    mbar_expect_tx(mb, n * NH * NC * 8);
+    bulk_g2s(hb + (q % 5) * HC + (i0 - lo) * NH * NC, scrh + (int64_t)(i0 - is) * NH * NC,
+             n * NH * NC * 8, mb);
+  };
+  auto fetch_u = [&](int q) {
+    if (q >= nq) return;
+    const int lo = 2 + UP * q, i0 = max(lo, is), n = min(lo + UP - 1, ie) - i0 + 1;
     if (bulk) {
+      uint64_t *mb = mbar + MU + (q & 3);
+      mbar_expect_tx(mb, (UC + SC) * 8);
       march_tma_load(ub + (q & 3) * UC, &maps.u, lo, j0, k0, 0, pan, mb);
       if constexpr (NY > 0) march_tma_load(spb + (q & 3) * SC, &maps.sp, lo, j0, k0, 1, pan, mb);
     }
+    bulk_prefetch_l2(scr + (int64_t)(i0 - is) * NCOMP * NC, n * NCOMP * NC * 8);
   };
   if (warp < C) {
     // C = 8: two warps per level, one for the densities, one for momenta and
@@ -818,27 +835,27 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     constexpr int N0 = NY > 0 ? 2 * NY + 2 : 1;  // values of the densities' half
     constexpr int N1 = NT + 4;                        // and of the momenta and energy
     constexpr int NL = HALVES == 2 ? (N0 > N1 ? N0 : N1) : N0 + N1;
+    constexpr int OFF1 = HALVES == 2 ? 0 : N0;
     double cur[NL], nxt[NL];
     // scratch of the update: du and the sum of the densities, then u1
     auto load_scr = [&](int q, double *v) {
       const int i = 2 + UP * q + lev;
       if (q >= nq || i < is || i > ie) return;
       const double *si = scr + (int64_t)(i - is) * NCOMP * NC + lane;
-      int x = 0;
       if (half != 1) {
+        constexpr int NM = N0 - NY - 1;  // du of the species and the sum
 #pragma unroll
-        for (int n = 0; n <= NY - (NY > 0 ? 0 : 1); ++n) v[x++] = si[(NT + n) * NC];
+        for (int n = 0; n < NM; ++n) v[n] = si[(NT + n) * NC];
         if (stage != 0)
 #pragma unroll
-          for (int n = 0; n <= NY; ++n) v[x + n] = si[(ND + n) * NC];
-        x += NY + 1;
+          for (int n = 0; n <= NY; ++n) v[NM + n] = si[(ND + n) * NC];
       }
       if (half != 0) {
 #pragma unroll
-        for (int n = 0; n < NT; ++n) v[x++] = si[n * NC];
+        for (int n = 0; n < NT; ++n) v[OFF1 + n] = si[n * NC];
         if (stage != 0)
 #pragma unroll
-          for (int n = 0; n < 4; ++n) v[x + n] = si[(ND + S::IVX + n) * NC];
+          for (int n = 0; n < 4; ++n) v[OFF1 + NT + n] = si[(ND + S::IVX + n) * NC];
       }
     };
     // without TMA, u and the species of w through registers
@@ -885,7 +902,6 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
       if (q >= 0) load_scr(q + 1, nxt);
       const int i = 2 + UP * q + lev;
       if (q >= 0 && q < nq && i >= is && i <= ie) {
-        if (bulk) wait(2 + (q & 3), (q >> 2) & 1);
         double *uc = ub + (q & 3) * UC;
         const double *xi = xs + (q & 1) * UP * N * NC + lev * N * NC;
         double *s1 = scr + (int64_t)(i - is) * NCOMP * NC + ND * NC + lane;
@@ -921,7 +937,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
           update(std::integral_constant<int, NY + 1>(), 0, dv, cur + (NY > 0 ? NY + 1 : 0));
         }
         if (half != 0) {
-          const double *cm = cur + (HALVES == 2 ? 0 : NL - N1);
+          const double *cm = cur + OFF1;
           const double dv[4] = {xi[NC], NT ? cm[0] : xi[2 * NC], NT ? cm[1] : xi[3 * NC],
                                 xi[(N - 1) * NC]};
           update(std::integral_constant<int, 4>(), S::IVX, dv, cm + NT);
@@ -937,15 +953,21 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     }
   } else if (warp == C + 1) {
     // the copies
-    if (lane == 0) fetch_up(0);
+    if (lane == 0) {
+      for (int q = 0; q < 2; ++q) fetch_h(q);
+      fetch_u(0);
+    }
     for (int q = -1; q <= nq; ++q) {
       if (lane == 0) {
+        fetch_h(q + 3);
         if (bulk && q >= 1)
           march_tma_store(&maps.u, 2 + UP * (q - 1), j0, k0, 0, pan, ub + ((q - 1) & 3) * UC);
         // chunk q - 2 has been read out: its place takes chunk q + 2
         asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-        fetch_up(q + 2);
+        fetch_u(q + 2);
       }
+      // for the level warps of the next phase
+      if (bulk && q + 1 < nq) wait(MU + ((q + 1) & 3), ((q + 1) >> 2) & 1);
       __syncwarp();
       march_sync<0, NTA>();
     }
@@ -956,30 +978,33 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     for (int a = 0; a < N; ++a) x[a] = 0.;
     for (int q = -1; q <= nq; ++q) {
       if (q + 1 < nq) {
-        wait(2 + ((q + 1) & 3), ((q + 1) >> 2) & 1);
+        wait(MH + (q + 1) % 5, (q + 1) / 5 & 1);
         double *xo = xs + ((q + 1) & 1) * UP * N * NC;
-        const double *hc = hb + ((q + 1) & 3) * HC + lane;
+        const double *hc = hb + (q + 1) % 5 * HC + lane;
 #pragma unroll
         for (int o = 0; o < UP; ++o) {
           const int i = 2 + UP * (q + 1) + o;
-          if (i < is || i > ie) continue;
+          // (levels outside the column hold what the buffer held: not used)
+          const bool in = i >= is && i <= ie;
           double y[N];
 #pragma unroll
+          for (int a = 0; a < N; ++a) y[a] = hc[(o * NH + N * N + a) * NC];
+#pragma unroll
+          for (int e = 0; e < N; ++e)
+#pragma unroll
+            for (int a = 0; a < N; ++a) y[a] += hc[(o * NH + N * a + e) * NC] * x[e];
+#pragma unroll
           for (int a = 0; a < N; ++a) {
-            y[a] = 0.;
-#pragma unroll
-            for (int e = 0; e < N; ++e) y[a] += hc[(o * NH + N * a + e) * NC] * x[e];
-            y[a] += hc[(o * NH + N * N + a) * NC];
+            x[a] = in ? y[a] : x[a];
+            xo[(o * N + a) * NC] = x[a];
           }
-#pragma unroll
-          for (int a = 0; a < N; ++a) xo[(o * N + a) * NC] = x[a] = y[a];
         }
       }
       march_sync<0, NTA>();
     }
   }
   if (!ok)  // copies still in flight get a second bounded wait
-    for (int q = 0; q < 6; ++q) mbar_wait(mbar + q, 0);
+    for (int q = 0; q < NMB; ++q) mbar_wait(mbar + q, 0);
 }
 
 // the tensor map encoder of the driver (null where there is none)
