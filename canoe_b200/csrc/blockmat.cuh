@@ -223,8 +223,8 @@ __device__ __forceinline__ void abs_jacobian(M<N> &A, const TH &th,
     wl[n] = T(wl_[n]);
     wr[n] = T(wr_[n]);
   }
-  T sqrtdl = sqrt(wl[0]);
-  T sqrtdr = sqrt(wr[0]);
+  T sqrtdl = qsqrt(wl[0]);
+  T sqrtdr = qsqrt(wr[0]);
   T isdlpdr = pdiv(T(1), sqrtdl + sqrtdr);
   prim[0] = sqrtdl * sqrtdr;
   prim[S::IVX] = (sqrtdl * wl[S::IVX] + sqrtdr * wr[S::IVX]) * isdlpdr;

@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(ColPlan<N, PER, GEO>::threads, ColPlan<N, PER,
       __syncthreads();
       for (int i = tid; i < nc1; i += nth) {
         double a = psf[i], b = psf[i + 1];
-        double pv = fabs(a - b) < 1.E-6 ? 0.5 * (a + b) : (a - b) / log(a / b);
+        double pv = fabs(a - b) < 1.E-6 ? 0.5 * (a + b) : qdiv(a - b, log(qdiv(a, b)));
         double feps = 1.;
 #pragma unroll
         for (int n = 1; n <= NY; ++n)
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(ColPlan<N, PER, GEO>::threads, ColPlan<N, PER,
         const bool ob = (i < is && g.bc[0] == CANOE_BC_OUTFLOW);
         const bool ot = (i > ie && g.bc[1] == CANOE_BC_OUTFLOW);
         if (!ob && !ot) {
-          rho[i] = R(pre0[i] / (rho0[i] * gm));
+          rho[i] = R(qdiv(pre0[i], rho0[i] * gm));
           pre[i] = R(pre0[i] - pv);
         }
       }
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(ColPlan<N, PER, GEO>::threads, ColPlan<N, PER,
       }
       const double pf = grav != 0. ? psf[f] : pcst;
       if (grav != 0.) {
-        const double gamma = sqrt(gam[f] * gam[f - 1]);
+        const double gamma = qsqrt(gam[f] * gam[f - 1]);
         if constexpr (PERT) {
           // keep p' relative to psf(f); floor p = psf(f) as the reference does
           R pr = wr[S::IPR], pl = wl[S::IPR];
@@ -385,17 +385,17 @@ __global__ void __launch_bounds__(ColPlan<N, PER, GEO>::threads, ColPlan<N, PER,
           if (R(pf) + pl < R(0)) pl = R(0);
           wr[S::IPR] = pr;
           wl[S::IPR] = pl;
-          wr[0] = (R(pf) + pr) / (wr[0] * R(gamma));
-          wl[0] = (R(pf) + pl) / (wl[0] * R(gamma));
+          wr[0] = qdiv(R(pf) + pr, wr[0] * R(gamma));
+          wl[0] = qdiv(R(pf) + pl, wl[0] * R(gamma));
         } else {
           double pr = wr[S::IPR] + pf;
           if (pr < 0.) pr = pf;
           wr[S::IPR] = pr;
-          wr[0] = pr / (wr[0] * gamma);
+          wr[0] = qdiv(pr, wr[0] * gamma);
           double pl = wl[S::IPR] + pf;
           if (pl < 0.) pl = pf;
           wl[S::IPR] = pl;
-          wl[0] = pl / (wl[0] * gamma);
+          wl[0] = qdiv(pl, wl[0] * gamma);
         }
       }
       return pf;
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(ColPlan<N, PER, GEO>::threads, ColPlan<N, PER,
     // P4
     for (int i = is + tid; i <= ie; i += nth) {
       const int f0 = i - is;
-      const double idx = 1. / g.dx1f[i];
+      const double idx = qdiv(1., g.dx1f[i]);
       // constant x1 acceleration (HydroSourceTerms::ConstantAcceleration
       // with canoe patches/25.constant_acc.patch:35-52): src = dt rho g on
       // the x1 momentum, src v1 on the energy

@@ -404,8 +404,9 @@ __global__ void k_shell_c2p(const double *__restrict__ u, double *__restrict__ w
   double v1 = u_m1 * di, v2 = u_m2 * di, v3 = u_m3 * di;
   const double sth2 = 1. - cth * cth;
   const double a = v2, b = v3;
-  v2 = a / sth2 - b * cth / sth2;
-  v3 = -a * cth / sth2 + b / sth2;
+  const Recip<double> is2(sth2);
+  v2 = is2.of(a) - is2.of(b * cth);
+  v3 = is2.of(-a * cth) + is2.of(b);
   const double e_k = 0.5 * (u_m1 * v1 + u_m2 * v2 + u_m3 * v3);
   const double pr = gm1 * (u_e - e_k);
   const double wv[kNV] = {u_d, v1, v2, v3, pr};
@@ -503,8 +504,8 @@ __device__ __forceinline__ void shell_face_flux(const Geom &g, const canoe_therm
   if (DIR == 1) {
     // PrimToLocal2 with Face2Metric: T22 = 1/sqrt(gi22), T32 = g23/sqrt(g33)
     const double ct = g.shell[kTabCosF2 * nkj + kj], st = g.shell[kTabSinF2 * nkj + kj];
-    const double gi22 = 1.0 / (st * st);
-    const double T22 = 1.0 / sqrt(gi22), T32 = ct / sqrt(1.0), T33 = sqrt(1.0);
+    const double gi22 = qdiv(1.0, st * st), rg = qsqrt(gi22);
+    const double T22 = qdiv(1.0, rg), T32 = ct, T33 = 1.0;
     auto loc = [&](R *x) {
       const R u2 = x[2], u3 = x[3];
       x[2] = R(T22) * u2;
@@ -519,7 +520,7 @@ __device__ __forceinline__ void shell_face_flux(const Geom &g, const canoe_therm
 #pragma unroll
     for (int n = 0; n < kNV; ++n) fx[n] = fr[n];
     if (PERT) fx[2] += pref;
-    const double F22 = sqrt(gi22), F32 = -sqrt(gi22) * ct / 1.0, F33 = 1.0 / sqrt(1.0);
+    const double F22 = rg, F32 = -rg * ct, F33 = 1.0;
     const double txy = fx[2], txz = fx[3];
     fx[2] = F22 * txy;
     fx[3] = F32 * txy + F33 * txz;
@@ -531,8 +532,8 @@ __device__ __forceinline__ void shell_face_flux(const Geom &g, const canoe_therm
     // PrimToLocal3 with Face3Metric: T22 = sqrt(g22), T23 = g23/sqrt(g22),
     // T33 = 1/sqrt(gi33)
     const double ct = g.shell[kTabCosF3 * nkj + kj], st = g.shell[kTabSinF3 * nkj + kj];
-    const double gi33 = 1.0 / (st * st);
-    const double T22 = sqrt(1.0), T23 = ct / sqrt(1.0), T33 = 1.0 / sqrt(gi33);
+    const double gi33 = qdiv(1.0, st * st), rg = qsqrt(gi33);
+    const double T22 = 1.0, T23 = ct, T33 = qdiv(1.0, rg);
     auto loc = [&](R *x) {
       const R u2 = x[2], u3 = x[3];
       x[2] = R(T22) * u2 + R(T23) * u3;
@@ -547,7 +548,7 @@ __device__ __forceinline__ void shell_face_flux(const Geom &g, const canoe_therm
 #pragma unroll
     for (int n = 0; n < kNV; ++n) fx[n] = fr[n];
     if (PERT) fx[3] += pref;
-    const double F22 = 1.0 / sqrt(1.0), F23 = -ct / 1.0 * sqrt(gi33), F33 = sqrt(gi33);
+    const double F22 = 1.0, F23 = -ct * rg, F33 = rg;
     const double txy = fx[2], txz = fx[3];
     fx[2] = F22 * txy + F23 * txz;
     fx[3] = F33 * txz;
@@ -676,7 +677,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2)
     const int kc = DIR == 1 ? o : dc, jc = DIR == 1 ? dc : o;
     const int64_t kj = (int64_t)kc * g.nc2 + jc;
     const double d2 = g.shell[kTabDx2A * nkj + kj], d3 = g.shell[kTabDx3A * nkj + kj];
-    const double vol = df * d2 * d3 * xv * xv * g.shell[kTabSinC * nkj + kj];
+    const Recip<double> ivol(df * d2 * d3 * xv * xv * g.shell[kTabSinC * nkj + kj]);
     double am, ap;
     if (DIR == 1) {
       am = xv * g.shell[kTabDx3AF2 * nkj + kj] * df;
@@ -690,11 +691,11 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2)
     for (int n = 0; n < kNV; ++n) {
       const double dfl = ap * F[n][c + 1][tx] - am * F[n][c][tx];
       if (DIR == 1)
-        du[n * g.sv + off] = -(wght * dfl / vol);
+        du[n * g.sv + off] = -ivol.of(wght * dfl);
       else if (blockDim.y >= TD)
-        du[n * g.sv + off] = dpre[n] - wght * dfl / vol;  // c == ty: the prefetched cell
+        du[n * g.sv + off] = dpre[n] - ivol.of(wght * dfl);  // c == ty: the prefetched cell
       else
-        du[n * g.sv + off] -= wght * dfl / vol;
+        du[n * g.sv + off] -= ivol.of(wght * dfl);
     }
   }
 }
@@ -841,15 +842,15 @@ __global__ void __launch_bounds__(32 * SBY)
         const int kc = DIR == 1 ? o : c - 1, jc = DIR == 1 ? c - 1 : o;
         const int64_t kjc = (int64_t)kc * g.nc2 + jc;
         const double d2 = g.shell[kTabDx2A * nkj + kjc], d3 = g.shell[kTabDx3A * nkj + kjc];
-        const double vol = df * d2 * d3 * xv * xv * g.shell[kTabSinC * nkj + kjc];
+        const Recip<double> ivol(df * d2 * d3 * xv * xv * g.shell[kTabSinC * nkj + kjc]);
         const int64_t off = base + (int64_t)(c - 1) * sd;
 #pragma unroll
         for (int n = 0; n < kNV; ++n) {
           const double dfl = ac * fx[n] - amp * fp[n];
           if (DIR == 1)
-            du[n * g.sv + off] = -(wght * dfl / vol);
+            du[n * g.sv + off] = -ivol.of(wght * dfl);
           else
-            du[n * g.sv + off] = dpre[n] - wght * dfl / vol;
+            du[n * g.sv + off] = dpre[n] - ivol.of(wght * dfl);
         }
       }
 #pragma unroll

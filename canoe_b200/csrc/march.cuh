@@ -56,9 +56,9 @@ constexpr int kMarchCols = 32;  // columns per CTA
 constexpr int kMarchUp = 4;     // levels per chunk of the way back up
 // Fewest columns that march.  A tile takes the same time alone on an SM as
 // beside another, so up to 148 tiles (4736 columns) the march takes as long as
-// for one: 128 levels 126 us in FP32, 236 us in FP64, where the CTA-per-column
+// for one: 128 levels 121 us in FP32, 186 us in FP64, where the CTA-per-column
 // kernel takes 38 and 46 ns a column.
-constexpr int kMarchMinCols32 = 3500, kMarchMinCols64 = 5500;
+constexpr int kMarchMinCols32 = 3400, kMarchMinCols64 = 4300;
 // with 5x5 blocks one tile fills an SM: 128 levels 227 us a round of 148 tiles
 // against 188 ns a column
 constexpr int kMarchMinCols5 = 1200;
@@ -180,17 +180,6 @@ template <int C>
 __device__ __forceinline__ int march_box(int n, int c, int o) {
   if constexpr (C == 8) return (n * kMarchCols + c) * 8 + ((((o >> 1) ^ (c >> 1)) & 3) << 1) + (o & 1);
   else return (n * kMarchCols + c) * 4 + ((((o >> 1) ^ (c >> 2)) & 1) << 1) + (o & 1);
-}
-
-// reciprocal by two Newton-Raphson steps on the hardware's approximation
-// (relative error 2^-20 -> 2^-40 -> below one ulp for normal numbers): no
-// branch for the rare ranges, so that a row's elimination schedules as one
-// block of instructions
-__device__ __forceinline__ double march_rcp(double d) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  r = fma(r, fma(-d, r, 1.), r);
-  return fma(r, fma(-d, r, 1.), r);
 }
 
 template <int NY, int RECON, int RS, typename R, int GEO, int C, int N>
@@ -367,7 +356,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
           }
           psr[(t & (RP - 1)) * NC] = a;
         }
-        const double pv = fabs(a - b) < 1.E-6 ? 0.5 * (a + b) : (a - b) / log(a / b);
+        const double pv = fabs(a - b) < 1.E-6 ? 0.5 * (a + b) : qdiv(a - b, log(qdiv(a, b)));
         double feps = 1.;
 #pragma unroll
         for (int n = 1; n <= NY; ++n)
@@ -375,7 +364,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
         const double gmv = th.rd * feps;
         gmr[wrap(bq + warp) * NC] = gmv;
         R *qo = qb + wrap(bq + warp) * NV * NC;
-        qo[0] = R(wv[S::IPR] / (wv[0] * gmv));
+        qo[0] = R(qdiv(wv[S::IPR], wv[0] * gmv));
         qo[S::IPR * NC] = R(wv[S::IPR] - pv);
 #pragma unroll
         for (int n = 1; n < NV - 1; ++n) qo[n * NC] = R(wv[n]);
@@ -470,24 +459,24 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
           wr[n] = fo[n * NC];
         }
         const double pf = psr[((t - 3) & (RP - 1)) * NC];
-        const double gamma = sqrt(gmr[wrap(bq + warp - 3) * NC] * gmr[wrap(bq + warp - 2) * NC]);
+        const double gamma = qsqrt(gmr[wrap(bq + warp - 3) * NC] * gmr[wrap(bq + warp - 2) * NC]);
         if constexpr (PERT) {
           R pr = wr[S::IPR], pl = wl[S::IPR];
           if (R(pf) + pr < R(0)) pr = R(0);
           if (R(pf) + pl < R(0)) pl = R(0);
           wr[S::IPR] = pr;
           wl[S::IPR] = pl;
-          wr[0] = (R(pf) + pr) / (wr[0] * R(gamma));
-          wl[0] = (R(pf) + pl) / (wl[0] * R(gamma));
+          wr[0] = qdiv(R(pf) + pr, wr[0] * R(gamma));
+          wl[0] = qdiv(R(pf) + pl, wl[0] * R(gamma));
         } else {
           double pr = wr[S::IPR] + pf;
           if (pr < 0.) pr = pf;
           wr[S::IPR] = pr;
-          wr[0] = pr / (wr[0] * gamma);
+          wr[0] = qdiv(pr, wr[0] * gamma);
           double pl = wl[S::IPR] + pf;
           if (pl < 0.) pl = pf;
           wl[S::IPR] = pl;
-          wl[0] = pl / (wl[0] * gamma);
+          wl[0] = qdiv(pl, wl[0] * gamma);
         }
         if constexpr (GEO) {
           if constexpr (PERT) hllc_pert<R, NY, 0, true>(mx, wl, wr, R(pf), fx, R(cosc));
@@ -527,6 +516,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
             const double a1m = d2 * d3 * g.x1f[i] * g.x1f[i] * sc;
             const double a1p = d2 * d3 * g.x1f[i + 1] * g.x1f[i + 1] * sc;
             const double vol = df * d2 * d3 * xv * xv * sc;
+            const Recip<double> ivol(vol), ixv(xv), ia(a1m);
             const double a2m = xv * tab(kTabDx3AF2, k, j) * df;
             const double a2p = xv * tab(kTabDx3AF2, k, j + 1) * df;
             const double a3m = xv * tab(kTabDx2AF3, k, j) * df;
@@ -536,18 +526,18 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
             const double pr = ru[NC];
             const double v_2 = v2 + v3 * cs, v_3 = v3 + v2 * cs, sine2 = sc * sc;
             const double x_ov_rD =
-                (a2m * tab(kTabSinF2, k, j) - a2p * tab(kTabSinF2, k, j + 1)) / vol;
+                ivol.of(a2m * tab(kTabSinF2, k, j) - a2p * tab(kTabSinF2, k, j + 1));
             const double y_ov_rC =
-                (a3m * tab(kTabSinF3, k, j) - a3p * tab(kTabSinF3, k + 1, j)) / vol;
+                ivol.of(a3m * tab(kTabSinF3, k, j) - a3p * tab(kTabSinF3, k + 1, j));
             double csrc[3];
-            csrc[0] = wght * ((2.0 * pr + rho * (v2 * v_2 + v3 * v_3)) / xv);
-            csrc[1] = wght * (-x_ov_rD * (pr + rho * v3 * v3 * sine2) - rho * v1 * v_2 / xv);
-            csrc[2] = wght * (-y_ov_rC * (pr + rho * v2 * v2 * sine2) - rho * v1 * v_3 / xv);
+            csrc[0] = wght * ixv.of(2.0 * pr + rho * (v2 * v_2 + v3 * v_3));
+            csrc[1] = wght * (-x_ov_rD * (pr + rho * v3 * v3 * sine2) - ixv.of(rho * v1 * v_2));
+            csrc[2] = wght * (-y_ov_rC * (pr + rho * v2 * v2 * sine2) - ixv.of(rho * v1 * v_3));
 #pragma unroll
             for (int n = 0; n < NV; ++n) {
               double dfl = a1p * (double)fhi[n * NC] - a1m * (double)flo[n * NC];
               if (PERT && n == S::IVX) dfl += a1p * phi - a1m * plo;
-              double v = -(wght * dfl / vol);
+              double v = -ivol.of(wght * dfl);
               if (n == S::IVX) v += csrc[0];
               if (n == S::IVY) v += csrc[1];
               if (n == S::IVZ) v += csrc[2];
@@ -555,10 +545,10 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
               if (n == S::IPR) v += gsrc * v1;
               dv[n] = v;
             }
-            dd = idt * (2. * vol / a1m);
-            ra = a1p / a1m;
+            dd = idt * ia.of(2. * vol);
+            ra = ia.of(a1p);
           } else {
-            const double idx = 1. / sdx[i];
+            const double idx = qdiv(1., sdx[i]);
 #pragma unroll
             for (int n = 0; n < NV; ++n) {
               double d = ((double)fhi[n * NC] - (double)flo[n * NC]) * idx;
@@ -722,7 +712,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
         K[0][2] = D[0][1] * D[1][2] - D[0][2] * D[1][1];
         K[1][2] = D[0][2] * D[1][0] - D[0][0] * D[1][2];
         K[2][2] = D[0][0] * D[1][1] - D[0][1] * D[1][0];
-        const double id = march_rcp(D[0][0] * K[0][0] + D[0][1] * K[1][0] + D[0][2] * K[2][0]);
+        const double id = Recip<double>(D[0][0] * K[0][0] + D[0][1] * K[1][0] + D[0][2] * K[2][0]).r;
 #pragma unroll
         for (int x = 0; x < 3; ++x) {
 #pragma unroll
@@ -739,7 +729,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
         double rp[N];
 #pragma unroll
         for (int q = 0; q < N; ++q) {
-          rp[q] = march_rcp(D[q][q]);
+          rp[q] = Recip<double>(D[q][q]).r;
 #pragma unroll
           for (int x = q + 1; x < N; ++x) {
             D[x][q] *= rp[q];

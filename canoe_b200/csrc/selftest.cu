@@ -188,3 +188,46 @@ extern "C" int canoe_measure_fma_peak(int fp32, double *h_tflops) {
   }
   return fp32 ? fma_peak<float>(1 << 17, h_tflops) : fma_peak<double>(1 << 14, h_tflops);
 }
+
+// ---------------------------------------------------------------------------
+// The branch-free division and square root of physics.cuh on host operands.
+
+namespace cb {
+namespace {
+
+template <typename R>
+__global__ void k_fastmath(const double *__restrict__ a, const double *__restrict__ b,
+                           double *__restrict__ out, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const R x = R(a[i]);
+  out[i] = b ? double(qdiv(x, R(b[i]))) : double(qsqrt(x));
+}
+
+}  // namespace
+}  // namespace cb
+
+extern "C" int canoe_selftest_fastmath(int fp32, const double *h_a, const double *h_b,
+                                       double *h_out, int n) {
+  using namespace cb;
+  if (!h_a || !h_out || n < 1) {
+    set_error("canoe_selftest_fastmath: operands and a result pointer");
+    return CANOE_ERR_ARG;
+  }
+  const size_t bytes = (size_t)n * sizeof(double);
+  double *d = nullptr;
+  CB_CUDA(cudaMalloc(&d, 3 * bytes));
+  double *da = d, *db = h_b ? d + n : nullptr, *dout = d + 2 * (size_t)n;
+  cudaError_t e = cudaMemcpy(da, h_a, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && h_b) e = cudaMemcpy(db, h_b, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    const unsigned nb = (unsigned)((n + 255) / 256);
+    if (fp32) k_fastmath<float><<<nb, 256>>>(da, db, dout, n);
+    else k_fastmath<double><<<nb, 256>>>(da, db, dout, n);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(h_out, dout, bytes, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  CB_CUDA(e);
+  return 0;
+}

@@ -171,6 +171,13 @@ int canoe_selftest_bounded_wait(int spins, int complete, uint32_t *h_bits);
  * both cases.  No reference counterpart. */
 int canoe_selftest_umma_wait(int spins, int issue, uint32_t *h_bits);
 
+/* Self-test of the kernels' branch-free division and square root: n host
+ * operands (rounded to FP32 first when fp32 != 0), h_out[i] = h_a[i] / h_b[i],
+ * or sqrt(h_a[i]) when h_b is NULL.  Operands and results in the normal range.
+ * No reference counterpart. */
+int canoe_selftest_fastmath(int fp32, const double *h_a, const double *h_b, double *h_out,
+                            int n);
+
 /* Measured non-tensor FMA throughput of the current GPU in TFLOP/s (2 flops
  * per FMA): FP64 (fp32 == 0) or FP32, eight independent chains per thread on
  * every SM, timed with CUDA events after a warm-up launch.  The denominator
