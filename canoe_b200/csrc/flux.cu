@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(32 * RBY)
   if (i > g.ie || o > (DIR == 1 ? g.ke : g.je)) return;
   const int dlo = DIR == 1 ? g.js : g.ks;
   const int dhi = DIR == 1 ? g.je : g.ke;
-  const int RL = g.flux_run > 0 ? g.flux_run : run_len<R>();
+  const int RL = g.flux_run;
   const int s0 = dlo + blockIdx.z * RL;
   const int s1 = min(s0 + RL, dhi + 1);  // one past the run's last cell
   const int64_t sd = DIR == 1 ? g.nc1 : g.sk;
@@ -294,6 +294,9 @@ __global__ void __launch_bounds__(32 * RBY)
   }
 }
 
+// warps below which the default runs get shorter: four per SM
+constexpr int kRunMinWarps = 4 * 148;
+
 // 1: the x2 / x3 fluxes run as k_flux_x23_run, 0: as the tile kernel
 constexpr int kFluxRun = 1;
 
@@ -308,14 +311,24 @@ int run_x23(const Geom &g, const canoe_thermo_t &th, const double *w, double *du
             const double *dtp, double beta, double *fo, cudaStream_t st) {
   const int nd = DIR == 1 ? g.nx2 : g.nx3;
   const int no = DIR == 1 ? g.nx3 : g.nx2;
-  const int RL = g.flux_run > 0 ? g.flux_run : run_len<R>();
+  // a small block's default runs leave the chip idle while each thread marches
+  // its cells one latency after another (32x16x16 in FP32: 16 warps, 31 us):
+  // its runs are halved, at two extra cells a run, until there are four warps
+  // per SM or two cells per run (13 us)
+  int RL = g.flux_run;
+  if (RL <= 0)
+    for (RL = run_len<R>();
+         RL > 2 && (int64_t)((g.nx1 + 31) / 32) * no * ((nd + RL - 1) / RL) < kRunMinWarps;)
+      RL /= 2;
   // a 2-D block (one line across the flux direction) keeps the tile kernel:
   // its runs would fill one warp in four of each CTA, and the 150 x 100
   // bubble would march 20 warps in all (x2 pass 4 x slower than the tiles);
   // thin 3-D blocks keep the runs, whose launches overlap in a batch
   if (kFluxRun != 0 && no >= RBY) {
     dim3 grid((g.nx1 + 31) / 32, (no + RBY - 1) / RBY, (nd + RL - 1) / RL);
-    k_flux_x23_run<NY, RECON, RS, DIR, WF, R><<<grid, dim3(32, RBY), 0, st>>>(g, th, w, du, dtp,
+    Geom gr = g;
+    gr.flux_run = RL;
+    k_flux_x23_run<NY, RECON, RS, DIR, WF, R><<<grid, dim3(32, RBY), 0, st>>>(gr, th, w, du, dtp,
                                                                               beta, fo);
     CB_CUDA(cudaGetLastError());
     return 0;
