@@ -37,7 +37,7 @@ size_t march_doubles(const Geom &g, const canoe_thermo_t &th, int flag, int prec
   const int n = flag & 8 ? 5 : 3;
   const int least = n == 5 ? kMarchMinCols5
                            : (prec == CANOE_FP32_PERTURBATION ? kMarchMinCols32 : kMarchMinCols64);
-  if (ncol < least) return 0;
+  if (ncol < least || !march_available()) return 0;
   // columns too long for the CTA-per-column kernel stay refused there
   if (sizeof(double) * col_smem(g.nv, g.nc1, g.nx1, n, 0, 1).total > 227 * 1024) return 0;
   return march_scratch_doubles(th.ny, n, g.nx1, g.nx2, g.nx3, g.npanel > 1 ? g.npanel : 1);

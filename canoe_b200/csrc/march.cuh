@@ -32,8 +32,10 @@
 // in memory.  TMA moves them: a box of C levels x 32 columns x NV variables
 // per request (a probe of the access pattern on w of 128x256x256: 5.9 TB/s,
 // 3.0 TB/s with cp.async, 4.5 TB/s with loads and shared-memory stores).  A
-// tensor map needs rows of a multiple of 16 bytes, so columns of an odd
-// number of levels go through registers instead (g.bulk = 0).
+// tensor map needs rows of a multiple of 16 bytes: for columns of an odd number
+// of levels (g.bulk = 0) the map's rows are pairs of columns, and a request
+// takes every second column of one variable from the 16-byte boundary below
+// the chunk's first level, two levels more than the chunk.
 //
 // Measured against the CTA-per-column kernel (one launch, 128x256x256 moist,
 // PPM + HLLC): FP32 fluxes 2.52 -> 1.27 ms, FP64 3.05 -> 2.01 ms.  What bounds
@@ -78,9 +80,11 @@ __host__ __device__ constexpr int march_comp(int ny, int n) { return march_nd(ny
 struct MarchTile {
   int bj, bk, nj, nk;
 };
-inline MarchTile march_tile(int nx2, int nx3) {
+inline MarchTile march_tile(int nx1, int nx2, int nx3) {
   MarchTile best{0, 0, 0, 0};
-  for (int bj = 32; bj >= 1; bj /= 2) {
+  // odd columns need a request per variable, k and parity of j, each to a
+  // 128-byte boundary of shared memory
+  for (int bj = 32; bj >= (nx1 % 2 ? 16 : 1); bj /= 2) {
     const int bk = kMarchCols / bj;
     const MarchTile t{bj, bk, (nx2 + bj - 1) / bj, (nx3 + bk - 1) / bk};
     if (!best.bj || (int64_t)t.nj * t.nk < (int64_t)best.nj * best.nk) best = t;
@@ -89,7 +93,7 @@ inline MarchTile march_tile(int nx2, int nx3) {
 }
 
 inline size_t march_scratch_doubles(int ny, int n, int nx1, int nx2, int nx3, int npanel) {
-  const MarchTile t = march_tile(nx2, nx3);
+  const MarchTile t = march_tile(nx1, nx2, nx3);
   return (size_t)t.nj * t.nk * npanel * nx1 * (march_h(n) + march_comp(ny, n)) * kMarchCols;
 }
 
@@ -121,23 +125,28 @@ struct MarchSmem {
   static constexpr int hg = aj + rsz(RR * NAJ * NC);  // [NH][32] H, g of the last row
   static constexpr int NH = march_h(N);
   static constexpr int total1 = hg + NH * NC;
-  // way back up: u and the species of w of four chunks, H and g of five, and x
+  // way back up: u and the species of w of four chunks, H and g of three, and x
   // of two
   static constexpr int UP = kMarchUp;
-  static constexpr int u = 0;                    // [4][NV][32][UP], swizzled
-  static constexpr int sp = u + 4 * UP * NV * NC;  // [4][ny][32][UP], swizzled
-  static constexpr int h = sp + 4 * UP * ny * NC;  // [5][UP][NH][32]
-  static constexpr int x = h + 5 * UP * NH * NC;   // [2][UP][N][32]
-  static constexpr int total2 = x + 2 * UP * N * NC;
-  static constexpr int total = total1 > total2 ? total1 : total2;
+  // [4][NV][32][lev] u and [4][ny][32][lev] species first, then H, g and x
+  static constexpr int hx(int lev) { return 4 * (NV + ny) * lev * NC; }
+  static constexpr int nhx = 3 * UP * NH * NC + 2 * UP * N * NC;
+  // columns of an odd number of levels keep two levels more of w and d each,
+  // which shifts what follows, and of u and sp
+  static constexpr int shift = 2 * NV * NC;
+  static constexpr int total(bool odd) {
+    const int a = total1 + (odd ? 2 * shift : 0), b = hx(odd ? UP + 2 : UP) + nhx;
+    return a > b ? a : b;
+  }
   // the levels' dx follow at `total`
-  static constexpr size_t bytes(int nc1) { return sizeof(double) * ((size_t)total + nc1); }
+  static constexpr size_t bytes(int nc1) { return sizeof(double) * ((size_t)total(nc1 % 2) + nc1); }
 };
 
-// levels per chunk
+// levels per chunk: eight in FP32, as far as two CTAs (3x3) or one (5x5) fit an
+// SM with them (77x83x61 with eight and one CTA: 192 us, with four and two: 150)
 template <typename R>
-constexpr int march_chunk(int ny) {
-  return sizeof(R) == 4 && ny <= 3 ? 8 : 4;
+constexpr int march_chunk(int ny, int n, int odd) {
+  return sizeof(R) == 4 && ny <= (n == 3 && odd ? 2 : 3) ? 8 : 4;
 }
 
 // barriers reached from the level warps' and the elimination warp's own loops
@@ -161,6 +170,14 @@ __device__ __forceinline__ void march_tma_load(double *dst, const CUtensorMap *m
       "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
       "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(smem_addr(dst)),
       "l"(map), "r"(x), "r"(j), "r"(k), "r"(n), "r"(pan), "r"(smem_addr(m))
+      : "memory");
+}
+__device__ __forceinline__ void march_tma_load2(double *dst, const CUtensorMap *map, int x, int y,
+                                                uint64_t *m) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3}], [%4];" ::"r"(smem_addr(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(smem_addr(m))
       : "memory");
 }
 __device__ __forceinline__ void march_tma_store(const CUtensorMap *map, int x, int j, int k, int n,
@@ -197,8 +214,8 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
   constexpr bool PERT = sizeof(R) == 4;
   constexpr int NTP = C * 32, NTA = NTP + 64;
   extern __shared__ __align__(1024) double sm[];
-  // w, du; of the way back up u and species (4 chunks), H and g (5)
-  constexpr int MU = 2, MH = 6, NMB = 11;
+  // w, du; of the way back up u and species (4 chunks), H and g (3)
+  constexpr int MU = 2, MH = 6, NMB = 9;
   __shared__ __align__(8) uint64_t mbar[NMB];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nc1 = g.nc1, is = g.is, ie = g.ie;
@@ -211,27 +228,46 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
   const int tj = blockIdx.x % tl.nj, tkp = blockIdx.x / tl.nj;
   const int pan = tkp / tl.nk;
   const int j0 = g.js + tj * tl.bj, k0 = g.ks + (tkp - pan * tl.nk) * tl.bk;
-  auto column = [&](int c, int &j, int &k) {  // nearest column of the block
-    j = min(j0 + c % tl.bj, g.je);
-    k = min(k0 + c / tl.bj, g.ke);
-  };
-  int j, k;
-  column(lane, j, k);
+  const int j = min(j0 + lane % tl.bj, g.je), k = min(k0 + lane / tl.bj, g.ke);
   const int lc = (k - k0) * tl.bj + (j - j0);
   const bool on = lc == lane;
   const int64_t pbase = g.npanel > 1 ? (int64_t)pan * g.pstride : 0;
   const int64_t base = pbase + (int64_t)k * g.sk + (int64_t)j * nc1;
+  // without boxes: the columns' first cells, and which columns are the tile's
+  __shared__ int64_t colb[NC];
+  const unsigned mine = __ballot_sync(~0u, on);
+  if (threadIdx.x < NC) colb[threadIdx.x] = base;
+  constexpr int WO = C + 2, UO = UP + 2;  // levels of a column in such a copy
+  // parity of this column's first cell and of the step to the next variable:
+  // where the 16-byte boundary lies
+  const int par = (int)(base & 1), psv = (int)(g.sv & 1);
+  // variables n0 .. n0 + nn - 1 of an array from level lo, by a warp; a box of
+  // wl levels for each variable, k and parity of j, the even j's first
+  auto pairs = [&](double *dst, const CUtensorMap *map, int n0, int nn, int lo, int wl, uint64_t *m) {
+    for (int e = lane; e < nn * 2 * tl.bk; e += 32) {
+      const int kk = e % tl.bk, pj = e / tl.bk % 2, n = e / (2 * tl.bk);
+      const int row = (int)(pbase / nc1) + ((n0 + n) * g.nc3 + k0 + kk) * g.nc2 + j0 + pj;
+      const int x = (row & 1) * nc1 + lo;
+      march_tma_load2(dst + (n * NC + pj * (NC / 2) + kk * (tl.bj / 2)) * wl, map, x - (x & 1),
+                      row >> 1, m);
+    }
+  };
+  auto pcol = [&](int c) { return (c % tl.bj % 2) * (NC / 2) + c / tl.bj * (tl.bj / 2) + c % tl.bj / 2; };
+  const int lp = bulk ? 0 : pcol(lc);
   double *scrh = scr + (int64_t)blockIdx.x * g.nx1 * NH * NC;  // H, g of the tile
   scr += (int64_t)gridDim.x * g.nx1 * NH * NC + (int64_t)blockIdx.x * g.nx1 * NCOMP * NC;
   const double grav = th.grav;
   const double wght = st.beta * dtp[0], idt = 1. / wght;
-  double *wb = sm + P::w, *db = sm + P::d, *rb = sm + P::r + lane;
-  double *psr = sm + P::ps + lane, *gmr = sm + P::gm + lane, *rawb = sm + P::raw + lane;
-  R *qb = reinterpret_cast<R *>(sm + P::q) + lane;
-  R *fb = reinterpret_cast<R *>(sm + P::f) + lane;
+  double *wb = sm + P::w, *db = sm + P::d + (bulk ? 0 : P::shift);
+  double *const sm2 = sm + (bulk ? 0 : 2 * P::shift);  // what follows w and d
+  const int VS = NC * (bulk ? C : WO);  // doubles per variable of w, du
+  double *rb = sm2 + P::r + lane;
+  double *psr = sm2 + P::ps + lane, *gmr = sm2 + P::gm + lane, *rawb = sm2 + P::raw + lane;
+  R *qb = reinterpret_cast<R *>(sm2 + P::q) + lane;
+  R *fb = reinterpret_cast<R *>(sm2 + P::f) + lane;
   R *wrb = reinterpret_cast<R *>(sm + P::wr) + lane;
-  R *ajb = reinterpret_cast<R *>(sm + P::aj) + lane;
-  double *sdx = sm + P::total;  // dx1f
+  R *ajb = reinterpret_cast<R *>(sm2 + P::aj) + lane;
+  double *sdx = sm + P::total(!bulk);  // dx1f
   const int last_m = nc1 / C;  // rows lag the levels by four: t = nc1 ends them
 
   // The elimination warps, which have time to spare, wait for the copies; the
@@ -245,7 +281,6 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
       if (g.err) atomicOr(g.err, (uint32_t)CANOE_EBIT_TIMEOUT);
     }
   };
-  constexpr uint32_t kBoxBytes = C * NV * NC * 8;
   if (leader) {
     for (int q = 0; q < NMB; ++q) mbar_init(mbar + q, 1);
     fence_mbar_init();
@@ -262,52 +297,28 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
       sinc = tab(kTabSinC, k, j);
       cth1 = tab(kTabCth1, k, j);
     }
-    // without TMA: this warp's variables of a box through registers, lanes
-    // along the levels of 32 / C columns at a time
-    constexpr int NPW = (NV + C - 1) / C;  // variables per warp
-    constexpr int CPI = 32 / C;            // columns per load
-    double ld[NPW][C];
-    auto reg_load = [&](const double *arr, int lo) {
-      const int l = lo + lane % C;
-#pragma unroll
-      for (int q = 0; q < C; ++q) {
-        int cj, ck;
-        column(q * CPI + lane / C, cj, ck);
-        const double *src = arr + pbase + (int64_t)ck * g.sk + (int64_t)cj * nc1 + l;
-#pragma unroll
-        for (int v = 0; v < NPW; ++v) {
-          const int n = warp + v * C;
-          ld[v][q] = n < NV && l >= 0 && l < nc1 ? src[n * g.sv] : 0.;
-        }
-      }
-    };
-    auto reg_store = [&](double *dst) {
-#pragma unroll
-      for (int q = 0; q < C; ++q)
-#pragma unroll
-        for (int v = 0; v < NPW; ++v) {
-          const int n = warp + v * C;
-          if (n < NV) dst[march_box<C>(n, q * CPI + lane / C, lane % C)] = ld[v][q];
-        }
-    };
     // chunk m: w of levels lo .. lo + C - 1; du of the rows it completes, four
     // levels up
     auto chunk_lo = [&](int m) { return nc1 - C * (m + 1); };
-    auto tma_w = [&](int m) {
-      if (leader && m <= last_m) {
-        mbar_expect_tx(mbar, kBoxBytes);
-        march_tma_load(wb, &maps.w, chunk_lo(m), j0, k0, 0, pan, mbar);
+    auto fetch = [&](double *dst, const CUtensorMap *map, int lo, int q) {
+      if (leader) {
+        mbar_expect_tx(mbar + q, VS * NV * 8);
+        if (bulk) march_tma_load(dst, map, lo, j0, k0, 0, pan, mbar + q);
+      }
+      if (!bulk && warp == 0) {
+        __syncwarp();
+        pairs(dst, map, 0, NV, lo, WO, mbar + q);
       }
     };
+    // place of level lo + o of this lane's column, in the even / odd variables
+    const int pw0 = (par + nc1) & 1, pw1 = pw0 ^ psv;  // lo has nc1's parity
+    auto at0 = [&](int o) { return bulk ? march_box<C>(0, lc, o) : lp * WO + o + pw0; };
+    auto at1 = [&](int o) { return bulk ? march_box<C>(0, lc, o) : lp * WO + o + pw1; };
+    const int a0 = at0(C - 1 - warp), a1 = at1(C - 1 - warp);  // this warp's level
     auto wrap = [](int s) { return s < 0 ? s + RQ : (s >= RQ ? s - RQ : s); };
     static_assert(RR == RQ, "rows and levels share their ring places");
     int bq = 0;  // ring place of the chunk's first level and row
-    if (bulk) {
-      tma_w(0);
-    } else {
-      reg_load(w, chunk_lo(0));
-      reg_store(wb);
-    }
+    fetch(wb, &maps.w, chunk_lo(0), 0);
     if (warp == 0) {
       // face pressures from the top of the column up through the ghosts
       // (t = 2 is the face ie + 1)
@@ -326,16 +337,11 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     for (int m = 0; m <= last_m; ++m) {
       const int t = m * C + warp;
       // ---- phase 1
-      if (bulk) {
-        if (leader) {
-          mbar_expect_tx(mbar + 1, kBoxBytes);
-          march_tma_load(db, &maps.du, chunk_lo(m) + 4, j0, k0, 0, pan, mbar + 1);
-        }
-      }
+      fetch(db, &maps.du, chunk_lo(m) + 4, 1);
       if (t < nc1) {
         double wv[NV];
 #pragma unroll
-        for (int n = 0; n < NV; ++n) wv[n] = wb[march_box<C>(n, lc, C - 1 - warp)];
+        for (int n = 0; n < NV; ++n) wv[n] = wb[n * VS + (n & 1 ? a1 : a0)];
         double a, b;  // psf(l), psf(l + 1)
         if (t <= 2) {
           a = psr[t * NC];
@@ -350,7 +356,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
           for (int s = t0 + 1; s <= t; ++s) {
             const int i = nc1 - 1 - s;
             const double gg = i < is && g.bc[0] == CANOE_BC_REFLECT ? -grav : grav;
-            const double x = gg * wb[march_box<C>(0, lc, C - 1 - (s - m * C))];
+            const double x = gg * wb[at0(C - 1 - (s - m * C))];
             b = a;
             a = a - x * sdx[i];
           }
@@ -379,7 +385,6 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
       }
       march_sync<1, NTP>();
       // ---- phase 2: cells t - 2, by (variable, group of four cells)
-      if (!bulk) reg_load(du, chunk_lo(m) + 4);
       {
       // the warp's group of four cells and its first variable; its next ones
       // are four apart
@@ -447,7 +452,6 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
         }
       }
       }
-      if (!bulk) reg_store(db);
       march_sync<1, NTP>();
       // ---- phase 3: face t - 3, between the cells t - 2 (left) and t - 3
       if (t >= 5 && t < nc1) {
@@ -495,8 +499,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // wR's place takes w
       march_sync<0, NTA>();
       // ---- phase 4: row i, level t - 4
-      if (bulk) tma_w(m + 1);
-      else reg_load(w, chunk_lo(m + 1));
+      if (m < last_m) fetch(wb, &maps.w, chunk_lo(m + 1), 0);
       if (t >= 5 && t <= nc1) {
         const int i = nc1 - 1 - (t - 4);
         const double *rd = rawb + wrap(bq + warp - 3) * NR * NC;  // cell i - 1
@@ -561,7 +564,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
             dd = idt * (2. * sdx[i]);
           }
 #pragma unroll
-          for (int n = 0; n < NV; ++n) dv[n] = db[march_box<C>(n, lc, C - 1 - warp)] + dv[n];
+          for (int n = 0; n < NV; ++n) dv[n] = db[n * VS + (n & 1 ? a1 : a0)] + dv[n];
           double dsum = dv[0];
 #pragma unroll
           for (int n = 1; n <= NY; ++n) dsum += dv[n];
@@ -624,7 +627,6 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
           for (int e = 0; e < N * N; ++e) ao[e * NC] = R(mt.a[e / N][e % N]);
         }
       }
-      if (!bulk) reg_store(wb);
       bq = wrap(bq + C);
       march_sync<0, NTA>();
     }
@@ -632,7 +634,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     // ---- elimination of the rows of chunk m, while the level warps work on
     // chunk m + 1; this warp takes every second row
     const int e2 = warp - C;
-    double *hg = sm + P::hg + lane;
+    double *hg = sm2 + P::hg + lane;
     auto row = [&](int t) {
       if (t < 7 || t > nc1) return;  // rows ie .. is
       const int i = nc1 - 1 - (t - 4);
@@ -766,7 +768,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
       for (int e = 0; e < NH; ++e) so[e * NC] = h[e];
     };
     auto arrived = [&](int q, int m) {  // w (q = 0) or du (1) of chunk m
-      if (bulk && e2 == q) wait(q, m & 1);
+      if (e2 == q) wait(q, m & 1);
     };
     arrived(0, 0);
     march_sync<0, NTA>();
@@ -794,28 +796,38 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
   asm volatile("fence.proxy.async;" ::: "memory");  // H, g and the buffers, before bulk copies
   march_sync<0, NTA>();
   const int nq = (ie - 2) / UP + 1;
-  double *ub = sm + P::u, *spb = sm + P::sp, *hb = sm + P::h, *xs = sm + P::x + lane;
-  constexpr int UC = UP * NV * NC, SC = UP * NY * NC, HC = UP * NH * NC;
+  double *hb = sm + P::hx(bulk ? UP : UO), *xs = hb + 3 * UP * NH * NC + lane;
+  const int UVS = NC * (bulk ? UP : UO), UC = UVS * NV, SC = UVS * NY;
+  double *ub = sm, *spb = sm + 4 * UC;
+  constexpr int HC = UP * NH * NC;
   // by one lane: H and g of chunk q, used first, and the rest of it; what the
   // level warps read from scratch themselves starts towards L2
   auto fetch_h = [&](int q) {
     if (q >= nq) return;
     const int lo = 2 + UP * q, i0 = max(lo, is), n = min(lo + UP - 1, ie) - i0 + 1;
-    uint64_t *mb = mbar + MH + q % 5;
+    uint64_t *mb = mbar + MH + q % 3;
     mbar_expect_tx(mb, n * NH * NC * 8);
-    bulk_g2s(hb + (q % 5) * HC + (i0 - lo) * NH * NC, scrh + (int64_t)(i0 - is) * NH * NC,
+    bulk_g2s(hb + (q % 3) * HC + (i0 - lo) * NH * NC, scrh + (int64_t)(i0 - is) * NH * NC,
              n * NH * NC * 8, mb);
   };
-  auto fetch_u = [&](int q) {
+  auto fetch_u = [&](int q) {  // by the whole warp
     if (q >= nq) return;
     const int lo = 2 + UP * q, i0 = max(lo, is), n = min(lo + UP - 1, ie) - i0 + 1;
-    if (bulk) {
-      uint64_t *mb = mbar + MU + (q & 3);
+    uint64_t *mb = mbar + MU + (q & 3);
+    double *du_ = ub + (q & 3) * UC, *ds = spb + (q & 3) * SC;
+    if (lane == 0) {
       mbar_expect_tx(mb, (UC + SC) * 8);
-      march_tma_load(ub + (q & 3) * UC, &maps.u, lo, j0, k0, 0, pan, mb);
-      if constexpr (NY > 0) march_tma_load(spb + (q & 3) * SC, &maps.sp, lo, j0, k0, 1, pan, mb);
+      if (bulk) {
+        march_tma_load(du_, &maps.u, lo, j0, k0, 0, pan, mb);
+        if constexpr (NY > 0) march_tma_load(ds, &maps.sp, lo, j0, k0, 1, pan, mb);
+      }
+      bulk_prefetch_l2(scr + (int64_t)(i0 - is) * NCOMP * NC, n * NCOMP * NC * 8);
     }
-    bulk_prefetch_l2(scr + (int64_t)(i0 - is) * NCOMP * NC, n * NCOMP * NC * 8);
+    if (!bulk) {
+      __syncwarp();
+      pairs(du_, &maps.u, 0, NV, lo, UO, mb);
+      pairs(ds, &maps.sp, 1, NY, lo, UO, mb);
+    }
   };
   if (warp < C) {
     // C = 8: two warps per level, one for the densities, one for momenta and
@@ -848,64 +860,46 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
           for (int n = 0; n < 4; ++n) v[OFF1 + NT + n] = si[(ND + S::IVX + n) * NC];
       }
     };
-    // without TMA, u and the species of w through registers
-    constexpr int NE = (NV + NY) * UP * NC, NLD = (NE + NTP - 1) / NTP;
-    double rg[NLD];
-    auto reg_up = [&](int q, bool put) {
-#pragma unroll
-      for (int z = 0; z < NLD; ++z) {
-        const int e = threadIdx.x + z * NTP;
-        const int o = e % UP, c = e / UP % NC, n = e / (UP * NC);
-        const int l = 2 + UP * q + o;
-        if (e >= NE || q >= nq || l >= nc1) continue;
-        if (put) {
-          if (n < NV) ub[(q & 3) * UC + march_box<UP>(n, c, o)] = rg[z];
-          else spb[(q & 3) * SC + march_box<UP>(n - NV, c, o)] = rg[z];
-        } else {
-          int cj, ck;
-          column(c, cj, ck);
-          const int64_t at = pbase + (int64_t)ck * g.sk + (int64_t)cj * nc1 + l;
-          rg[z] = n < NV ? u[n * g.sv + at] : w[(n - NV + 1) * g.sv + at];
-        }
-      }
-    };
-    if (!bulk) {
-      reg_up(0, false);
-      reg_up(0, true);
-    }
+    // places of this warp's level in the boxes of the even / odd variables (the
+    // species' first is an odd one); without boxes a thread writes back one
+    // level of one column, of every NTP / (UP * 32)-th variable
+    const int b0 = bulk ? march_box<UP>(0, lane, lev) : lp * UO + lev + par;
+    const int b1 = bulk ? b0 : lp * UO + lev + (par ^ psv);
+    const int s0 = bulk ? march_box<UP>(0, lc, lev) : b1, s1 = bulk ? s0 : b0;
+    constexpr int ZN = NTP / (UP * NC);
+    const int ro = threadIdx.x % UP, rc = threadIdx.x / UP % NC, rn = threadIdx.x / (UP * NC);
+    const int rp = bulk ? 0 : pcol(rc);
     load_scr(0, cur);
     for (int q = -1; q <= nq; ++q) {
       if (!bulk) {
-        if (q >= 1) {
-          const double *src = ub + ((q - 1) & 3) * UC;
-          for (int e = threadIdx.x; e < UC; e += NTP) {
-            const int o = e % UP, c = e / UP % NC, n = e / (UP * NC), l = 2 + UP * (q - 1) + o;
-            int cj, ck;
-            column(c, cj, ck);
-            if ((ck - k0) * tl.bj + cj - j0 == c && l >= is && l <= ie)
-              u[n * g.sv + pbase + (int64_t)ck * g.sk + (int64_t)cj * nc1 + l] =
-                  src[march_box<UP>(n, c, o)];
+        const int l = 2 + UP * (q - 1) + ro;
+        if (q >= 1 && ((mine >> rc) & 1) && l >= is && l <= ie) {
+          const double *src = ub + ((q - 1) & 3) * UC + rp * UO + ro;
+          const int64_t at = colb[rc] + l;
+#pragma unroll
+          for (int z = 0; z < (NV + ZN - 1) / ZN; ++z) {
+            const int n = rn + z * ZN;
+            if (n < NV) u[n * g.sv + at] = src[n * UVS + (int)((n * g.sv + colb[rc]) & 1)];
           }
         }
-        reg_up(q + 2, false);
       }
       if (q >= 0) load_scr(q + 1, nxt);
       const int i = 2 + UP * q + lev;
       if (q >= 0 && q < nq && i >= is && i <= ie) {
         double *uc = ub + (q & 3) * UC;
         const double *xi = xs + (q & 1) * UP * N * NC + lev * N * NC;
-        double *s1 = scr + (int64_t)(i - is) * NCOMP * NC + ND * NC + lane;
+        double *su = scr + (int64_t)(i - is) * NCOMP * NC + ND * NC + lane;
         // slots n0 .. n0 + NN - 1: their increments dv, and u1 as loaded
         auto update = [&](auto nn, int n0, const double *dv, const double *u1) {
           constexpr int NN = decltype(nn)::value;
           double uo[NN];
 #pragma unroll
-          for (int n = 0; n < NN; ++n) uo[n] = uc[march_box<UP>(n0 + n, lane, lev)];
+          for (int n = 0; n < NN; ++n) uo[n] = uc[(n0 + n) * UVS + ((n0 + n) & 1 ? b1 : b0)];
 #pragma unroll
           for (int n = 0; n < NN; ++n) {
-            if (stage == 0) s1[(n0 + n) * NC] = uo[n];
+            if (stage == 0) su[(n0 + n) * NC] = uo[n];
             const double s = st.g1 * uo[n] + st.g2 * (stage == 0 ? uo[n] : u1[n]);
-            if (on) uc[march_box<UP>(n0 + n, lane, lev)] = s + dv[n];
+            if (on) uc[(n0 + n) * UVS + ((n0 + n) & 1 ? b1 : b0)] = s + dv[n];
           }
         };
         if (half != 1) {
@@ -917,7 +911,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
             const double dens = x0 - cur[NY];
             const double *wc = spb + (q & 3) * SC;
 #pragma unroll
-            for (int n = 1; n <= NY; ++n) dv[n] = wc[march_box<UP>(n - 1, lc, lev)];
+            for (int n = 1; n <= NY; ++n) dv[n] = wc[(n - 1) * UVS + (n & 1 ? s0 : s1)];
 #pragma unroll
             for (int n = 1; n <= NY; ++n) {
               dv[n] = cur[n - 1] + dens * dv[n];
@@ -937,16 +931,14 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
 #pragma unroll
         for (int z = 0; z < NL; ++z) cur[z] = nxt[z];
       }
-      if (!bulk) reg_up(q + 2, true);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       march_sync<0, NTA>();
     }
   } else if (warp == C + 1) {
     // the copies
-    if (lane == 0) {
+    if (lane == 0)
       for (int q = 0; q < 2; ++q) fetch_h(q);
-      fetch_u(0);
-    }
+    fetch_u(0);
     for (int q = -1; q <= nq; ++q) {
       if (lane == 0) {
         fetch_h(q + 3);
@@ -954,11 +946,11 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
           march_tma_store(&maps.u, 2 + UP * (q - 1), j0, k0, 0, pan, ub + ((q - 1) & 3) * UC);
         // chunk q - 2 has been read out: its place takes chunk q + 2
         asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-        fetch_u(q + 2);
       }
-      // for the level warps of the next phase
-      if (bulk && q + 1 < nq) wait(MU + ((q + 1) & 3), ((q + 1) >> 2) & 1);
       __syncwarp();
+      fetch_u(q + 2);
+      // for the level warps of the next phase
+      if (q + 1 < nq) wait(MU + ((q + 1) & 3), ((q + 1) >> 2) & 1);
       march_sync<0, NTA>();
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -968,9 +960,9 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     for (int a = 0; a < N; ++a) x[a] = 0.;
     for (int q = -1; q <= nq; ++q) {
       if (q + 1 < nq) {
-        wait(MH + (q + 1) % 5, (q + 1) / 5 & 1);
+        wait(MH + (q + 1) % 3, (q + 1) / 3 & 1);
         double *xo = xs + ((q + 1) & 1) * UP * N * NC;
-        const double *hc = hb + (q + 1) % 5 * HC + lane;
+        const double *hc = hb + (q + 1) % 3 * HC + lane;
 #pragma unroll
         for (int o = 0; o < UP; ++o) {
           const int i = 2 + UP * (q + 1) + o;
@@ -1013,6 +1005,8 @@ inline PFN_cuTensorMapEncodeTiled march_encoder() {
   return f;
 }
 
+inline bool march_available() { return march_encoder() != nullptr; }
+
 // launcher for one NY (instantiated in march_ny*.cu)
 template <int NY, int N>
 int run_x1march(const Geom &g, const canoe_thermo_t &th, int recon, int rs, int prec,
@@ -1021,11 +1015,15 @@ int run_x1march(const Geom &g, const canoe_thermo_t &th, int recon, int rs, int 
   const bool ppm = recon == CANOE_RECON_PPM, hllc = rs == CANOE_RSOLVER_HLLC;
   const bool f32 = prec == CANOE_FP32_PERTURBATION;
   const int npan = g.npanel > 1 ? g.npanel : 1;
-  const MarchTile tl = march_tile(g.nx2, g.nx3);
+  const MarchTile tl = march_tile(g.nx1, g.nx2, g.nx3);
   Geom gg = g;
   MarchMaps maps{};
   auto al16 = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
-  gg.bulk = g.nc1 % 2 == 0 && al16(w) && al16(du) && al16(u) && march_encoder() ? 1 : 0;
+  if (!(al16(w) && al16(du) && al16(u))) {
+    set_error("the column march copies from 16-byte aligned arrays");
+    return CANOE_ERR_ARG;
+  }
+  gg.bulk = g.nc1 % 2 == 0;
   // box of `lev` levels x the tile's columns x nn variables
   auto encode = [&](CUtensorMap &m, const double *p, int lev, int nn) {
     const cuuint64_t dim[5] = {(cuuint64_t)g.nc1, (cuuint64_t)g.nc2, (cuuint64_t)g.nc3,
@@ -1036,26 +1034,42 @@ int run_x1march(const Geom &g, const canoe_thermo_t &th, int recon, int rs, int 
     const cuuint32_t box[5] = {(cuuint32_t)lev, (cuuint32_t)tl.bj, (cuuint32_t)tl.bk,
                                (cuuint32_t)nn, 1};
     const cuuint32_t one[5] = {1, 1, 1, 1, 1};
-    return march_encoder()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, const_cast<double *>(p), dim,
-                           str, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           lev == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+    if (gg.bulk)
+      return march_encoder()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, const_cast<double *>(p), dim,
+                             str, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                             lev == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    // rows of two columns (the array's last column, a ghost, may be left out)
+    const cuuint64_t dim2[2] = {2 * (cuuint64_t)g.nc1, (cuuint64_t)npan * pst / g.nc1 / 2};
+    const cuuint64_t str2[1] = {(cuuint64_t)g.nc1 * 16};
+    const cuuint32_t box2[2] = {(cuuint32_t)lev + 2, (cuuint32_t)tl.bj / 2};
+    return march_encoder()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double *>(p), dim2,
+                           str2, box2, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   };
   auto go = [&](auto kern, const auto &mx, int C, size_t smem) -> int {
-    if (gg.bulk && !(encode(maps.w, w, C, 5 + NY) && encode(maps.du, du, C, 5 + NY) &&
-                     encode(maps.u, u, kMarchUp, 5 + NY) &&
-                     encode(maps.sp, w, kMarchUp, NY > 0 ? NY : 1)))
-      gg.bulk = 0;
+    if (!march_encoder() ||
+        !(encode(maps.w, w, C, 5 + NY) && encode(maps.du, du, C, 5 + NY) &&
+          encode(maps.u, u, kMarchUp, 5 + NY) && encode(maps.sp, w, kMarchUp, NY > 0 ? NY : 1))) {
+      set_error("cuTensorMapEncodeTiled failed");
+      return CANOE_ERR_CUDA;
+    }
     if (int rc = ensure_smem((const void *)kern, smem)) return rc;
     kern<<<(unsigned)(tl.nj * tl.nk * npan), (C + 2) * 32, smem, st>>>(
         gg, th, mx, tl, maps, w, du, u, g.march, dtp, s, stage);
     CB_CUDA(cudaGetLastError());
     return 0;
   };
-#define CB_MK(RC, RSV, R, GEO)                                            \
-  go(k_x1march<NY, RC, RSV, R, GEO, march_chunk<R>(NY), N>, make_mix<R>(th), \
-     march_chunk<R>(NY), MarchSmem<5 + NY, march_chunk<R>(NY), R, GEO, N>::bytes(g.nc1))
+#define CB_MK(RC, RSV, R, GEO)                                                        \
+  (g.nc1 % 2 && march_chunk<R>(NY, N, 1) != march_chunk<R>(NY, N, 0)                          \
+       ? go(k_x1march<NY, RC, RSV, R, GEO, march_chunk<R>(NY, N, 1), N>, make_mix<R>(th),   \
+            march_chunk<R>(NY, N, 1),                                                      \
+            MarchSmem<5 + NY, march_chunk<R>(NY, N, 1), R, GEO, N>::bytes(g.nc1))          \
+       : go(k_x1march<NY, RC, RSV, R, GEO, march_chunk<R>(NY, N, 0), N>, make_mix<R>(th),   \
+            march_chunk<R>(NY, N, 0),                                                      \
+            MarchSmem<5 + NY, march_chunk<R>(NY, N, 0), R, GEO, N>::bytes(g.nc1)))
   if (g.shell) {
     if constexpr (NY == 0) {
       if (!hllc) {
