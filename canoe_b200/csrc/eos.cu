@@ -172,6 +172,17 @@ __global__ void k_dt_finalize(double *d_dt, unsigned long long *acc, double cfl,
 // saturation adjustment (model and algorithm as documented in the header of
 // this function's host entry point, canoe_saturation_adjust)
 
+// constants of the evaluations that the thermodynamics alone determine, in
+// shared memory: log(p3) of each vapour, and the dry c_v
+struct SatConst {
+  double lnp3[CANOE_MAX_VAPOR], cvd;
+};
+__device__ __forceinline__ void sat_const(const canoe_thermo_t &th, SatConst *sc) {
+  if (threadIdx.x < (unsigned)th.nvapor) sc->lnp3[threadIdx.x] = log(th.p3[threadIdx.x]);
+  if (threadIdx.x == 32) sc->cvd = th.rd / (th.gammad - 1.);
+  __syncthreads();
+}
+
 template <int NY>
 struct SatCell {
   double rho, ie, qd;
@@ -180,10 +191,11 @@ struct SatCell {
 };
 
 template <int NY>
-__device__ __forceinline__ void sat_eval(const canoe_thermo_t &th, const SatCell<NY> &c,
-                                         double T, int fv, int fphase, double &f,
+__device__ __forceinline__ void sat_eval(const canoe_thermo_t &th, const SatConst &sc,
+                                         const SatCell<NY> &c, double T, int fv, int fphase, double &f,
                                          double &fp, double *q) {
-  const double cvd = th.rd / (th.gammad - 1.);
+  const double cvd = sc.cvd;
+  const Recip<double> iT(T);
 #pragma unroll
   for (int n = 0; n <= NY; ++n) q[n] = c.qinert[n];
   double cvs = c.qd, lat = 0., dlat = 0.;
@@ -211,13 +223,13 @@ __device__ __forceinline__ void sat_eval(const canoe_thermo_t &th, const SatCell
     const double delta = liquid ? th.delta_l[v] : th.delta_s[v];
     const double rv = th.rd * (1. + th.inv_mu_ratio_m1[vs - 1]);
     const double lnps =
-        log(th.p3[v]) + beta * (1. - th.t3[v] / T) - delta * log(T / th.t3[v]);
-    const double qs = exp(lnps) / (c.rho * rv * T);
+        sc.lnp3[v] + beta * (1. - iT.of(th.t3[v])) - delta * log(qdiv(T, th.t3[v]));
+    const double qs = qdiv(exp(lnps), c.rho * rv * T);
     double qv, qc, dqv;
     if (qs < c.qt[v]) {
       qv = qs;
       qc = c.qt[v] - qs;
-      dqv = qs * (beta * th.t3[v] / (T * T) - delta / T - 1. / T);
+      dqv = qs * (qdiv(beta * th.t3[v], T * T) - iT.of(delta) - iT.of(1.));
     } else {
       qv = c.qt[v];
       qc = 0.;
@@ -261,23 +273,24 @@ constexpr double kSatGate = 0.05;
 // (o.warm): 0 the unadjusted temperature (cold); 1 the guess; 2 gated: the
 // guess if it exceeds the cold start by kSatGate.
 template <int NY>
-__device__ int sat_cell(const canoe_thermo_t &th, const canoe_satadj_opts_t &o,
+__device__ int sat_cell(const canoe_thermo_t &th, const SatConst &sc, const canoe_satadj_opts_t &o,
                         double *uc, double t_guess, double &t_out, int &flags) {
   using S = Slots<NY>;
-  const double cvd = th.rd / (th.gammad - 1.);
+  const double cvd = sc.cvd;
   SatCell<NY> c;
   c.rho = uc[0];
 #pragma unroll
   for (int n = 1; n <= NY; ++n) c.rho += uc[n];
   const double m1 = uc[S::IVX], m2 = uc[S::IVY], m3 = uc[S::IVZ];
-  const double ke = 0.5 * (m1 * m1 + m2 * m2 + m3 * m3) / c.rho;
+  const Recip<double> ir(c.rho);
+  const double ke = ir.of(0.5 * (m1 * m1 + m2 * m2 + m3 * m3));
   c.ie = uc[S::IPR] - ke;
   double q[NY + 1];
   double qsum = 0.;
   q[0] = 0.;
 #pragma unroll
   for (int n = 1; n <= NY; ++n) {
-    q[n] = uc[n] / c.rho;
+    q[n] = ir.of(uc[n]);
     qsum += q[n];
   }
   c.qd = 1. - qsum;
@@ -321,7 +334,7 @@ __device__ int sat_cell(const canoe_thermo_t &th, const canoe_satadj_opts_t &o,
     cvs += q[n] * (1. + th.cv_ratio_m1[n - 1]);
     lat += q[n] * th.u0[n - 1];
   }
-  const double t_cold = (c.ie / c.rho - lat) / (cvd * cvs);
+  const double t_cold = qdiv(ir.of(c.ie) - lat, cvd * cvs);
 
   int iters = 0;
   bool fallback = false, converged = false;
@@ -340,7 +353,7 @@ __device__ int sat_cell(const canoe_thermo_t &th, const canoe_satadj_opts_t &o,
   const bool dry_in = all_vapour<NY>(th, q);
   const int it0 = 0;
   for (int it = it0; it < o.max_iter && !converged; ++it) {
-    sat_eval<NY>(th, c, T, -1, 0, f, fp, qn);
+    sat_eval<NY>(th, sc, c, T, -1, 0, f, fp, qn);
     if (it == 0 && dry_in && T == t_cold) {
       if (all_vapour<NY>(th, qn)) {
         t_out = t_cold;
@@ -352,7 +365,7 @@ __device__ int sat_cell(const canoe_thermo_t &th, const canoe_satadj_opts_t &o,
       fallback = true;
       break;
     }
-    const double dT = -f / fp;
+    const double dT = qdiv(-f, fp);
     T += dT;
     iters++;
     fprev = fabs(f);
@@ -360,8 +373,8 @@ __device__ int sat_cell(const canoe_thermo_t &th, const canoe_satadj_opts_t &o,
       converged = true;
       // one polishing Newton step: the result no longer depends on which
       // iterate first met the tolerance (cold vs warm start agree to roundoff)
-      sat_eval<NY>(th, c, T, -1, 0, f, fp, qn);
-      T -= f / fp;
+      sat_eval<NY>(th, sc, c, T, -1, 0, f, fp, qn);
+      T -= qdiv(f, fp);
       iters++;
       break;
     }
@@ -371,25 +384,25 @@ __device__ int sat_cell(const canoe_thermo_t &th, const canoe_satadj_opts_t &o,
     double lo = 1., hi = 1.e4;
     if (!(T > lo && T < hi)) T = t_cold;
     for (int it = 0; it < 200; ++it) {
-      sat_eval<NY>(th, c, T, -1, 0, f, fp, qn);
+      sat_eval<NY>(th, sc, c, T, -1, 0, f, fp, qn);
       if (f < 0.) lo = T;
       else hi = T;
-      double tn = T - f / fp;
+      double tn = T - qdiv(f, fp);
       if (!(tn > lo && tn < hi)) tn = 0.5 * (lo + hi);
       const double dT = tn - T;
       T = tn;
       iters++;
       if (fabs(dT) < o.tol || hi - lo < o.tol) {
         converged = true;
-        sat_eval<NY>(th, c, T, -1, 0, f, fp, qn);
+        sat_eval<NY>(th, sc, c, T, -1, 0, f, fp, qn);
         // polish unless the step leaves the bracket (a root on a jump)
-        const double tp = T - f / fp;
+        const double tp = T - qdiv(f, fp);
         if (tp > lo - 2. * o.tol && tp < hi + 2. * o.tol) T = tp;
         break;
       }
     }
   }
-  sat_eval<NY>(th, c, T, -1, 0, f, fp, qn);
+  sat_eval<NY>(th, sc, c, T, -1, 0, f, fp, qn);
   // root on a liquid / ice jump at t3: split the condensate
 #pragma unroll
   for (int v = 0; v < (NY > 0 ? NY : 1); ++v) {
@@ -401,8 +414,8 @@ __device__ int sat_cell(const canoe_thermo_t &th, const canoe_satadj_opts_t &o,
     if (fabs(T - th.t3[v]) > 1e-3) continue;
     double fl, fs, fpl, fps;
     double ql[NY + 1], qs_[NY + 1];
-    sat_eval<NY>(th, c, th.t3[v], v, 0, fl, fpl, ql);
-    sat_eval<NY>(th, c, th.t3[v], v, 1, fs, fps, qs_);
+    sat_eval<NY>(th, sc, c, th.t3[v], v, 0, fl, fpl, ql);
+    sat_eval<NY>(th, sc, c, th.t3[v], v, 1, fs, fps, qs_);
     if ((fl > 0.) == (fs > 0.)) continue;
     const double x = -fs / (fl - fs);
     T = th.t3[v];
@@ -428,14 +441,15 @@ __device__ int sat_cell(const canoe_thermo_t &th, const canoe_satadj_opts_t &o,
 // network inputs of a conserved cell: rho, specific internal energy, total
 // of the first and second condensable families
 template <int NY>
-__device__ __forceinline__ double mlp_features(const canoe_thermo_t &th, const double *uc,
-                                               float *x) {
+__device__ __forceinline__ double mlp_features(const canoe_thermo_t &th, const SatConst &sc,
+                                               const double *uc, float *x) {
   using S = Slots<NY>;
   double rho = uc[0];
 #pragma unroll
   for (int n = 1; n <= NY; ++n) rho += uc[n];
-  const double ke = 0.5 * (uc[S::IVX] * uc[S::IVX] + uc[S::IVY] * uc[S::IVY] +
-                           uc[S::IVZ] * uc[S::IVZ]) / rho;
+  const Recip<double> ir(rho);
+  const double ke = ir.of(0.5 * (uc[S::IVX] * uc[S::IVX] + uc[S::IVY] * uc[S::IVY] +
+                                 uc[S::IVZ] * uc[S::IVZ]));
   double fam[2] = {0., 0.};
 #pragma unroll
   for (int v = 0; v < 2; ++v) {
@@ -444,17 +458,18 @@ __device__ __forceinline__ double mlp_features(const canoe_thermo_t &th, const d
     for (int n = 1; n <= NY; ++n)
       if (n == 1 + v || n == th.liq_slot[v] || n == th.ice_slot[v]) fam[v] += uc[n];
   }
-  const double ev = (uc[S::IPR] - ke) / rho;
+  const double ev = ir.of(uc[S::IPR] - ke);
   x[0] = (float)rho;
   x[1] = (float)ev;
-  x[2] = (float)(fam[0] / rho);
-  x[3] = (float)(fam[1] / rho);
+  const double q0 = ir.of(fam[0]), q1 = ir.of(fam[1]);
+  x[2] = (float)q0;
+  x[3] = (float)q1;
   // temperature with all water as vapour: the baseline the network corrects
   double cvs = 1.;
 #pragma unroll
   for (int v = 0; v < 2; ++v)
-    if (v < th.nvapor) cvs += fam[v] / rho * th.cv_ratio_m1[v];
-  return ev / (th.rd / (th.gammad - 1.) * cvs);
+    if (v < th.nvapor) cvs += (v == 0 ? q0 : q1) * th.cv_ratio_m1[v];
+  return qdiv(ev, sc.cvd * cvs);
 }
 
 // true when a condensable family of the cell is at or above saturation at
@@ -528,8 +543,8 @@ __device__ __forceinline__ float mlp_infer_call(uint8_t *sm, const float *p, con
 // memory and the warpgroup's tensor-core state.
 template <int NY, bool LEARNED>
 __device__ __forceinline__ void satadj_chunk(
-    const canoe_thermo_t &th, const canoe_satadj_opts_t &o, double *__restrict__ u,
-    int64_t ncells, int64_t stride, const Geom &g, int use_geom,
+    const canoe_thermo_t &th, const SatConst &sc, const canoe_satadj_opts_t &o,
+    double *__restrict__ u, int64_t ncells, int64_t stride, const Geom &g, int use_geom,
     const double *__restrict__ t_guess, double *__restrict__ t_out,
     int32_t *__restrict__ iters, unsigned long long *stats, const MlpView &mv,
     double *__restrict__ guess_out, uint32_t *err, int64_t t, uint8_t *sm, UmmaState &us,
@@ -559,7 +574,7 @@ __device__ __forceinline__ void satadj_chunk(
     // stay unsaturated
     float x[kMlpIn] = {0.f, 0.f, 0.f, 0.f};
     if (active) {
-      tdry = mlp_features<NY>(th, uc, x);
+      tdry = mlp_features<NY>(th, sc, uc, x);
       need = may_condense<NY>(th, uc, tdry);
     }
     tg = __longlong_as_double(0x7ff8000000000000LL);  // no guess: cold start
@@ -594,7 +609,7 @@ __device__ __forceinline__ void satadj_chunk(
     if (active && iters) iters[t] = 0;
   } else if (active) {
     double T;
-    it = sat_cell<NY>(th, o, uc, tg, T, fl);
+    it = sat_cell<NY>(th, sc, o, uc, tg, T, fl);
     if (!(fl & 4)) {
 #pragma unroll
       for (int n = 1; n <= NY; ++n) u[n * stride + off] = uc[n];
@@ -628,8 +643,10 @@ __global__ void __launch_bounds__(256, 3)
              int64_t ncells, int64_t stride, Geom g, int use_geom,
              const double *__restrict__ t_guess, double *__restrict__ t_out,
              int32_t *__restrict__ iters, unsigned long long *stats) {
+  __shared__ SatConst sc;
+  sat_const(th, &sc);
   UmmaState us{0u, false, false, {0u, 0u, 0u, 0u}};
-  satadj_chunk<NY, false>(th, o, u, ncells, stride, g, use_geom, t_guess, t_out, iters, stats,
+  satadj_chunk<NY, false>(th, sc, o, u, ncells, stride, g, use_geom, t_guess, t_out, iters, stats,
                           MlpView{}, nullptr, nullptr,
                           (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nullptr, us, 0);
   // one set of atomics per warp: a CTA-wide sum first (a barrier at the end)
@@ -650,13 +667,15 @@ __global__ void __launch_bounds__(kSatWg * kUmmaM, 1)
                      int32_t *__restrict__ iters, unsigned long long *stats, MlpView mv,
                      double *__restrict__ guess_out, uint32_t *err) {
   extern __shared__ __align__(1024) uint8_t dsm[];
+  __shared__ SatConst sc;
+  sat_const(th, &sc);
   mlp_umma_setup<kSatWg>(dsm, mv.p, mv.w2h);
   UmmaState us{0u, true, false, {0u, 0u, 0u, 0u}};
   const int wg = threadIdx.x / kUmmaM;
   const int64_t nchunk = (ncells + kUmmaM - 1) / kUmmaM;
   for (int64_t c = (int64_t)blockIdx.x * kSatWg + wg; c < nchunk;
        c += (int64_t)gridDim.x * kSatWg)
-    satadj_chunk<NY, true>(th, o, u, ncells, stride, g, use_geom, t_guess, t_out, iters, stats,
+    satadj_chunk<NY, true>(th, sc, o, u, ncells, stride, g, use_geom, t_guess, t_out, iters, stats,
                            mv, guess_out, err, c * kUmmaM + threadIdx.x % kUmmaM, dsm, us, wg);
   if (stats && (threadIdx.x & 31) == 0) satadj_flush(stats, us.acc);
   mlp_umma_teardown<kSatWg>(dsm, us.pending, us.phase);
