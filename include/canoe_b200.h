@@ -388,12 +388,15 @@ int canoe_block_error_word(canoe_block_t b, uint32_t *bits);
  * 64..256, 0 for the default (with the 3x3 implicit solve the column height
  * rounded up to a multiple of 32, within 64..128; 224 with the 5x5 solve;
  * 160 otherwise).  Kernels without the 3x3 solve use at most 160
- * and the 5x5 solve always 224.  Results do not depend on it.  No reference
- * counterpart (the reference sweeps columns serially). */
+ * and the 5x5 solve always 224.  Blocks of so many columns that the x1 stage
+ * marches down them, a column per thread, have no such CTA: there the number
+ * has no effect.  Results do not depend on it.  No reference counterpart (the
+ * reference sweeps columns serially). */
 int canoe_block_set_column_threads(canoe_block_t b, int threads);
 
 /* Cells per thread of the x2 / x3 register-window flux runs (4..256; 0 = 16
- * with the FP32 flux path, 32 in FP64).  The results do not depend on it.
+ * with the FP32 flux path, 32 in FP64, shorter in blocks too small to fill the
+ * GPU with such runs).  The results do not depend on it.
  * No reference counterpart: the reference's CalculateFluxes loops over
  * whole pencils (patches/19.calculate_fluxes.patch). */
 int canoe_block_set_flux_run(canoe_block_t b, int cells);
