@@ -233,6 +233,7 @@ int validate_block_config(const canoe_block_config_t &c) {
 static int block_free(canoe_block *b) {
   if (!b) return 0;
   if (b->gexec) cudaGraphExecDestroy(b->gexec);
+  if (b->d_u1 == b->d_u) b->d_u1 = nullptr;
   for (void *p : {(void *)b->d_u, (void *)b->d_w, (void *)b->d_u1, (void *)b->d_du,
                   (void *)b->d_x1f, (void *)b->d_x1v, (void *)b->d_dx1f,
                   (void *)b->d_scr, (void *)b->d_dt, (void *)b->d_pref, (void *)b->d_dtacc,
@@ -449,7 +450,6 @@ int canoe_block_create(const canoe_block_config_t *cfg, canoe_block_t *out) {
   cudaError_t e;
   if ((e = cudaMalloc(&b->d_u, bytes))) return fail(e, "cudaMalloc u");
   if ((e = cudaMalloc(&b->d_w, bytes))) return fail(e, "cudaMalloc w");
-  if ((e = cudaMalloc(&b->d_u1, bytes))) return fail(e, "cudaMalloc u1");
   if ((e = cudaMalloc(&b->d_du, bytes))) return fail(e, "cudaMalloc du");
   if ((e = cudaMalloc(&b->d_x1f, (g.nc1 + 1) * sizeof(double)))) return fail(e, "cudaMalloc x1f");
   if ((e = cudaMalloc(&b->d_x1v, g.nc1 * sizeof(double)))) return fail(e, "cudaMalloc x1v");
@@ -463,7 +463,6 @@ int canoe_block_create(const canoe_block_config_t *cfg, canoe_block_t *out) {
   if ((e = cudaMemset(b->d_sat, 0, 4 * sizeof(unsigned long long)))) return fail(e, "cudaMemset sat");
   if ((e = cudaMemset(b->d_u, 0, bytes))) return fail(e, "cudaMemset u");
   if ((e = cudaMemset(b->d_w, 0, bytes))) return fail(e, "cudaMemset w");
-  if ((e = cudaMemset(b->d_u1, 0, bytes))) return fail(e, "cudaMemset u1");
   if ((e = cudaMemset(b->d_du, 0, bytes))) return fail(e, "cudaMemset du");
   if ((e = cudaMemset(b->d_err, 0, sizeof(uint32_t)))) return fail(e, "cudaMemset err");
   unsigned long long inf = 0x7ff0000000000000ULL;
@@ -486,14 +485,20 @@ int canoe_block_create(const canoe_block_config_t *cfg, canoe_block_t *out) {
     if ((e = cudaMemcpy(b->d_dxl, dl.data(), dl.size() * sizeof(double), cudaMemcpyHostToDevice)))
       return fail(e, "copy");
   }
-  // without memory for the march's scratch the block keeps the kernel that
-  // needs none
+  // without memory for the march's scratch, which holds its u1 too, the block
+  // keeps the kernel that needs none
   if (const size_t nm = march_doubles(g, b->th, cfg->implicit_flag, cfg->precision))
     if (cudaMalloc(&b->d_march, nm * sizeof(double))) {
       b->d_march = nullptr;
       cudaGetLastError();
     }
   g.march = b->d_march;
+  if (b->d_march) {
+    b->d_u1 = b->d_u;  // the modes without a register update take one and leave it
+  } else {
+    if ((e = cudaMalloc(&b->d_u1, bytes))) return fail(e, "cudaMalloc u1");
+    if ((e = cudaMemset(b->d_u1, 0, bytes))) return fail(e, "cudaMemset u1");
+  }
   if ((e = cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking))) return fail(e, "stream");
   b->own_stream = true;
   g.x1f = b->d_x1f;

@@ -27,7 +27,8 @@
 //                      swapped states at panel edges, and the divergence
 //                      with face areas and cell volumes
 //   k_x1col<.., GEO=1> x1 fluxes, coordinate sources, implicit x1 solve and
-//                      the RK update (column.cuh)
+//                      the RK update (column.cuh), or with enough columns
+//                      the same as a march down them (march.cuh)
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -897,6 +898,7 @@ struct canoe_shell {
 
 static int shell_free(canoe_shell *s) {
   if (!s) return 0;
+  if (s->d_u1 == s->d_u) s->d_u1 = nullptr;
   for (void *p : {(void *)s->d_u, (void *)s->d_w, (void *)s->d_u1, (void *)s->d_du, (void *)s->d_march,
                   (void *)s->d_x1f, (void *)s->d_x1v, (void *)s->d_dx1f, (void *)s->d_dt,
                   (void *)s->d_tabs, (void *)s->d_lr, (void *)s->d_pref, (void *)s->d_dtacc,
@@ -1059,7 +1061,6 @@ int canoe_shell_create(const canoe_shell_config_t *cfg, canoe_shell_t *out) {
   };
   if ((e = cudaMalloc(&s->d_u, bytes))) return fail(e, "cudaMalloc u");
   if ((e = cudaMalloc(&s->d_w, bytes))) return fail(e, "cudaMalloc w");
-  if ((e = cudaMalloc(&s->d_u1, bytes))) return fail(e, "cudaMalloc u1");
   if ((e = cudaMalloc(&s->d_du, bytes))) return fail(e, "cudaMalloc du");
   if ((e = cudaMalloc(&s->d_lr, lr_bytes))) return fail(e, "cudaMalloc lr");
   if ((e = cudaMalloc(&s->d_x1f, xf.size() * sizeof(double)))) return fail(e, "cudaMalloc x1f");
@@ -1073,7 +1074,7 @@ int canoe_shell_create(const canoe_shell_config_t *cfg, canoe_shell_t *out) {
   if ((e = cudaMalloc(&s->d_tabs, tabs.size() * sizeof(double)))) return fail(e, "cudaMalloc tabs");
   if ((e = cudaMalloc(&s->d_ghost, gr.size() * sizeof(GhostRow)))) return fail(e, "cudaMalloc ghost");
   if ((e = cudaMalloc(&s->d_edge, er.size() * sizeof(EdgeRow)))) return fail(e, "cudaMalloc edge");
-  for (double *p : {s->d_u, s->d_w, s->d_u1, s->d_du})
+  for (double *p : {s->d_u, s->d_w, s->d_du})
     if ((e = cudaMemset(p, 0, bytes))) return fail(e, "cudaMemset state");
   if ((e = cudaMemset(s->d_lr, 0, lr_bytes))) return fail(e, "cudaMemset lr");
   if ((e = cudaMemset(s->d_err, 0, sizeof(uint32_t)))) return fail(e, "cudaMemset err");
@@ -1090,7 +1091,7 @@ int canoe_shell_create(const canoe_shell_config_t *cfg, canoe_shell_t *out) {
              {s->d_edge, er.data(), er.size() * sizeof(EdgeRow)}};
   for (auto &c : cps)
     if ((e = cudaMemcpy(c.d, c.h, c.n, cudaMemcpyHostToDevice))) return fail(e, "copy tables");
-  {  // scratch of the column march, all panels in one launch; optional
+  {  // scratch of the column march with its u1, all panels in one launch; optional
     Geom g6 = g;
     g6.npanel = 6;
     if (const size_t nm = march_doubles(g6, s->th, cfg->implicit_flag, cfg->precision))
@@ -1099,6 +1100,12 @@ int canoe_shell_create(const canoe_shell_config_t *cfg, canoe_shell_t *out) {
         cudaGetLastError();
       }
     g.march = s->d_march;
+  }
+  if (s->d_march) {
+    s->d_u1 = s->d_u;  // the flux-only launch takes one and leaves it
+  } else {
+    if ((e = cudaMalloc(&s->d_u1, bytes))) return fail(e, "cudaMalloc u1");
+    if ((e = cudaMemset(s->d_u1, 0, bytes))) return fail(e, "cudaMemset u1");
   }
   if ((e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking))) return fail(e, "stream");
   s->own_stream = true;
