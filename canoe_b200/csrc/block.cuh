@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <string>
 
+#include "bulk.cuh"
 #include "physics.cuh"
 
 namespace cb {
@@ -48,6 +49,9 @@ struct Geom {
   // scratch of the column march (march.cuh), march_doubles() long; null: the
   // fused x1 stage runs one CTA per column (column.cuh)
   double *march = nullptr;
+  // polls after which the march's bounded waits give up, on its way down and
+  // back up (canoe_selftest_march_wait)
+  int polls = kBulkSpin, polls_up = kBulkSpin;
 };
 
 // geometry tables of a cubed-sphere panel (gnomonic_equiangle.cpp:140-222)

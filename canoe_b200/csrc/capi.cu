@@ -613,6 +613,20 @@ int canoe_block_solve_implicit(canoe_block_t b, double *d_du, double dt) {
   return 0;
 }
 
+int canoe_selftest_march_wait(canoe_block_t b, int polls, int polls_up) {
+  if (!b || polls < 0 || polls > kBulkSpin || polls_up < 0 || polls_up > kBulkSpin) {
+    set_error("canoe_selftest_march_wait: a block, polls in 0..2^18");
+    return CANOE_ERR_ARG;
+  }
+  b->g.polls = polls;
+  b->g.polls_up = polls_up;
+  if (b->gexec) {  // the captured step changes
+    cudaGraphExecDestroy(b->gexec);
+    b->gexec = nullptr;
+  }
+  return 0;
+}
+
 int canoe_block_use_graph(canoe_block_t b, int on) {
   if (!b) return CANOE_ERR_ARG;
   b->graph = on != 0;

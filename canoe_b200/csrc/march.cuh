@@ -218,6 +218,10 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
   // w, du; of the way back up u and species (4 chunks), H and g (3)
   constexpr int MU = 2, MH = 6, NMB = 9;
   __shared__ __align__(8) uint64_t mbar[NMB];
+  // bit q: a wait for barrier q gave up; of each barrier, 1 + the parity of the
+  // phase armed last (0: none)
+  __shared__ int lost_, armed[NMB];
+  volatile int *const lost = &lost_;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nc1 = g.nc1, is = g.is, ie = g.ie;
   const bool bulk = g.bulk != 0;
@@ -273,17 +277,46 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
 
   // The elimination warps, which have time to spare, wait for the copies; the
   // barrier that they then join hands the data to the level warps.  A bounded
-  // wait that gave up is reported once; the tile then runs on without waiting
-  // (its values are lost, nothing hangs).
-  bool ok = true;
+  // wait that gave up is reported and sets `lost`, which other warps see behind
+  // that barrier at the latest: the barrier whose phase is still open is not
+  // armed again, no copy is issued to its buffer and nothing written to u.  The
+  // tile runs its barriers out on whatever the buffers hold, gives the phases
+  // still in flight a second bounded wait and leaves.
+  bool ok = true;  // what this warp's own waits found
   auto wait = [&](int q, uint32_t parity) {
-    if (ok && !mbar_wait(mbar + q, parity)) {
+    if (ok && !mbar_wait(mbar + q, parity, q < MU ? g.polls : g.polls_up)) {
       ok = false;
+      atomicOr(&lost_, 1 << q);
       if (g.err) atomicOr(g.err, (uint32_t)CANOE_EBIT_TIMEOUT);
     }
   };
+  auto arm = [&](int q, uint32_t parity, uint32_t bytes) {
+    armed[q] = 1 + (int)parity;
+    mbar_expect_tx(mbar + q, bytes);
+  };
+  // w (q = 0) or du (1) of chunk m: w of levels lo .. lo + C - 1, du of the rows
+  // that the chunk completes, four levels up.  A box is one request, by the
+  // level warps' leader; the many of columns of odd levels are left to an
+  // elimination warp (77x83x61: 429 -> 417 us a step).
+  auto fetch = [&](int q, int m) {
+    double *dst = q ? db : wb;
+    const CUtensorMap *map = q ? &maps.du : &maps.w;
+    const int lo = nc1 - C * (m + 1) + (q ? 4 : 0);
+    if (lane == 0) {
+      arm(q, m & 1, VS * NV * 8);
+      if (bulk) march_tma_load(dst, map, lo, j0, k0, 0, pan, mbar + q);
+    }
+    if (!bulk) {
+      __syncwarp();
+      pairs(dst, map, 0, NV, lo, WO, mbar + q);
+    }
+  };
   if (leader) {
-    for (int q = 0; q < NMB; ++q) mbar_init(mbar + q, 1);
+    *lost = 0;
+    for (int q = 0; q < NMB; ++q) {
+      armed[q] = 0;
+      mbar_init(mbar + q, 1);
+    }
     fence_mbar_init();
   }
   for (int i = threadIdx.x; i < nc1; i += NTA) sdx[i] = g.dx1f[i];
@@ -298,19 +331,6 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
       sinc = tab(kTabSinC, k, j);
       cth1 = tab(kTabCth1, k, j);
     }
-    // chunk m: w of levels lo .. lo + C - 1; du of the rows it completes, four
-    // levels up
-    auto chunk_lo = [&](int m) { return nc1 - C * (m + 1); };
-    auto fetch = [&](double *dst, const CUtensorMap *map, int lo, int q) {
-      if (leader) {
-        mbar_expect_tx(mbar + q, VS * NV * 8);
-        if (bulk) march_tma_load(dst, map, lo, j0, k0, 0, pan, mbar + q);
-      }
-      if (!bulk && warp == 0) {
-        __syncwarp();
-        pairs(dst, map, 0, NV, lo, WO, mbar + q);
-      }
-    };
     // place of level lo + o of this lane's column, in the even / odd variables
     const int pw0 = (par + nc1) & 1, pw1 = pw0 ^ psv;  // lo has nc1's parity
     auto at0 = [&](int o) { return bulk ? march_box<C>(0, lc, o) : lp * WO + o + pw0; };
@@ -319,7 +339,10 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     auto wrap = [](int s) { return s < 0 ? s + RQ : (s >= RQ ? s - RQ : s); };
     static_assert(RR == RQ, "rows and levels share their ring places");
     int bq = 0;  // ring place of the chunk's first level and row
-    fetch(wb, &maps.w, chunk_lo(0), 0);
+    if (bulk && leader) fetch(0, 0);
+    // `lost`, read behind one fetch for the next, whose buffer's last wait lies
+    // before the barrier that opened this phase
+    int gone = 0;
     if (warp == 0) {
       // face pressures from the top of the column up through the ghosts
       // (t = 2 is the face ie + 1)
@@ -338,7 +361,8 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     for (int m = 0; m <= last_m; ++m) {
       const int t = m * C + warp;
       // ---- phase 1
-      fetch(db, &maps.du, chunk_lo(m) + 4, 1);
+      if (bulk && leader && !(gone & 2)) fetch(1, m);
+      gone = *lost;
       if (t < nc1) {
         double wv[NV];
 #pragma unroll
@@ -500,7 +524,8 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // wR's place takes w
       march_sync<0, NTA>();
       // ---- phase 4: row i, level t - 4
-      if (m < last_m) fetch(wb, &maps.w, chunk_lo(m + 1), 0);
+      if (bulk && leader && !(gone & 1) && m < last_m) fetch(0, m + 1);
+      gone = *lost;
       if (t >= 5 && t <= nc1) {
         const int i = nc1 - 1 - (t - 4);
         const double *rd = rawb + wrap(bq + warp - 3) * NR * NC;  // cell i - 1
@@ -771,9 +796,14 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     auto arrived = [&](int q, int m) {  // w (q = 0) or du (1) of chunk m
       if (e2 == q) wait(q, m & 1);
     };
+    auto request = [&](int q, int m) {
+      if (!bulk && e2 == q && __all_sync(~0u, ok)) fetch(q, m);
+    };
+    request(0, 0);
     arrived(0, 0);
     march_sync<0, NTA>();
     for (int m = -1; m <= last_m; ++m) {
+      if (m < last_m) request(1, m + 1);
       if (m >= 0)
         for (int p = e2; p < C - 2; p += 2) row(m * C + p);
       // all but the chunk's last two rows are done before the next chunk's
@@ -781,6 +811,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
       if (m < last_m) {
         arrived(1, m + 1);
         march_sync<0, NTA>();  // phase 3 of chunk m + 1
+        if (m + 2 <= last_m) request(0, m + 2);
       }
       if (m >= 0) row(m * C + C - 2 + e2);
       if (m < last_m) {
@@ -796,28 +827,32 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
   // chunk q - 1 is written out and chunk q + 2 fetched.
   asm volatile("fence.proxy.async;" ::: "memory");  // H, g and the buffers, before bulk copies
   march_sync<0, NTA>();
-  const int nq = (ie - 2) / UP + 1;
+  // a tile that lost a copy on the way down does not go back up; no wait comes
+  // between the two barriers, so that all warps read the same
+  const bool down = *lost == 0;
+  march_sync<0, NTA>();
+  const int nq = down ? (ie - 2) / UP + 1 : -2;
   double *hb = sm + P::hx(bulk ? UP : UO), *xs = hb + 3 * UP * NH * NC + lane;
   const int UVS = NC * (bulk ? UP : UO), UC = UVS * NV, SC = UVS * NY;
   double *ub = sm, *spb = sm + 4 * UC;
   constexpr int HC = UP * NH * NC;
-  // by one lane: H and g of chunk q, used first, and the rest of it; what the
-  // level warps read from scratch themselves starts towards L2
+  // H and g of chunk q, by the lane 0 that waits for them
   auto fetch_h = [&](int q) {
-    if (q >= nq) return;
+    if (q >= nq || !ok) return;
     const int lo = 2 + UP * q, i0 = max(lo, is), n = min(lo + UP - 1, ie) - i0 + 1;
-    uint64_t *mb = mbar + MH + q % 3;
-    mbar_expect_tx(mb, n * NH * NC * 8);
+    arm(MH + q % 3, q / 3 & 1, n * NH * NC * 8);
     bulk_g2s(hb + (q % 3) * HC + (i0 - lo) * NH * NC, scrh + (int64_t)(i0 - is) * NH * NC,
-             n * NH * NC * 8, mb);
+             n * NH * NC * 8, mbar + MH + q % 3);
   };
-  auto fetch_u = [&](int q) {  // by the whole warp
-    if (q >= nq) return;
+  // u and the species of chunk q, by the whole warp that waits for them; what
+  // the level warps read from scratch themselves starts towards L2
+  auto fetch_u = [&](int q) {
+    if (q >= nq || !(bulk ? ok : __all_sync(~0u, ok))) return;
     const int lo = 2 + UP * q, i0 = max(lo, is), n = min(lo + UP - 1, ie) - i0 + 1;
     uint64_t *mb = mbar + MU + (q & 3);
     double *du_ = ub + (q & 3) * UC, *ds = spb + (q & 3) * SC;
     if (lane == 0) {
-      mbar_expect_tx(mb, (UC + SC) * 8);
+      arm(MU + (q & 3), q >> 2 & 1, (UC + SC) * 8);
       if (bulk) {
         march_tma_load(du_, &maps.u, lo, j0, k0, 0, pan, mb);
         if constexpr (NY > 0) march_tma_load(ds, &maps.sp, lo, j0, k0, 1, pan, mb);
@@ -874,7 +909,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     for (int q = -1; q <= nq; ++q) {
       if (!bulk) {
         const int l = 2 + UP * (q - 1) + ro;
-        if (q >= 1 && ((mine >> rc) & 1) && l >= is && l <= ie) {
+        if (q >= 1 && ((mine >> rc) & 1) && l >= is && l <= ie && !*lost) {
           const double *src = ub + ((q - 1) & 3) * UC + rp * UO + ro;
           const int64_t at = colb[rc] + l;
 #pragma unroll
@@ -936,14 +971,12 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
       march_sync<0, NTA>();
     }
   } else if (warp == C + 1) {
-    // the copies
-    if (lane == 0)
-      for (int q = 0; q < 2; ++q) fetch_h(q);
+    // the copies of u and the species
     fetch_u(0);
+    int gone = 0;  // x of chunk q - 1 was lost in the phase before the last
     for (int q = -1; q <= nq; ++q) {
       if (lane == 0) {
-        fetch_h(q + 3);
-        if (bulk && q >= 1)
+        if (bulk && q >= 1 && ok && !gone)
           march_tma_store(&maps.u, 2 + UP * (q - 1), j0, k0, 0, pan, ub + ((q - 1) & 3) * UC);
         // chunk q - 2 has been read out: its place takes chunk q + 2
         asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
@@ -952,6 +985,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
       fetch_u(q + 2);
       // for the level warps of the next phase
       if (q + 1 < nq) wait(MU + ((q + 1) & 3), ((q + 1) >> 2) & 1);
+      gone = *lost;
       march_sync<0, NTA>();
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -959,6 +993,8 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     double x[N];
 #pragma unroll
     for (int a = 0; a < N; ++a) x[a] = 0.;
+    if (lane == 0)
+      for (int q = 0; q < 3; ++q) fetch_h(q);
     for (int q = -1; q <= nq; ++q) {
       if (q + 1 < nq) {
         wait(MH + (q + 1) % 3, (q + 1) / 3 & 1);
@@ -982,12 +1018,15 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
             xo[(o * N + a) * NC] = x[a];
           }
         }
+        __syncwarp();
+        if (lane == 0) fetch_h(q + 4);
       }
       march_sync<0, NTA>();
     }
   }
-  if (!ok)  // copies still in flight get a second bounded wait
-    for (int q = 0; q < NMB; ++q) mbar_wait(mbar + q, 0);
+  if (*lost)  // copies still in flight get a second bounded wait
+    for (int q = 0; q < NMB; ++q)
+      if (armed[q]) mbar_wait(mbar + q, armed[q] - 1);
 }
 
 // the tensor map encoder of the driver (null where there is none)

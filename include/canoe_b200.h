@@ -171,6 +171,13 @@ int canoe_selftest_bounded_wait(int spins, int complete, uint32_t *h_bits);
  * both cases.  No reference counterpart. */
 int canoe_selftest_umma_wait(int spins, int issue, uint32_t *h_bits);
 
+/* Self-test of the bounded waits of the column march (the fused x1 stage of a
+ * block of many columns): the polls after which they give up in block b, on
+ * the march's way down the columns and on its way back up.  0 gives up at the
+ * first wait, although its copies arrive (CANOE_EBIT_TIMEOUT; u keeps what the
+ * stage found); 2^18 is the default.  No reference counterpart. */
+int canoe_selftest_march_wait(canoe_block_t b, int polls, int polls_up);
+
 /* Self-test of the kernels' branch-free division and square root: n host
  * operands (rounded to FP32 first when fp32 != 0), h_out[i] = h_a[i] / h_b[i],
  * or sqrt(h_a[i]) when h_b is NULL.  Operands and results in the normal range.
