@@ -115,6 +115,10 @@ SIGNATURES = [
     ("canoe_selftest_march_wait", c_int, [c_void_p, c_int, c_int]),
     ("canoe_selftest_fastmath", c_int, [c_int, c_void_p, c_void_p, c_void_p, c_int]),
     ("canoe_measure_fma_peak", c_int, [c_int, POINTER(c_double)]),
+    ("canoe_block_set_march", c_int, [c_void_p, c_int]),
+    ("canoe_block_marches", c_int, [c_void_p, POINTER(c_int)]),
+    ("canoe_shell_set_march", c_int, [c_void_p, c_int]),
+    ("canoe_shell_marches", c_int, [c_void_p, POINTER(c_int)]),
     ("canoe_block_set_neighbor", c_int, [c_void_p, c_int, c_void_p]),
     ("canoe_block_stage", c_int, [c_void_p, c_int, c_double]),
     ("canoe_block_exchange_ghosts", c_int, [c_void_p]),

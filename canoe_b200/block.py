@@ -78,6 +78,16 @@ class MeshBlock:
         """the dense sinking bubble's dissipation source (straka.cpp:125-190)"""
         check(self.lib.canoe_block_set_diffusion(self.h, float(K), float(p0)), "set_diffusion")
 
+    def set_march(self, on):
+        """whether the x1 stage may march down the block's columns (before the first step)"""
+        check(self.lib.canoe_block_set_march(self.h, 1 if on else 0), "set_march")
+
+    def marches(self):
+        """whether it does"""
+        m = ctypes.c_int()
+        check(self.lib.canoe_block_marches(self.h, ctypes.byref(m)), "marches")
+        return m.value != 0
+
     def set_fixed_dt(self, dt):
         check(self.lib.canoe_block_set_fixed_dt(self.h, float(dt)), "set_fixed_dt")
 

@@ -46,9 +46,10 @@ struct Geom {
   // (the six panels of a cubed-sphere shell share one geometry)
   int npanel = 1;
   int64_t pstride = 0;
-  // scratch of the column march (march.cuh), march_doubles() long; null: the
-  // fused x1 stage runs one CTA per column (column.cuh)
-  double *march = nullptr;
+  // scratch of the column march and its RK register u1 (march.cuh), from
+  // march_scratch(); null: the fused x1 stage runs one CTA per column
+  // (column.cuh)
+  double *march = nullptr, *march_u1 = nullptr;
   // polls after which the march's bounded waits give up, on its way down and
   // back up (canoe_selftest_march_wait)
   int polls = kBulkSpin, polls_up = kBulkSpin;
@@ -97,9 +98,15 @@ int launch_x1col(const Geom &g, const canoe_thermo_t &th, int recon, int rs,
                  int implicit_flag, int precision, int mode, const double *w, double *du, double *u,
                  double *u1, const double *dtp, const Stage &s, int stage,
                  double *flx_out, cudaStream_t st);
-// scratch of the column march of a block's fused x1 stage (march.cuh) in
-// doubles; 0 when the block keeps the CTA-per-column kernel
-size_t march_doubles(const Geom &g, const canoe_thermo_t &th, int implicit_flag, int precision);
+// Decides whether a block's fused x1 stage marches down its columns (march.cuh):
+// sets g.march and g.march_u1 and returns the scratch for the owner to free, or
+// nulls when the block keeps the CTA-per-column kernel (too few columns, a form
+// the march does not provide, or no memory left).  u1: the block's register
+// array, which the march lays out in its own order
+double *march_scratch(Geom &g, const canoe_thermo_t &th, int implicit_flag, int precision,
+                      double *u1, size_t u1_doubles);
+// the device's memory that the march's scratch leaves free: one in so many
+constexpr int kMarchReserve = 32;
 // implicit solves along x2 (dir 1) and x3 (dir 2) of a dry block (lines.cu):
 // whether the flag asks for one in a direction the block has, the doubles
 // of each of the two line-major scratch arrays, and the solve of du in place

@@ -142,6 +142,8 @@ struct canoe_block {
   // (nx2 + 2 NG entries of dx2, then nx3 + 2 NG of dx3)
   double *d_wt = nullptr, *d_dut = nullptr, *d_dxl = nullptr;
   double *d_march = nullptr;  // scratch of the column march (Geom::march)
+  bool march = true;          // the x1 stage may march
+  bool stepped = false;       // whether it does is decided
   bool lines = false;
   cudaStream_t st = nullptr;
   bool own_stream = false;
@@ -233,7 +235,6 @@ int validate_block_config(const canoe_block_config_t &c) {
 static int block_free(canoe_block *b) {
   if (!b) return 0;
   if (b->gexec) cudaGraphExecDestroy(b->gexec);
-  if (b->d_u1 == b->d_u) b->d_u1 = nullptr;
   for (void *p : {(void *)b->d_u, (void *)b->d_w, (void *)b->d_u1, (void *)b->d_du,
                   (void *)b->d_x1f, (void *)b->d_x1v, (void *)b->d_dx1f,
                   (void *)b->d_scr, (void *)b->d_dt, (void *)b->d_pref, (void *)b->d_dtacc,
@@ -271,11 +272,21 @@ static int line_solves(canoe_block *b, double *du, const double *dtp, const Stag
   return 0;
 }
 
+// whether the x1 stage of b marches, decided once: a step's stages share u1
+static void decide_march(canoe_block *b) {
+  if (b->stepped) return;
+  b->stepped = true;
+  if (b->march)
+    b->d_march = march_scratch(b->g, b->th, b->cfg.implicit_flag, b->cfg.precision, b->d_u1,
+                               b->nvals);
+}
+
 // one RK stage of block b on stream st (the per-stage task list up to
 // cons2prim with the physical boundaries); dtp: the step's device dt, acc:
 // the CFL accumulator fed at the last stage
 static int stage_launches(canoe_block *b, int s, double *dtp, unsigned long long *acc,
                           cudaStream_t st, StepTimer *tm = nullptr) {
+  decide_march(b);
   const Geom &g = b->g;
   const Stage &sg = kRK3[s];
   int rc;
@@ -450,6 +461,7 @@ int canoe_block_create(const canoe_block_config_t *cfg, canoe_block_t *out) {
   cudaError_t e;
   if ((e = cudaMalloc(&b->d_u, bytes))) return fail(e, "cudaMalloc u");
   if ((e = cudaMalloc(&b->d_w, bytes))) return fail(e, "cudaMalloc w");
+  if ((e = cudaMalloc(&b->d_u1, bytes))) return fail(e, "cudaMalloc u1");
   if ((e = cudaMalloc(&b->d_du, bytes))) return fail(e, "cudaMalloc du");
   if ((e = cudaMalloc(&b->d_x1f, (g.nc1 + 1) * sizeof(double)))) return fail(e, "cudaMalloc x1f");
   if ((e = cudaMalloc(&b->d_x1v, g.nc1 * sizeof(double)))) return fail(e, "cudaMalloc x1v");
@@ -463,6 +475,7 @@ int canoe_block_create(const canoe_block_config_t *cfg, canoe_block_t *out) {
   if ((e = cudaMemset(b->d_sat, 0, 4 * sizeof(unsigned long long)))) return fail(e, "cudaMemset sat");
   if ((e = cudaMemset(b->d_u, 0, bytes))) return fail(e, "cudaMemset u");
   if ((e = cudaMemset(b->d_w, 0, bytes))) return fail(e, "cudaMemset w");
+  if ((e = cudaMemset(b->d_u1, 0, bytes))) return fail(e, "cudaMemset u1");
   if ((e = cudaMemset(b->d_du, 0, bytes))) return fail(e, "cudaMemset du");
   if ((e = cudaMemset(b->d_err, 0, sizeof(uint32_t)))) return fail(e, "cudaMemset err");
   unsigned long long inf = 0x7ff0000000000000ULL;
@@ -484,20 +497,6 @@ int canoe_block_create(const canoe_block_config_t *cfg, canoe_block_t *out) {
     if ((e = cudaMalloc(&b->d_dxl, dl.size() * sizeof(double)))) return fail(e, "cudaMalloc dxl");
     if ((e = cudaMemcpy(b->d_dxl, dl.data(), dl.size() * sizeof(double), cudaMemcpyHostToDevice)))
       return fail(e, "copy");
-  }
-  // without memory for the march's scratch, which holds its u1 too, the block
-  // keeps the kernel that needs none
-  if (const size_t nm = march_doubles(g, b->th, cfg->implicit_flag, cfg->precision))
-    if (cudaMalloc(&b->d_march, nm * sizeof(double))) {
-      b->d_march = nullptr;
-      cudaGetLastError();
-    }
-  g.march = b->d_march;
-  if (b->d_march) {
-    b->d_u1 = b->d_u;  // the modes without a register update take one and leave it
-  } else {
-    if ((e = cudaMalloc(&b->d_u1, bytes))) return fail(e, "cudaMalloc u1");
-    if ((e = cudaMemset(b->d_u1, 0, bytes))) return fail(e, "cudaMemset u1");
   }
   if ((e = cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking))) return fail(e, "stream");
   b->own_stream = true;
@@ -787,6 +786,23 @@ int canoe_block_set_column_threads(canoe_block_t b, int threads) {
     cudaGraphExecDestroy(b->gexec);
     b->gexec = nullptr;
   }
+  return 0;
+}
+
+int canoe_block_set_march(canoe_block_t b, int on) {
+  if (!b) return CANOE_ERR_ARG;
+  if (b->stepped) {
+    set_error("canoe_block_set_march: before the block's first step");
+    return CANOE_ERR_ARG;
+  }
+  b->march = on != 0;
+  return 0;
+}
+
+int canoe_block_marches(canoe_block_t b, int *marches) {
+  if (!b || !marches) return CANOE_ERR_ARG;
+  decide_march(b);
+  *marches = b->d_march != nullptr;
   return 0;
 }
 

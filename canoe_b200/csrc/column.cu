@@ -28,19 +28,51 @@ CB_DECL2(6)
 #undef CB_DECL2
 #undef CB_DECL
 
-size_t march_doubles(const Geom &g, const canoe_thermo_t &th, int flag, int prec) {
+// whether the fused x1 stage of a block marches, its scratch granted
+static bool march_serves(const Geom &g, const canoe_thermo_t &th, int flag, int prec) {
   const int64_t ncol = (int64_t)g.nx2 * g.nx3 * (g.npanel > 1 ? g.npanel : 1);
   const bool lines = line_solve_on(g, flag, 1) || line_solve_on(g, flag, 2);
   // what the march provides: the x1 solve between walls, on the hydrostatic
   // decomposition, with du initialised by an x2 pass
-  if (!(flag & 1) || lines || g.bc[0] == CANOE_BC_PERIODIC || th.grav == 0. || !g.f2) return 0;
+  if (!(flag & 1) || lines || g.bc[0] == CANOE_BC_PERIODIC || th.grav == 0. || !g.f2) return false;
   const int n = flag & 8 ? 5 : 3;
   const int least = n == 5 ? kMarchMinCols5
                            : (prec == CANOE_FP32_PERTURBATION ? kMarchMinCols32 : kMarchMinCols64);
-  if (ncol < least || !march_available()) return 0;
+  if (ncol < least || !march_available()) return false;
   // columns too long for the CTA-per-column kernel stay refused there
-  if (sizeof(double) * col_smem(g.nv, g.nc1, g.nx1, n, 0, 1).total > 227 * 1024) return 0;
-  return march_scratch_doubles(th.ny, n, g.nx1, g.nx2, g.nx3, g.npanel > 1 ? g.npanel : 1);
+  return sizeof(double) * col_smem(g.nv, g.nc1, g.nx1, n, 0, 1).total <= 227 * 1024;
+}
+
+// Taken at a block's first step, not when it is created: a program makes its
+// blocks first, and as many fit the device as without the march (128x256x256
+// moist: 2.15 GB a block, and 1.21 GB of scratch).  A share of the device stays
+// free for what the program allocates later.
+double *march_scratch(Geom &g, const canoe_thermo_t &th, int flag, int prec, double *u1,
+                      size_t u1_doubles) {
+  g.march = g.march_u1 = nullptr;
+  if (!march_serves(g, th, flag, prec)) return nullptr;
+  const int n = flag & 8 ? 5 : 3;
+  const size_t cells = march_cells(g.nx1, g.nx2, g.nx3, g.npanel > 1 ? g.npanel : 1);
+  const size_t scr = cells * (march_h(n) + march_nd(th.ny, n)), reg = cells * (5 + th.ny);
+  const bool own = reg > u1_doubles;  // ragged tiles of long columns: u1's array is too short
+  const size_t bytes = (scr + (own ? reg : 0)) * sizeof(double);
+  // the first step may be captured into a graph, where other modes refuse an
+  // allocation
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  size_t left = 0, all = 0;
+  double *p = nullptr;
+  if (cudaMemGetInfo(&left, &all) != cudaSuccess || left < bytes + all / kMarchReserve ||
+      cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    p = nullptr;
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (p) {
+    g.march = p;
+    g.march_u1 = own ? p + scr : u1;
+  }
+  return p;
 }
 
 template <int N>

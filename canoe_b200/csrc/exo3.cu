@@ -884,6 +884,8 @@ struct canoe_shell {
   Geom g;
   int64_t pvals = 0;  // values per panel
   double *d_march = nullptr;  // scratch of the column march (Geom::march)
+  bool march = true;          // the x1 stage may march
+  bool stepped = false;       // whether it does is decided
   double *d_u = nullptr, *d_w = nullptr, *d_u1 = nullptr, *d_du = nullptr;
   double *d_x1f = nullptr, *d_x1v = nullptr, *d_dx1f = nullptr, *d_dt = nullptr;
   double *d_tabs = nullptr, *d_lr = nullptr, *d_pref = nullptr;
@@ -898,7 +900,6 @@ struct canoe_shell {
 
 static int shell_free(canoe_shell *s) {
   if (!s) return 0;
-  if (s->d_u1 == s->d_u) s->d_u1 = nullptr;
   for (void *p : {(void *)s->d_u, (void *)s->d_w, (void *)s->d_u1, (void *)s->d_du, (void *)s->d_march,
                   (void *)s->d_x1f, (void *)s->d_x1v, (void *)s->d_dx1f, (void *)s->d_dt,
                   (void *)s->d_tabs, (void *)s->d_lr, (void *)s->d_pref, (void *)s->d_dtacc,
@@ -1061,6 +1062,7 @@ int canoe_shell_create(const canoe_shell_config_t *cfg, canoe_shell_t *out) {
   };
   if ((e = cudaMalloc(&s->d_u, bytes))) return fail(e, "cudaMalloc u");
   if ((e = cudaMalloc(&s->d_w, bytes))) return fail(e, "cudaMalloc w");
+  if ((e = cudaMalloc(&s->d_u1, bytes))) return fail(e, "cudaMalloc u1");
   if ((e = cudaMalloc(&s->d_du, bytes))) return fail(e, "cudaMalloc du");
   if ((e = cudaMalloc(&s->d_lr, lr_bytes))) return fail(e, "cudaMalloc lr");
   if ((e = cudaMalloc(&s->d_x1f, xf.size() * sizeof(double)))) return fail(e, "cudaMalloc x1f");
@@ -1074,7 +1076,7 @@ int canoe_shell_create(const canoe_shell_config_t *cfg, canoe_shell_t *out) {
   if ((e = cudaMalloc(&s->d_tabs, tabs.size() * sizeof(double)))) return fail(e, "cudaMalloc tabs");
   if ((e = cudaMalloc(&s->d_ghost, gr.size() * sizeof(GhostRow)))) return fail(e, "cudaMalloc ghost");
   if ((e = cudaMalloc(&s->d_edge, er.size() * sizeof(EdgeRow)))) return fail(e, "cudaMalloc edge");
-  for (double *p : {s->d_u, s->d_w, s->d_du})
+  for (double *p : {s->d_u, s->d_w, s->d_u1, s->d_du})
     if ((e = cudaMemset(p, 0, bytes))) return fail(e, "cudaMemset state");
   if ((e = cudaMemset(s->d_lr, 0, lr_bytes))) return fail(e, "cudaMemset lr");
   if ((e = cudaMemset(s->d_err, 0, sizeof(uint32_t)))) return fail(e, "cudaMemset err");
@@ -1091,22 +1093,6 @@ int canoe_shell_create(const canoe_shell_config_t *cfg, canoe_shell_t *out) {
              {s->d_edge, er.data(), er.size() * sizeof(EdgeRow)}};
   for (auto &c : cps)
     if ((e = cudaMemcpy(c.d, c.h, c.n, cudaMemcpyHostToDevice))) return fail(e, "copy tables");
-  {  // scratch of the column march with its u1, all panels in one launch; optional
-    Geom g6 = g;
-    g6.npanel = 6;
-    if (const size_t nm = march_doubles(g6, s->th, cfg->implicit_flag, cfg->precision))
-      if (cudaMalloc(&s->d_march, nm * sizeof(double))) {
-        s->d_march = nullptr;
-        cudaGetLastError();
-      }
-    g.march = s->d_march;
-  }
-  if (s->d_march) {
-    s->d_u1 = s->d_u;  // the flux-only launch takes one and leaves it
-  } else {
-    if ((e = cudaMalloc(&s->d_u1, bytes))) return fail(e, "cudaMalloc u1");
-    if ((e = cudaMemset(s->d_u1, 0, bytes))) return fail(e, "cudaMemset u1");
-  }
   if ((e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking))) return fail(e, "stream");
   s->own_stream = true;
   g.x1f = s->d_x1f;
@@ -1195,11 +1181,43 @@ int canoe_shell_calculate_fluxes(canoe_shell_t s, double *d_f1, double *d_f2, do
   return 0;
 }
 
+// whether the x1 stage marches, its six panels in one launch, decided once: a
+// step's stages share u1
+static void decide_march(canoe_shell *s) {
+  if (s->stepped) return;
+  s->stepped = true;
+  if (!s->march) return;
+  Geom g6 = s->g;
+  g6.npanel = 6;
+  s->d_march = march_scratch(g6, s->th, s->cfg.implicit_flag, s->cfg.precision, s->d_u1,
+                             6 * (size_t)s->pvals);
+  s->g.march = g6.march;
+  s->g.march_u1 = g6.march_u1;
+}
+
+int canoe_shell_set_march(canoe_shell_t s, int on) {
+  if (!s) return CANOE_ERR_ARG;
+  if (s->stepped) {
+    set_error("canoe_shell_set_march: before the shell's first step");
+    return CANOE_ERR_ARG;
+  }
+  s->march = on != 0;
+  return 0;
+}
+
+int canoe_shell_marches(canoe_shell_t s, int *marches) {
+  if (!s || !marches) return CANOE_ERR_ARG;
+  decide_march(s);
+  *marches = s->d_march != nullptr;
+  return 0;
+}
+
 int canoe_shell_step(canoe_shell_t s, double dt) {
   if (!s || !(dt > 0.)) {
     set_error("canoe_shell_step: dt must be positive");
     return CANOE_ERR_ARG;
   }
+  decide_march(s);
   int rc;
   if ((rc = launch_dt_finalize(s->d_dt, s->d_dtacc, s->cfg.cfl, dt, s->st))) return rc;
   for (int stage = 0; stage < 3; ++stage) {

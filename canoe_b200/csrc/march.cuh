@@ -69,13 +69,13 @@ constexpr int kMarchMinCols5 = 1200;
 // scratch per level of a tile with N x N blocks: H and g (a tile's levels
 // contiguous); then du of the two transverse momenta (N = 3, whose solve
 // leaves them), of the species, and (with species) the sum of the density
-// increments, and the RK register u1
+// increments.  The RK register u1 lies in the block's own array of it, in the
+// same order of tiles, levels, components and lanes.
 __host__ __device__ constexpr int march_h(int n) { return n * n + n; }
 __host__ __device__ constexpr int march_nt(int n) { return n == 3 ? 2 : 0; }
 __host__ __device__ constexpr int march_nd(int ny, int n) {
   return march_nt(n) + ny + (ny > 0 ? 1 : 0);
 }
-__host__ __device__ constexpr int march_comp(int ny, int n) { return march_nd(ny, n) + 5 + ny; }
 
 // tiles of bj x bk = 32 columns that cover nx2 x nx3 with the fewest tiles
 struct MarchTile {
@@ -93,9 +93,10 @@ inline MarchTile march_tile(int nx1, int nx2, int nx3) {
   return best;
 }
 
-inline size_t march_scratch_doubles(int ny, int n, int nx1, int nx2, int nx3, int npanel) {
+// lanes times levels of all tiles: doubles per component of scratch and u1
+inline size_t march_cells(int nx1, int nx2, int nx3, int npanel) {
   const MarchTile t = march_tile(nx1, nx2, nx3);
-  return (size_t)t.nj * t.nk * npanel * nx1 * (march_h(n) + march_comp(ny, n)) * kMarchCols;
+  return (size_t)t.nj * t.nk * npanel * nx1 * kMarchCols;
 }
 
 // Shared memory of a tile, in doubles.  Levels are counted from the top (t = 0
@@ -205,11 +206,12 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     k_x1march(Geom g, canoe_thermo_t th, Mix<R> mx, MarchTile tl,
               const __grid_constant__ MarchMaps maps,
               const double *__restrict__ w, const double *__restrict__ du, double *u, double *scr,
+              double *u1,
               const double *__restrict__ dtp, Stage st, int stage) {
   using S = Slots<NY>;
   using P = MarchSmem<5 + NY, C, R, GEO, N>;
   constexpr int NV = S::NV, NC = kMarchCols, UP = kMarchUp;
-  constexpr int ND = march_nd(NY, N), NT = march_nt(N), NCOMP = march_comp(NY, N), NH = P::NH;
+  constexpr int ND = march_nd(NY, N), NT = march_nt(N), NH = P::NH;
   constexpr int RQ = P::RQ, RP = P::RP, NR = P::NR, RR = P::RR, NRH = P::NRH,
                 NAJ = P::NAJ;
   constexpr bool PERT = sizeof(R) == 4;
@@ -260,7 +262,8 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
   auto pcol = [&](int c) { return (c % tl.bj % 2) * (NC / 2) + c / tl.bj * (tl.bj / 2) + c % tl.bj / 2; };
   const int lp = bulk ? 0 : pcol(lc);
   double *scrh = scr + (int64_t)blockIdx.x * g.nx1 * NH * NC;  // H, g of the tile
-  scr += (int64_t)gridDim.x * g.nx1 * NH * NC + (int64_t)blockIdx.x * g.nx1 * NCOMP * NC;
+  scr += (int64_t)gridDim.x * g.nx1 * NH * NC + (int64_t)blockIdx.x * g.nx1 * ND * NC;
+  u1 += (int64_t)blockIdx.x * g.nx1 * NV * NC;
   const double grav = th.grav;
   const double wght = st.beta * dtp[0], idt = 1. / wght;
   double *wb = sm + P::w, *db = sm + P::d + (bulk ? 0 : P::shift);
@@ -604,7 +607,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
           ro[(N - 1) * NC] = dv[S::IPR] * dd;
           ro[N * NC] = dd;
           if constexpr (GEO) ro[(N + 1) * NC] = ra;
-          double *so = scr + (int64_t)(i - is) * NCOMP * NC + lane;
+          double *so = scr + (int64_t)(i - is) * ND * NC + lane;
 #pragma unroll
           for (int n = 1; n <= NY; ++n) so[(NT + n - 1) * NC] = dv[n];
           if constexpr (NT > 0) {
@@ -857,7 +860,9 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
         march_tma_load(du_, &maps.u, lo, j0, k0, 0, pan, mb);
         if constexpr (NY > 0) march_tma_load(ds, &maps.sp, lo, j0, k0, 1, pan, mb);
       }
-      bulk_prefetch_l2(scr + (int64_t)(i0 - is) * NCOMP * NC, n * NCOMP * NC * 8);
+      if constexpr (ND > 0)
+        bulk_prefetch_l2(scr + (int64_t)(i0 - is) * ND * NC, n * ND * NC * 8);
+      if (stage != 0) bulk_prefetch_l2(u1 + (int64_t)(i0 - is) * NV * NC, n * NV * NC * 8);
     }
     if (!bulk) {
       __syncwarp();
@@ -879,21 +884,22 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     auto load_scr = [&](int q, double *v) {
       const int i = 2 + UP * q + lev;
       if (q >= nq || i < is || i > ie) return;
-      const double *si = scr + (int64_t)(i - is) * NCOMP * NC + lane;
+      const double *si = scr + (int64_t)(i - is) * ND * NC + lane;
+      const double *s1 = u1 + (int64_t)(i - is) * NV * NC + lane;
       if (half != 1) {
         constexpr int NM = N0 - NY - 1;  // du of the species and the sum
 #pragma unroll
         for (int n = 0; n < NM; ++n) v[n] = si[(NT + n) * NC];
         if (stage != 0)
 #pragma unroll
-          for (int n = 0; n <= NY; ++n) v[NM + n] = si[(ND + n) * NC];
+          for (int n = 0; n <= NY; ++n) v[NM + n] = s1[n * NC];
       }
       if (half != 0) {
 #pragma unroll
         for (int n = 0; n < NT; ++n) v[OFF1 + n] = si[n * NC];
         if (stage != 0)
 #pragma unroll
-          for (int n = 0; n < 4; ++n) v[OFF1 + NT + n] = si[(ND + S::IVX + n) * NC];
+          for (int n = 0; n < 4; ++n) v[OFF1 + NT + n] = s1[(S::IVX + n) * NC];
       }
     };
     // places of this warp's level in the boxes of the even / odd variables (the
@@ -924,9 +930,9 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
       if (q >= 0 && q < nq && i >= is && i <= ie) {
         double *uc = ub + (q & 3) * UC;
         const double *xi = xs + (q & 1) * UP * N * NC + lev * N * NC;
-        double *su = scr + (int64_t)(i - is) * NCOMP * NC + ND * NC + lane;
-        // slots n0 .. n0 + NN - 1: their increments dv, and u1 as loaded
-        auto update = [&](auto nn, int n0, const double *dv, const double *u1) {
+        double *su = u1 + (int64_t)(i - is) * NV * NC + lane;
+        // slots n0 .. n0 + NN - 1: their increments dv, and u1 as loaded (uold)
+        auto update = [&](auto nn, int n0, const double *dv, const double *uold) {
           constexpr int NN = decltype(nn)::value;
           double uo[NN];
 #pragma unroll
@@ -934,7 +940,7 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
 #pragma unroll
           for (int n = 0; n < NN; ++n) {
             if (stage == 0) su[(n0 + n) * NC] = uo[n];
-            const double s = st.g1 * uo[n] + st.g2 * (stage == 0 ? uo[n] : u1[n]);
+            const double s = st.g1 * uo[n] + st.g2 * (stage == 0 ? uo[n] : uold[n]);
             if (on) uc[(n0 + n) * UVS + ((n0 + n) & 1 ? b1 : b0)] = s + dv[n];
           }
         };
@@ -1098,7 +1104,7 @@ int run_x1march(const Geom &g, const canoe_thermo_t &th, int recon, int rs, int 
     }
     if (int rc = ensure_smem((const void *)kern, smem)) return rc;
     kern<<<(unsigned)(tl.nj * tl.nk * npan), (C + 2) * 32, smem, st>>>(
-        gg, th, mx, tl, maps, w, du, u, g.march, dtp, s, stage);
+        gg, th, mx, tl, maps, w, du, u, g.march, g.march_u1, dtp, s, stage);
     CB_CUDA(cudaGetLastError());
     return 0;
   };

@@ -74,6 +74,16 @@ class Shell:
     def step(self, dt):
         check(self.lib.canoe_shell_step(self.h, float(dt)), "canoe_shell_step")
 
+    def set_march(self, on):
+        """whether the x1 stage may march down the columns (before the first step)"""
+        check(self.lib.canoe_shell_set_march(self.h, 1 if on else 0), "set_march")
+
+    def marches(self):
+        """whether it does"""
+        m = ctypes.c_int()
+        check(self.lib.canoe_shell_marches(self.h, ctypes.byref(m)), "marches")
+        return m.value != 0
+
     def synchronize(self):
         check(self.lib.canoe_shell_synchronize(self.h), "synchronize")
 

@@ -401,6 +401,21 @@ int canoe_block_error_word(canoe_block_t b, uint32_t *bits);
  * reference sweeps columns serially). */
 int canoe_block_set_column_threads(canoe_block_t b, int threads);
 
+/* Whether the fused x1 stage of a block of many columns may march down them, a
+ * column per thread (on != 0, the default), or runs a CTA per column as small
+ * blocks do.  Decided once, at the block's first step, where a block that
+ * marches allocates its scratch (14 doubles a cell with the 3x3 solve, 15 + ny
+ * with ny species; 30 or 31 + ny with the 5x5 solve) unless that would leave
+ * less than a thirty-second of the device's memory free: CANOE_ERR_ARG
+ * afterwards.
+ * canoe_block_marches tells, and decides where no step has.  The two forms
+ * eliminate in different orders: the same state to roundoff, not the same
+ * bits.  So blocks that cut one domain give the bits of its single block where
+ * all of them march, or none does.  No reference counterpart (the reference
+ * sweeps columns serially). */
+int canoe_block_set_march(canoe_block_t b, int on);
+int canoe_block_marches(canoe_block_t b, int *marches);
+
 /* Cells per thread of the x2 / x3 register-window flux runs (4..256; 0 = 16
  * with the FP32 flux path, 32 in FP64, shorter in blocks too small to fill the
  * GPU with such runs).  The results do not depend on it.
@@ -529,6 +544,9 @@ int canoe_shell_calculate_fluxes(canoe_shell_t s, double *d_f1, double *d_f2, do
 
 /* One RK3 step of all panels with time step dt (> 0). */
 int canoe_shell_step(canoe_shell_t s, double dt);
+/* canoe_block_set_march and canoe_block_marches for the six panels together */
+int canoe_shell_set_march(canoe_shell_t s, int on);
+int canoe_shell_marches(canoe_shell_t s, int *marches);
 int canoe_shell_synchronize(canoe_shell_t s);
 int canoe_shell_error_word(canoe_shell_t s, uint32_t *bits);
 

@@ -1,0 +1,150 @@
+"""Which blocks march down their columns (csrc/march.cuh) and what that costs and changes: scratch
+taken at the first step alone, the setting and the query, the kernel without scratch, equal bits
+among blocks of one route and roundoff across."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from canoe_b200 import CanoeError, Mesh, MeshBlock, Shell, problems
+from canoe_b200._abi import check, load
+from test_gpu_march import _perturbed, _rel
+
+pytestmark = pytest.mark.gpu
+
+
+def _p(nx1=12, nx2=72, nx3=62, **kw):
+    p = problems.moist3d(nx1=nx1, nx2=nx2, nx3=nx3, x1max=250.0 * nx1, x2max=250.0 * nx2,
+                         x3max=250.0 * nx3, satadj=0, **kw)
+    return _perturbed(p, 21)
+
+
+def _free():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_scratch_is_taken_at_the_first_step():
+    p = _p(60, 100, 100)
+    MeshBlock(_p(8, 8, 8)).step(0.1)  # the library's own memory
+    f0 = _free()
+    b = MeshBlock(p)
+    f1 = _free()
+    arrays = 4 * p.u.nbytes  # u, w, u1, du
+    assert f0 - f1 <= arrays + (16 << 20)
+    assert b.marches()
+    assert f1 - _free() >= 60 * 100 * 100 * 18 * 8
+    b.close()
+    assert abs(f0 - _free()) <= 16 << 20
+
+
+def test_setting_and_query():
+    p = _p()
+    a, b, c = MeshBlock(p), MeshBlock(p), MeshBlock(p)
+    b.set_march(False)
+    assert a.marches() and not b.marches()
+    c.step(0.2)
+    for x in (a, c):
+        with pytest.raises(CanoeError):
+            x.set_march(False)
+    a.step(0.2)
+    b.step(0.2)
+    assert np.array_equal(a.conserved(), c.conserved())
+    # each form is held to 5e-11 of the oracle
+    assert _rel(p, a.conserved(), b.conserved(), 0.2) < 1e-10
+    assert not MeshBlock(_p(12, 16, 12)).marches()
+    assert load().canoe_block_marches(None, ctypes.byref(ctypes.c_int())) != 0
+    assert load().canoe_block_set_march(None, 1) != 0
+
+
+def test_shell_setting_and_query():
+    p = problems.shell_c3(nx1=10, nside=32)
+    a, b = Shell(p), Shell(p)
+    b.set_march(False)
+    assert a.marches() and not b.marches()
+    with pytest.raises(CanoeError):
+        a.set_march(False)
+    a.step(30.0)
+    b.step(30.0)
+    x, y = p.interior(a.conserved()), p.interior(b.conserved())
+    for n in range(5):
+        s = np.linalg.norm(y[:, n])
+        if 1 <= n <= 3:  # the gravity impulse, as tests/test_gpu_march.py
+            s = max(s, 30.0 * 24.79 * np.linalg.norm(y[:, 0]))
+        assert np.linalg.norm(x[:, n] - y[:, n]) <= 1e-10 * s
+
+
+def test_block_without_room_for_scratch():
+    import torch
+    p = _p()
+    a, b = MeshBlock(p), MeshBlock(p)
+    b.set_march(False)
+    free, total = torch.cuda.mem_get_info()
+    ballast = torch.empty(free - total // 32, dtype=torch.uint8, device="cuda")
+    assert not a.marches()
+    del ballast
+    torch.cuda.empty_cache()
+    a.step(0.2)
+    b.step(0.2)
+    assert not a.marches()
+    assert np.array_equal(a.conserved(), b.conserved())
+
+
+def test_caller_allocated_step_has_the_bits_of_a_block_that_does_not_march():
+    import torch
+    p = _p(16, 72, 60)
+    a, b = MeshBlock(p), MeshBlock(p)
+    b.set_march(False)
+    assert a.marches()
+    u = torch.from_numpy(p.u).cuda()
+    w = torch.empty_like(u)
+    check(load().canoe_block_step_noalloc(ctypes.byref(p.cfg), u.data_ptr(), w.data_ptr(), None,
+                                          0.2, None))
+    torch.cuda.synchronize()
+    a.step(0.2)
+    b.step(0.2)
+    got = p.interior(u.cpu().numpy())
+    assert np.array_equal(got, p.interior(b.conserved()))
+    assert _rel(p, u.cpu().numpy(), a.conserved(), 0.2) < 1e-10
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_mesh_of_marching_blocks_has_the_single_blocks_bits(graph):
+    p = _p(12, 96, 92)
+    one, m = MeshBlock(p), Mesh(p, 2, 1, graph=graph)
+    assert one.marches() and all(b.marches() for b in m.blocks)
+    for _ in range(2):
+        one.step()
+        m.step()
+    assert np.array_equal(p.interior(one.conserved()), p.interior(m.conserved()))
+
+
+def test_mesh_across_the_threshold():
+    p = _p(12, 72, 62)
+    one, off, m = MeshBlock(p), MeshBlock(p), Mesh(p, 2, 1)
+    off.set_march(False)
+    assert one.marches() and not any(b.marches() for b in m.blocks)
+    for _ in range(2):
+        for x in (one, off, m):
+            x.step(0.2)
+    assert np.array_equal(p.interior(off.conserved()), p.interior(m.conserved()))
+    assert _rel(p, m.conserved(), one.conserved(), 0.4) < 1e-10
+
+
+def test_first_step_inside_a_callers_capture():
+    import torch
+    p = _p()
+    a, b = MeshBlock(p), MeshBlock(p)
+    a.step(0.2)
+    s = torch.cuda.Stream()
+    check(b.lib.canoe_block_set_stream(b.h, s.cuda_stream))
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=s):
+        b.step(0.2)
+    with torch.cuda.stream(s):
+        g.replay()
+    torch.cuda.synchronize()
+    assert b.marches()
+    assert np.array_equal(a.conserved(), b.conserved())
