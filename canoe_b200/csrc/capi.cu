@@ -1274,7 +1274,8 @@ int canoe_batch_synchronize(canoe_batch_t q) {
 }
 
 // Per block, time steps of the block alone with each candidate number of
-// threads per x1 pencil (64 .. 256) and keep the fastest; then time steps of
+// threads per x1 pencil (64 .. 256) and keep the fastest (a block that marches
+// has no such pencil: its choice is 0, the default, untimed); then time steps of
 // the whole batch with each candidate number of cells per x2 / x3 flux run
 // (the default, 8 .. 64) and keep the fastest for every block.  The blocks'
 // states, dt and counters are restored afterwards.  h_threads (may be NULL)
@@ -1316,9 +1317,11 @@ int canoe_batch_autotune(canoe_batch_t q, int32_t *h_threads) {
   for (size_t n = 0; n < nb && !rc; ++n) {
     canoe_block *b = q->blocks[n];
     float best = 1e30f, ms = 0.f;
-    int pick = kColThreads;
+    decide_march(b);
+    int pick = b->d_march ? 0 : kColThreads;
     b->g.flux_run = 0;
     for (int c : cand) {
+      if (b->d_march) break;
       b->g.col_threads = c;
       rc = step_launches(b, 0.);
       if (!rc) {

@@ -503,7 +503,8 @@ int canoe_batch_synchronize(canoe_batch_t q);
 /* pick, by timing, the fastest threads per x1 pencil of every block (each
  * block timed alone) and then the fastest cells per x2 / x3 flux run for the
  * batch (the whole batch timed); the blocks' states are restored;
- * h_threads[n] (may be NULL) gets the thread choices, canoe_block_get_shapes
+ * h_threads[n] (may be NULL) gets the thread choices (0, and nothing timed, for
+ * a block whose x1 stage marches), canoe_block_get_shapes
  * both */
 int canoe_batch_autotune(canoe_batch_t q, int32_t *h_threads);
 

@@ -6,7 +6,7 @@ import ctypes
 import numpy as np
 import pytest
 
-from canoe_b200 import CanoeError, Mesh, MeshBlock, Shell, problems
+from canoe_b200 import Batch, CanoeError, Mesh, MeshBlock, Shell, problems
 from canoe_b200._abi import check, load
 from test_gpu_march import _perturbed, _rel
 
@@ -148,3 +148,14 @@ def test_first_step_inside_a_callers_capture():
     torch.cuda.synchronize()
     assert b.marches()
     assert np.array_equal(a.conserved(), b.conserved())
+
+
+def test_autotuner_leaves_marching_blocks_alone():
+    blocks = [MeshBlock(_p()), MeshBlock(_p(12, 16, 12))]
+    ref = [b.conserved() for b in blocks]
+    bt = Batch(blocks)
+    choice = bt.autotune()
+    assert choice[0] == 0 and choice[1] in (64, 96, 128, 160, 192, 256)
+    assert [t for t, _ in bt.shapes()] == list(choice)
+    for b, r in zip(blocks, ref):
+        assert np.array_equal(b.conserved(), r)
