@@ -113,6 +113,7 @@ SIGNATURES = [
     ("canoe_selftest_bounded_wait", c_int, [c_int, c_int, c_void_p]),
     ("canoe_selftest_umma_wait", c_int, [c_int, c_int, c_void_p]),
     ("canoe_selftest_march_wait", c_int, [c_void_p, c_int, c_int]),
+    ("canoe_selftest_block_solve", c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int]),
     ("canoe_selftest_fastmath", c_int, [c_int, c_void_p, c_void_p, c_void_p, c_int]),
     ("canoe_measure_fma_peak", c_int, [c_int, POINTER(c_double)]),
     ("canoe_block_set_march", c_int, [c_void_p, c_int]),

@@ -144,11 +144,13 @@ struct MarchSmem {
   static constexpr size_t bytes(int nc1) { return sizeof(double) * ((size_t)total(nc1 % 2) + nc1); }
 };
 
-// levels per chunk: eight in FP32, as far as two CTAs (3x3) or one (5x5) fit an
-// SM with them (77x83x61 with eight and one CTA: 192 us, with four and two: 150)
+// levels per chunk: with 3x3 blocks eight in FP32, as far as two CTAs fit an SM
+// with them (77x83x61 with eight and one CTA: 192 us, with four and two: 150);
+// with 5x5 blocks four, whose six warps have the registers for the elimination
+// (64x96x96 with eight levels: 524 bytes of spills, 1097 us a step; four: 1076)
 template <typename R>
 constexpr int march_chunk(int ny, int n, int odd) {
-  return sizeof(R) == 4 && ny <= (n == 3 && odd ? 2 : 3) ? 8 : 4;
+  return sizeof(R) == 4 && n == 3 && ny <= (odd ? 2 : 3) ? 8 : 4;
 }
 
 // barriers reached from the level warps' and the elimination warp's own loops
@@ -199,6 +201,202 @@ template <int C>
 __device__ __forceinline__ int march_box(int n, int c, int o) {
   if constexpr (C == 8) return (n * kMarchCols + c) * 8 + ((((o >> 1) ^ (c >> 1)) & 3) << 1) + (o & 1);
   else return (n * kMarchCols + c) * 4 + ((((o >> 1) ^ (c >> 2)) & 1) << 1) + (o & 1);
+}
+
+// Blocks of row t, scaled by twice the cell's volume over its lower face area:
+// D x_i = v + b x_{i-1} + c x_{i+1}, from the rings of |A|, J (ajb) and the
+// right-hand side (rb); at the walls (`bottom`, `top`) the ghost cell mirrors
+// the boundary cell.  gw: gravity times the stage's time step
+template <int N, int GEO, int RR, int NRH, int NAJ, typename R>
+__device__ __forceinline__ void march_blocks(const R *ajb, const double *rb, int t, bool bottom,
+                                             bool top, double gw, double (&D)[N][N],
+                                             double (&b)[N][N], double (&c)[N][N], double (&v)[N]) {
+  constexpr int NC = kMarchCols;
+  // |A| at faces i and i + 1; J of cells i - 1, i and i + 1 (rows 1 ..)
+  const R *ai = ajb + (t % RR) * NAJ * NC, *ap = ajb + ((t - 1) % RR) * NAJ * NC;
+  const R *jm = ai + N * N * NC, *jc = ap + N * N * NC,
+          *jp = ajb + ((t - 2) % RR) * NAJ * NC + N * N * NC;
+  auto jrow = [](const R *j, int x, int y) {
+    return x == 0 ? (y == 1 ? 1. : 0.) : (double)j[((x - 1) * N + y) * NC];
+  };
+  const double *ri = rb + (t % RR) * NRH * NC;
+  const double dd = ri[N * NC];
+  const double ra = GEO ? ri[(N + 1) * NC] : 1.;
+#pragma unroll
+  for (int x = 0; x < N; ++x) {
+    v[x] = ri[x * NC];
+#pragma unroll
+    for (int y = 0; y < N; ++y) {
+      const double am = ai[(N * x + y) * NC], au = ap[(N * x + y) * NC];
+      if constexpr (GEO) {
+        D[x][y] = am + au * ra + (ra - 1.) * jrow(jc, x, y);
+        c[x][y] = (au - jrow(jp, x, y)) * ra;
+      } else {
+        D[x][y] = am + au;
+        c[x][y] = x == 0 && y != 1 ? au : au - jrow(jp, x, y);
+      }
+      b[x][y] = x == 0 && y != 1 ? am : am + jrow(jm, x, y);
+    }
+    D[x][x] += dd;
+  }
+  const double ph = gw * dd;  // gravity over the row's scale
+  D[1][0] -= ph;
+  D[N - 1][1] -= ph;
+  if (bottom) {
+#pragma unroll
+    for (int x = 0; x < N; ++x)
+#pragma unroll
+      for (int y = 0; y < N; ++y) {
+        D[x][y] += y == 1 ? b[x][y] : -b[x][y];
+        b[x][y] = 0.;
+      }
+  }
+  if (top) {
+#pragma unroll
+    for (int x = 0; x < N; ++x)
+#pragma unroll
+      for (int y = 0; y < N; ++y) D[x][y] += y == 1 ? c[x][y] : -c[x][y];
+  }
+}
+
+// D - c H and v + c g of the row above's H, g
+template <int N>
+__device__ __forceinline__ void march_above(const double *hg, double (&D)[N][N],
+                                            const double (&c)[N][N], double (&v)[N]) {
+  constexpr int NC = kMarchCols;
+#pragma unroll
+  for (int z = 0; z < N; ++z) {
+    double hz[N];
+#pragma unroll
+    for (int y = 0; y < N; ++y) hz[y] = hg[(N * z + y) * NC];
+    const double gz = hg[(N * N + z) * NC];
+#pragma unroll
+    for (int x = 0; x < N; ++x) {
+#pragma unroll
+      for (int y = 0; y < N; ++y) D[x][y] -= c[x][z] * hz[y];
+      v[x] += c[x][z] * gz;
+    }
+  }
+}
+
+// magnitude of x for comparisons: the high word of |x|, whose differences of
+// kPivotHigh are factors of 8
+constexpr int kPivotHigh = 3 << 20;
+__device__ __forceinline__ int high_word(double x) { return __double2hiint(x) & 0x7fffffff; }
+
+// D = L U in place without pivoting, rp the pivots' reciprocals.
+// Elimination does not feel a diagonal scaling, and at low Mach number or a
+// vertical Courant number of a few D is a multiple of the identity with some
+// |A| and flux differences (a host restatement of the recursion in 64 and 80
+// bits: 60 to 1000 times closer than pivoting by the largest entry, as the rows
+// differ in scale).  Beyond, pivots cancel: at Mach 1 and Courant number 300 it
+// was up to 4e5 times further off.  False, and L U is not to be used, where a
+// pivot is 8 times smaller or larger than the diagonal it came from, or not a
+// number: the restatement is then as close as with pivoting throughout, and at
+// Mach 0.05 no row of 10^4 fails up to Courant number 3, and 6 at 30.
+__device__ __forceinline__ bool march_factor(double (&D)[5][5], double (&rp)[5]) {
+  constexpr int N = 5;
+  int od[N];  // the diagonal before elimination
+#pragma unroll
+  for (int q = 1; q < N; ++q) od[q] = high_word(D[q][q]);
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    rp[q] = Recip<double>(D[q][q]).r;
+#pragma unroll
+    for (int x = q + 1; x < N; ++x) {
+      D[x][q] *= rp[q];
+#pragma unroll
+      for (int y = q + 1; y < N; ++y) D[x][y] -= D[x][q] * D[q][y];
+    }
+  }
+  bool good = true;
+#pragma unroll
+  for (int q = 1; q < N; ++q)
+    good &= (unsigned)(high_word(D[q][q]) - od[q] + kPivotHigh) < 2u * kPivotHigh;
+  return good;
+}
+
+// h = (L U)^-1 [b v]: row-major D^-1 b, then D^-1 v
+__device__ __forceinline__ void march_sweeps(const double (&D)[5][5], const double (&rp)[5],
+                                             const double (&b)[5][5], const double (&v)[5],
+                                             double (&h)[30]) {
+  constexpr int N = 5;
+#pragma unroll
+  for (int y = 0; y <= N; ++y) {
+    double r[N];
+#pragma unroll
+    for (int x = 0; x < N; ++x) {
+      r[x] = y < N ? b[x][y < N ? y : 0] : v[x];
+#pragma unroll
+      for (int q = 0; q < x; ++q) r[x] -= D[x][q] * r[q];
+    }
+#pragma unroll
+    for (int x = N - 1; x >= 0; --x) {
+#pragma unroll
+      for (int q = x + 1; q < N; ++q) r[x] -= D[x][q] * r[q];
+      r[x] *= rp[x];
+      h[y < N ? N * x + y : N * N + x] = r[x];
+    }
+  }
+}
+
+// The same by Gauss-Jordan elimination with partial pivoting, as inv(M<5>): the
+// way out of march_factor, rare, so that its rows lie in local memory
+static __device__ __noinline__ void march_pivoted(const double (&D)[5][5], const double (&b)[5][5],
+                                           const double (&v)[5], double (&h)[30]) {
+  constexpr int N = 5, NR = 2 * N + 1;
+  double a[N][NR];
+  for (int x = 0; x < N; ++x) {
+    for (int y = 0; y < N; ++y) {
+      a[x][y] = D[x][y];
+      a[x][N + y] = b[x][y];
+    }
+    a[x][2 * N] = v[x];
+  }
+#pragma unroll 1
+  for (int q = 0; q < N; ++q) {
+    int p = q;
+    for (int x = q + 1; x < N; ++x)
+      if (fabs(a[x][q]) > fabs(a[p][q])) p = x;
+    const double ip = 1. / a[p][q];
+    for (int y = q; y < NR; ++y) {
+      const double e = a[p][y] * ip;
+      a[p][y] = a[q][y];
+      a[q][y] = e;
+    }
+#pragma unroll 1
+    for (int x = 0; x < N; ++x) {
+      if (x == q) continue;
+      const double f = a[x][q];
+      for (int y = q; y < NR; ++y) a[x][y] -= f * a[q][y];
+    }
+  }
+  for (int x = 0; x < N; ++x) {
+    for (int y = 0; y < N; ++y) h[N * x + y] = a[x][N + y];
+    h[N * N + x] = a[x][2 * N];
+  }
+}
+
+// Row t from its blocks on, by either: H, g to hg and so.  For the warps of
+// which some lane's march_factor fails
+template <int GEO, int RR, int NRH, int NAJ, typename R>
+__device__ __noinline__ void march_row_pivoted(const R *ajb, const double *rb, double *hg,
+                                               double *so, int t, bool bottom, bool top,
+                                               double gw) {
+  constexpr int NC = kMarchCols;
+  double D[5][5], A[5][5], b[5][5], c[5][5], v[5], rp[5], h[30];
+  march_blocks<5, GEO, RR, NRH, NAJ>(ajb, rb, t, bottom, top, gw, D, b, c, v);
+  if (!top) march_above<5>(hg, D, c, v);
+#pragma unroll
+  for (int x = 0; x < 5; ++x)
+#pragma unroll
+    for (int y = 0; y < 5; ++y) A[x][y] = D[x][y];
+  if (march_factor(D, rp)) march_sweeps(D, rp, b, v, h);
+  else march_pivoted(A, b, v, h);
+  for (int e = 0; e < 30; ++e) {
+    hg[e * NC] = h[e];
+    so[e * NC] = h[e];
+  }
 }
 
 template <int NY, int RECON, int RS, typename R, int GEO, int C, int N>
@@ -667,70 +865,25 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
     auto row = [&](int t) {
       if (t < 7 || t > nc1) return;  // rows ie .. is
       const int i = nc1 - 1 - (t - 4);
-      // |A| at faces i and i + 1; J of cells i - 1, i and i + 1 (rows 1 ..)
-      const R *ai = ajb + (t % RR) * NAJ * NC, *ap = ajb + ((t - 1) % RR) * NAJ * NC;
-      const R *jm = ai + N * N * NC, *jc = ap + N * N * NC,
-              *jp = ajb + ((t - 2) % RR) * NAJ * NC + N * N * NC;
-      auto jrow = [](const R *j, int x, int y) {
-        return x == 0 ? (y == 1 ? 1. : 0.) : (double)j[((x - 1) * N + y) * NC];
-      };
-      const double *ri = rb + (t % RR) * NRH * NC;
-      const double dd = ri[N * NC];
-      const double ra = GEO ? ri[(N + 1) * NC] : 1.;
       double D[N][N], b[N][N], c[N][N], v[N];
-#pragma unroll
-      for (int x = 0; x < N; ++x) {
-        v[x] = ri[x * NC];
-#pragma unroll
-        for (int y = 0; y < N; ++y) {
-          const double am = ai[(N * x + y) * NC], au = ap[(N * x + y) * NC];
-          if constexpr (GEO) {
-            D[x][y] = am + au * ra + (ra - 1.) * jrow(jc, x, y);
-            c[x][y] = (au - jrow(jp, x, y)) * ra;
-          } else {
-            D[x][y] = am + au;
-            c[x][y] = x == 0 && y != 1 ? au : au - jrow(jp, x, y);
-          }
-          b[x][y] = x == 0 && y != 1 ? am : am + jrow(jm, x, y);
-        }
-        D[x][x] += dd;
-      }
-      const double ph = grav * wght * dd;  // gravity over the row's scale
-      D[1][0] -= ph;
-      D[N - 1][1] -= ph;
-      if (i == is) {  // walls: the ghost cell mirrors the boundary cell
-#pragma unroll
-        for (int x = 0; x < N; ++x)
-#pragma unroll
-          for (int y = 0; y < N; ++y) {
-            D[x][y] += y == 1 ? b[x][y] : -b[x][y];
-            b[x][y] = 0.;
-          }
-      }
-      if (i == ie) {
-#pragma unroll
-        for (int x = 0; x < N; ++x)
-#pragma unroll
-          for (int y = 0; y < N; ++y) D[x][y] += y == 1 ? c[x][y] : -c[x][y];
-      } else {
+      march_blocks<N, GEO, RR, NRH, NAJ>(ajb, rb, t, i == is, i == ie, grav * wght, D, b, c, v);
+      if (i != ie) {
         // H, g of the row above, from the other warp
         if (e2 == 0) march_sync<2, 64>();
         else march_sync<3, 64>();
-#pragma unroll
-        for (int z = 0; z < N; ++z) {
-          double hz[N];
-#pragma unroll
-          for (int y = 0; y < N; ++y) hz[y] = hg[(N * z + y) * NC];
-          const double gz = hg[(N * N + z) * NC];
-#pragma unroll
-          for (int x = 0; x < N; ++x) {
-#pragma unroll
-            for (int y = 0; y < N; ++y) D[x][y] -= c[x][z] * hz[y];
-            v[x] += c[x][z] * gz;
-          }
-        }
+        march_above<N>(hg, D, c, v);
       }
       double h[NH];
+      double *so = scrh + (int64_t)(i - is) * NH * NC + lane;
+      auto keep = [&](double *to) {
+#pragma unroll
+        for (int e = 0; e < NH; ++e) to[e * NC] = h[e];
+      };
+      auto arrive = [&] {
+        if (t >= nc1) return;
+        if (e2 == 0) march_arrive<3, 64>();
+        else march_arrive<2, 64>();
+      };
       if constexpr (N == 3) {
         // adjugate over the determinant, as inv(M<3>)
         double K[3][3];
@@ -752,49 +905,19 @@ __global__ void __launch_bounds__((C + 2) * 32, N == 3 ? 2 : 1)
           h[9 + x] = (K[x][0] * v[0] + K[x][1] * v[1] + K[x][2] * v[2]) * id;
         }
       } else {
-        // D = L U in place, then the N columns of b' and v through L and U.
-        // No pivoting: up to a diagonal scaling, which elimination does not
-        // feel, D is a multiple of the identity plus |A| (no negative
-        // eigenvalue) plus the antisymmetric part of the flux differences, so
-        // its pivots do not vanish
         double rp[N];
-#pragma unroll
-        for (int q = 0; q < N; ++q) {
-          rp[q] = Recip<double>(D[q][q]).r;
-#pragma unroll
-          for (int x = q + 1; x < N; ++x) {
-            D[x][q] *= rp[q];
-#pragma unroll
-            for (int y = q + 1; y < N; ++y) D[x][y] -= D[x][q] * D[q][y];
-          }
-        }
-#pragma unroll
-        for (int y = 0; y <= N; ++y) {
-          double r[N];
-#pragma unroll
-          for (int x = 0; x < N; ++x) {
-            r[x] = y < N ? b[x][y < N ? y : 0] : v[x];
-#pragma unroll
-            for (int q = 0; q < x; ++q) r[x] -= D[x][q] * r[q];
-          }
-#pragma unroll
-          for (int x = N - 1; x >= 0; --x) {
-#pragma unroll
-            for (int q = x + 1; q < N; ++q) r[x] -= D[x][q] * r[q];
-            r[x] *= rp[x];
-            h[y < N ? N * x + y : N * N + x] = r[x];
-          }
+        const bool good = march_factor(D, rp);
+        march_sweeps(D, rp, b, v, h);
+        if (!__all_sync(~0u, good)) {
+          march_row_pivoted<GEO, RR, NRH, NAJ>(ajb, rb, hg, so, t, i == is, i == ie, grav * wght);
+          __syncwarp();
+          arrive();
+          return;
         }
       }
-#pragma unroll
-      for (int e = 0; e < NH; ++e) hg[e * NC] = h[e];
-      if (t < nc1) {
-        if (e2 == 0) march_arrive<3, 64>();
-        else march_arrive<2, 64>();
-      }
-      double *so = scrh + (int64_t)(i - is) * NH * NC + lane;
-#pragma unroll
-      for (int e = 0; e < NH; ++e) so[e * NC] = h[e];
+      keep(hg);
+      arrive();
+      keep(so);
     };
     auto arrived = [&](int q, int m) {  // w (q = 0) or du (1) of chunk m
       if (e2 == q) wait(q, m & 1);

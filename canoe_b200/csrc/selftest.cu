@@ -4,6 +4,7 @@
 // Nothing faults: the barrier's phase is completed before the kernel exits.
 #include "block.cuh"
 #include "bulk.cuh"
+#include "march.cuh"
 #include "mlp.cuh"
 
 namespace cb {
@@ -227,6 +228,68 @@ extern "C" int canoe_selftest_fastmath(int fp32, const double *h_a, const double
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpy(h_out, dout, bytes, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  CB_CUDA(e);
+  return 0;
+}
+
+// ---------------------------------------------------------------------------
+// The 5x5 block solve of the column march on host matrices.
+
+namespace cb {
+namespace {
+
+__global__ void k_march_solve(const double *__restrict__ a, const double *__restrict__ rhs,
+                              double *__restrict__ x, int32_t *__restrict__ pivoted, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double D[5][5], A[5][5], b[5][5], v[5], h[30];
+#pragma unroll
+  for (int r = 0; r < 5; ++r) {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      D[r][c] = A[r][c] = a[25 * i + 5 * r + c];
+      b[r][c] = rhs[30 * i + 6 * r + c];
+    }
+    v[r] = rhs[30 * i + 6 * r + 5];
+  }
+  double rp[5];
+  const bool good = march_factor(D, rp);
+  if (good) march_sweeps(D, rp, b, v, h);
+  else march_pivoted(A, b, v, h);
+  pivoted[i] = !good;
+#pragma unroll
+  for (int r = 0; r < 5; ++r) {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) x[30 * i + 6 * r + c] = h[5 * r + c];
+    x[30 * i + 6 * r + 5] = h[25 + r];
+  }
+}
+
+}  // namespace
+}  // namespace cb
+
+extern "C" int canoe_selftest_block_solve(const double *h_a, const double *h_rhs, double *h_x,
+                                          int32_t *h_pivoted, int n) {
+  using namespace cb;
+  if (!h_a || !h_rhs || !h_x || !h_pivoted || n < 1 || n > (1 << 24)) {
+    set_error("canoe_selftest_block_solve: matrices, right-hand sides and results");
+    return CANOE_ERR_ARG;
+  }
+  const size_t na = 25 * (size_t)n, nr = 30 * (size_t)n;
+  double *d = nullptr;
+  CB_CUDA(cudaMalloc(&d, (na + 2 * nr) * sizeof(double) + n * sizeof(int32_t)));
+  int32_t *dp = reinterpret_cast<int32_t *>(d + na + 2 * nr);
+  cudaError_t e = cudaMemcpy(d, h_a, na * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(d + na, h_rhs, nr * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    k_march_solve<<<(unsigned)((n + 127) / 128), 128>>>(d, d + na, d + na + nr, dp, n);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess)
+    e = cudaMemcpy(h_x, d + na + nr, nr * sizeof(double), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(h_pivoted, dp, n * sizeof(int32_t), cudaMemcpyDeviceToHost);
   cudaFree(d);
   CB_CUDA(e);
   return 0;

@@ -178,6 +178,13 @@ int canoe_selftest_umma_wait(int spins, int issue, uint32_t *h_bits);
  * stage found); 2^18 is the default.  No reference counterpart. */
 int canoe_selftest_march_wait(canoe_block_t b, int polls, int polls_up);
 
+/* Self-test of the 5x5 block solve of the column march: n row-major host
+ * matrices h_a (n, 5, 5), right-hand sides h_rhs (n, 5, 6), h_x = h_a^-1 h_rhs;
+ * h_pivoted[i] tells whether the elimination without pivoting was given up for
+ * the one with.  No reference counterpart. */
+int canoe_selftest_block_solve(const double *h_a, const double *h_rhs, double *h_x,
+                               int32_t *h_pivoted, int n);
+
 /* Self-test of the kernels' branch-free division and square root: n host
  * operands (rounded to FP32 first when fp32 != 0), h_out[i] = h_a[i] / h_b[i],
  * or sqrt(h_a[i]) when h_b is NULL.  Operands and results in the normal range.
