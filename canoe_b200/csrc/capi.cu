@@ -46,7 +46,7 @@ namespace {
 
 // operator-level Riemann kernel over (NV, n) face arrays
 template <int NY, int RS, int DIR>
-__global__ void k_riemann_faces(canoe_thermo_t th, const double *__restrict__ wl,
+__global__ void k_riemann_faces(ExactThermo th, const double *__restrict__ wl,
                                 const double *__restrict__ wr,
                                 double *__restrict__ flx, int64_t n) {
   constexpr int NV = 5 + NY;
@@ -64,7 +64,7 @@ __global__ void k_riemann_faces(canoe_thermo_t th, const double *__restrict__ wl
 }
 
 template <int NY, int RS>
-int riemann_faces(const canoe_thermo_t &th, int dir, const double *wl,
+int riemann_faces(const ExactThermo &th, int dir, const double *wl,
                   const double *wr, double *flx, int64_t n, cudaStream_t st) {
   unsigned nb = (unsigned)((n + 127) / 128);
   if (dir == 0) k_riemann_faces<NY, RS, 0><<<nb, 128, 0, st>>>(th, wl, wr, flx, n);
@@ -87,9 +87,10 @@ int riemann_entry(int rs, const canoe_thermo_t *th, int ivx, const double *wl,
   }
   if (n == 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
+  const ExactThermo et{*th};
 #define CB_R(NY) \
-  return rs == CANOE_RSOLVER_LMARS ? riemann_faces<NY, 0>(*th, dir, wl, wr, flx, n, st) \
-                                   : riemann_faces<NY, 1>(*th, dir, wl, wr, flx, n, st)
+  return rs == CANOE_RSOLVER_LMARS ? riemann_faces<NY, 0>(et, dir, wl, wr, flx, n, st) \
+                                   : riemann_faces<NY, 1>(et, dir, wl, wr, flx, n, st)
   switch (th->ny) {
     case 0: CB_R(0);
     case 1: CB_R(1);

@@ -190,12 +190,12 @@ struct SatCell {
   double qinert[NY + 1];
 };
 
-template <int NY>
+template <int NY, class TH>
 __device__ __forceinline__ void sat_eval(const canoe_thermo_t &th, const SatConst &sc,
                                          const SatCell<NY> &c, double T, int fv, int fphase, double &f,
                                          double &fp, double *q) {
   const double cvd = sc.cvd;
-  const Recip<double> iT(T);
+  const TRecip<TH, double> iT(T);
 #pragma unroll
   for (int n = 0; n <= NY; ++n) q[n] = c.qinert[n];
   double cvs = c.qd, lat = 0., dlat = 0.;
@@ -223,13 +223,13 @@ __device__ __forceinline__ void sat_eval(const canoe_thermo_t &th, const SatCons
     const double delta = liquid ? th.delta_l[v] : th.delta_s[v];
     const double rv = th.rd * (1. + th.inv_mu_ratio_m1[vs - 1]);
     const double lnps =
-        sc.lnp3[v] + beta * (1. - iT.of(th.t3[v])) - delta * log(qdiv(T, th.t3[v]));
-    const double qs = qdiv(exp(lnps), c.rho * rv * T);
+        sc.lnp3[v] + beta * (1. - iT.of(th.t3[v])) - delta * log(tdiv<TH>(T, th.t3[v]));
+    const double qs = tdiv<TH>(exp(lnps), c.rho * rv * T);
     double qv, qc, dqv;
     if (qs < c.qt[v]) {
       qv = qs;
       qc = c.qt[v] - qs;
-      dqv = qs * (qdiv(beta * th.t3[v], T * T) - iT.of(delta) - iT.of(1.));
+      dqv = qs * (tdiv<TH>(beta * th.t3[v], T * T) - iT.of(delta) - iT.of(1.));
     } else {
       qv = c.qt[v];
       qc = 0.;
@@ -268,11 +268,28 @@ __device__ __forceinline__ bool all_vapour(const canoe_thermo_t &th, const doubl
 // exact in one step for cells that stay unsaturated
 constexpr double kSatGate = 0.05;
 
+// Whether sums, squares and quotients of a cell's values stay in the range where
+// the branch-free division serves (physics.cuh).  What a caller hands over
+// beyond it takes the same steps with IEEE's division, out of line.
+template <int NY>
+__device__ __forceinline__ bool ordinary_cell(const double *uc) {
+  constexpr int lo = 0x20d00000, hi = 0x5f100000;  // high words of about 1e-150, 1e150
+  double rho = uc[0];
+  int most = 0;
+#pragma unroll
+  for (int n = 1; n < Slots<NY>::NV; ++n) {
+    if (n <= NY) rho += uc[n];
+    most = max(most, __double2hiint(uc[n]) & 0x7fffffff);
+  }
+  const int r = __double2hiint(rho) & 0x7fffffff;
+  return r > lo && max(r, most) < hi;
+}
+
 // returns the number of f evaluations; flags bit0 fallback, bit1 not
 // converged, bit2 the cell is returned unchanged (no write needed).  Start
 // (o.warm): 0 the unadjusted temperature (cold); 1 the guess; 2 gated: the
 // guess if it exceeds the cold start by kSatGate.
-template <int NY>
+template <int NY, class TH>
 __device__ int sat_cell(const canoe_thermo_t &th, const SatConst &sc, const canoe_satadj_opts_t &o,
                         double *uc, double t_guess, double &t_out, int &flags) {
   using S = Slots<NY>;
@@ -282,7 +299,7 @@ __device__ int sat_cell(const canoe_thermo_t &th, const SatConst &sc, const cano
 #pragma unroll
   for (int n = 1; n <= NY; ++n) c.rho += uc[n];
   const double m1 = uc[S::IVX], m2 = uc[S::IVY], m3 = uc[S::IVZ];
-  const Recip<double> ir(c.rho);
+  const TRecip<TH, double> ir(c.rho);
   const double ke = ir.of(0.5 * (m1 * m1 + m2 * m2 + m3 * m3));
   c.ie = uc[S::IPR] - ke;
   double q[NY + 1];
@@ -334,7 +351,7 @@ __device__ int sat_cell(const canoe_thermo_t &th, const SatConst &sc, const cano
     cvs += q[n] * (1. + th.cv_ratio_m1[n - 1]);
     lat += q[n] * th.u0[n - 1];
   }
-  const double t_cold = qdiv(ir.of(c.ie) - lat, cvd * cvs);
+  const double t_cold = tdiv<TH>(ir.of(c.ie) - lat, cvd * cvs);
 
   int iters = 0;
   bool fallback = false, converged = false;
@@ -353,7 +370,7 @@ __device__ int sat_cell(const canoe_thermo_t &th, const SatConst &sc, const cano
   const bool dry_in = all_vapour<NY>(th, q);
   const int it0 = 0;
   for (int it = it0; it < o.max_iter && !converged; ++it) {
-    sat_eval<NY>(th, sc, c, T, -1, 0, f, fp, qn);
+    sat_eval<NY, TH>(th, sc, c, T, -1, 0, f, fp, qn);
     if (it == 0 && dry_in && T == t_cold) {
       if (all_vapour<NY>(th, qn)) {
         t_out = t_cold;
@@ -365,7 +382,7 @@ __device__ int sat_cell(const canoe_thermo_t &th, const SatConst &sc, const cano
       fallback = true;
       break;
     }
-    const double dT = qdiv(-f, fp);
+    const double dT = tdiv<TH>(-f, fp);
     T += dT;
     iters++;
     fprev = fabs(f);
@@ -373,8 +390,8 @@ __device__ int sat_cell(const canoe_thermo_t &th, const SatConst &sc, const cano
       converged = true;
       // one polishing Newton step: the result no longer depends on which
       // iterate first met the tolerance (cold vs warm start agree to roundoff)
-      sat_eval<NY>(th, sc, c, T, -1, 0, f, fp, qn);
-      T -= qdiv(f, fp);
+      sat_eval<NY, TH>(th, sc, c, T, -1, 0, f, fp, qn);
+      T -= tdiv<TH>(f, fp);
       iters++;
       break;
     }
@@ -384,25 +401,25 @@ __device__ int sat_cell(const canoe_thermo_t &th, const SatConst &sc, const cano
     double lo = 1., hi = 1.e4;
     if (!(T > lo && T < hi)) T = t_cold;
     for (int it = 0; it < 200; ++it) {
-      sat_eval<NY>(th, sc, c, T, -1, 0, f, fp, qn);
+      sat_eval<NY, TH>(th, sc, c, T, -1, 0, f, fp, qn);
       if (f < 0.) lo = T;
       else hi = T;
-      double tn = T - qdiv(f, fp);
+      double tn = T - tdiv<TH>(f, fp);
       if (!(tn > lo && tn < hi)) tn = 0.5 * (lo + hi);
       const double dT = tn - T;
       T = tn;
       iters++;
       if (fabs(dT) < o.tol || hi - lo < o.tol) {
         converged = true;
-        sat_eval<NY>(th, sc, c, T, -1, 0, f, fp, qn);
+        sat_eval<NY, TH>(th, sc, c, T, -1, 0, f, fp, qn);
         // polish unless the step leaves the bracket (a root on a jump)
-        const double tp = T - qdiv(f, fp);
+        const double tp = T - tdiv<TH>(f, fp);
         if (tp > lo - 2. * o.tol && tp < hi + 2. * o.tol) T = tp;
         break;
       }
     }
   }
-  sat_eval<NY>(th, sc, c, T, -1, 0, f, fp, qn);
+  sat_eval<NY, TH>(th, sc, c, T, -1, 0, f, fp, qn);
   // root on a liquid / ice jump at t3: split the condensate
 #pragma unroll
   for (int v = 0; v < (NY > 0 ? NY : 1); ++v) {
@@ -414,8 +431,8 @@ __device__ int sat_cell(const canoe_thermo_t &th, const SatConst &sc, const cano
     if (fabs(T - th.t3[v]) > 1e-3) continue;
     double fl, fs, fpl, fps;
     double ql[NY + 1], qs_[NY + 1];
-    sat_eval<NY>(th, sc, c, th.t3[v], v, 0, fl, fpl, ql);
-    sat_eval<NY>(th, sc, c, th.t3[v], v, 1, fs, fps, qs_);
+    sat_eval<NY, TH>(th, sc, c, th.t3[v], v, 0, fl, fpl, ql);
+    sat_eval<NY, TH>(th, sc, c, th.t3[v], v, 1, fs, fps, qs_);
     if ((fl > 0.) == (fs > 0.)) continue;
     const double x = -fs / (fl - fs);
     T = th.t3[v];
@@ -440,14 +457,14 @@ __device__ int sat_cell(const canoe_thermo_t &th, const SatConst &sc, const cano
 
 // network inputs of a conserved cell: rho, specific internal energy, total
 // of the first and second condensable families
-template <int NY>
+template <int NY, class TH>
 __device__ __forceinline__ double mlp_features(const canoe_thermo_t &th, const SatConst &sc,
                                                const double *uc, float *x) {
   using S = Slots<NY>;
   double rho = uc[0];
 #pragma unroll
   for (int n = 1; n <= NY; ++n) rho += uc[n];
-  const Recip<double> ir(rho);
+  const TRecip<TH, double> ir(rho);
   const double ke = ir.of(0.5 * (uc[S::IVX] * uc[S::IVX] + uc[S::IVY] * uc[S::IVY] +
                                  uc[S::IVZ] * uc[S::IVZ]));
   double fam[2] = {0., 0.};
@@ -469,7 +486,20 @@ __device__ __forceinline__ double mlp_features(const canoe_thermo_t &th, const S
 #pragma unroll
   for (int v = 0; v < 2; ++v)
     if (v < th.nvapor) cvs += (v == 0 ? q0 : q1) * th.cv_ratio_m1[v];
-  return qdiv(ev, sc.cvd * cvs);
+  return tdiv<TH>(ev, sc.cvd * cvs);
+}
+
+template <int NY>
+__device__ __noinline__ int sat_cell_any(const canoe_thermo_t &th, const SatConst &sc,
+                                         const canoe_satadj_opts_t &o, double *uc, double t_guess,
+                                         double &t_out, int &flags) {
+  return sat_cell<NY, ExactThermo>(th, sc, o, uc, t_guess, t_out, flags);
+}
+
+template <int NY>
+__device__ __noinline__ double mlp_features_any(const canoe_thermo_t &th, const SatConst &sc,
+                                                const double *uc, float *x) {
+  return mlp_features<NY, ExactThermo>(th, sc, uc, x);
 }
 
 // true when a condensable family of the cell is at or above saturation at
@@ -564,6 +594,7 @@ __device__ __forceinline__ void satadj_chunk(
 #pragma unroll
     for (int n = 0; n < S::NV; ++n) uc[n] = u[n * stride + off];
   }
+  const bool ordinary = !active || ordinary_cell<NY>(uc);
   double tg = t_guess && active ? t_guess[t] : 0.;
   double tdry = 0.;
   bool need = false;
@@ -574,7 +605,17 @@ __device__ __forceinline__ void satadj_chunk(
     // stay unsaturated
     float x[kMlpIn] = {0.f, 0.f, 0.f, 0.f};
     if (active) {
-      tdry = mlp_features<NY>(th, sc, uc, x);
+      if (ordinary) {
+        tdry = mlp_features<NY, canoe_thermo_t>(th, sc, uc, x);
+      } else {
+        double ua[S::NV];
+        float xa[kMlpIn];
+#pragma unroll
+        for (int n = 0; n < S::NV; ++n) ua[n] = uc[n];
+        tdry = mlp_features_any<NY>(th, sc, ua, xa);
+#pragma unroll
+        for (int n = 0; n < kMlpIn; ++n) x[n] = xa[n];
+      }
       need = may_condense<NY>(th, uc, tdry);
     }
     tg = __longlong_as_double(0x7ff8000000000000LL);  // no guess: cold start
@@ -609,7 +650,19 @@ __device__ __forceinline__ void satadj_chunk(
     if (active && iters) iters[t] = 0;
   } else if (active) {
     double T;
-    it = sat_cell<NY>(th, sc, o, uc, tg, T, fl);
+    if (ordinary) {
+      it = sat_cell<NY, canoe_thermo_t>(th, sc, o, uc, tg, T, fl);
+    } else {
+      double ua[S::NV], Ta;
+      int fa = 0;
+#pragma unroll
+      for (int n = 0; n < S::NV; ++n) ua[n] = uc[n];
+      it = sat_cell_any<NY>(th, sc, o, ua, tg, Ta, fa);
+#pragma unroll
+      for (int n = 0; n < S::NV; ++n) uc[n] = ua[n];
+      T = Ta;
+      fl = fa;
+    }
     if (!(fl & 4)) {
 #pragma unroll
       for (int n = 1; n <= NY; ++n) u[n * stride + off] = uc[n];
@@ -639,7 +692,8 @@ __device__ __forceinline__ void satadj_chunk(
 // registers)
 template <int NY>
 __global__ void __launch_bounds__(256, 3)
-    k_satadj(canoe_thermo_t th, canoe_satadj_opts_t o, double *__restrict__ u,
+    k_satadj(const __grid_constant__ canoe_thermo_t th,
+             const __grid_constant__ canoe_satadj_opts_t o, double *__restrict__ u,
              int64_t ncells, int64_t stride, Geom g, int use_geom,
              const double *__restrict__ t_guess, double *__restrict__ t_out,
              int32_t *__restrict__ iters, unsigned long long *stats) {
@@ -661,7 +715,8 @@ __global__ void __launch_bounds__(256, 3)
 // kSatWg, ..., independently of the CTA's other warpgroups.
 template <int NY>
 __global__ void __launch_bounds__(kSatWg * kUmmaM, 1)
-    k_satadj_learned(canoe_thermo_t th, canoe_satadj_opts_t o, double *__restrict__ u,
+    k_satadj_learned(const __grid_constant__ canoe_thermo_t th,
+                     const __grid_constant__ canoe_satadj_opts_t o, double *__restrict__ u,
                      int64_t ncells, int64_t stride, Geom g, int use_geom,
                      const double *__restrict__ t_guess, double *__restrict__ t_out,
                      int32_t *__restrict__ iters, unsigned long long *stats, MlpView mv,

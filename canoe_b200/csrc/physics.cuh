@@ -8,6 +8,8 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "../../include/canoe_b200.h"
 
 namespace cb {
@@ -33,9 +35,11 @@ struct Slots {
 //     IBM J. Res. Dev. 34, 1990)
 //   square root: Goldschmidt's coupled iteration on the hardware's reciprocal
 //     root, corrected by its residual (Markstein 1990)
-// Both come out correctly rounded (2^21 random operands of each type; one unit
-// in the last place is what tests/test_gpu_fastmath.py demands).  A zero or
-// infinite divisor gives NaN.  Measured, x1 stage at 128x256x256 moist: FP64
+// Within one unit in the last place (tests/test_gpu_fastmath.py; its 2^20 operands
+// of each type all came out correctly rounded), for normal operands whose result
+// is normal.  A divisor that is zero, infinite or subnormal gives NaN, one above
+// 2^1022 (FP32: 2^126) zero: no valid state holds one, and the entry points that
+// take any state divide as IEEE does (ExactThermo).  Measured, x1 stage at 128x256x256 moist: FP64
 // 1.95 -> 1.62 ms, FP32 1.19 -> 1.16 ms.
 template <typename R>
 struct Recip {
@@ -108,6 +112,28 @@ inline Mix<R> make_mix(const canoe_thermo_t &th) {
   }
   return m;
 }
+// canoe_thermo_t for the entry points that solve whatever states a caller has:
+// the solvers then divide and take roots as IEEE does at every operand
+struct ExactThermo : canoe_thermo_t {};
+template <class TH, typename R>
+__device__ __forceinline__ R tdiv(R a, R b) {
+  if constexpr (std::is_same<TH, ExactThermo>::value) return a / b;
+  else return qdiv(a, b);
+}
+template <class TH, typename R>
+__device__ __forceinline__ R tsqrt(R x) {
+  if constexpr (std::is_same<TH, ExactThermo>::value) return sqrt(x);
+  else return qsqrt(x);
+}
+template <typename R>
+struct ExactRecip {
+  R b;
+  __device__ __forceinline__ explicit ExactRecip(R b_) : b(b_) {}
+  __device__ __forceinline__ R of(R a) const { return a / b; }
+};
+template <class TH, typename R>
+using TRecip = typename std::conditional<std::is_same<TH, ExactThermo>::value, ExactRecip<R>,
+                                         Recip<R>>::type;
 template <typename R>
 __device__ __forceinline__ R mix_gm1(const canoe_thermo_t &th) { return R(th.gammad - 1.); }
 template <typename R>
@@ -127,14 +153,14 @@ __device__ __forceinline__ R get_gamma(const TH &th, const R *w) {
     else
       feps -= w[n];
   }
-  return R(1) + qdiv(mix_gm1<R>(th) * feps, fsig);
+  return R(1) + tdiv<TH>(mix_gm1<R>(th) * feps, fsig);
 }
 
 // EquationOfState::SoundSpeed (canoe src/snap/eos/ideal_moist_hydro.cpp:87-91)
 template <typename R, int NY, class TH>
 __device__ __forceinline__ R sound_speed(const TH &th, const R *w) {
   R gamma = get_gamma<R, NY>(th, w);
-  return qsqrt(qdiv(gamma * w[Slots<NY>::IPR], w[0]));
+  return tsqrt<TH>(tdiv<TH>(gamma * w[Slots<NY>::IPR], w[0]));
 }
 
 // ---------------------------------------------------------------------------
@@ -227,21 +253,22 @@ __device__ __forceinline__ void lmars(const TH &th, const R *wli,
   constexpr int ivy = S::IVX + (DIR + 1) % 3;
   constexpr int ivz = S::IVX + (DIR + 2) % 3;
   constexpr int ipr = S::IPR;
-  R kappal = qdiv(R(1), get_gamma<R, NY>(th, wli) - R(1));
-  R kappar = qdiv(R(1), get_gamma<R, NY>(th, wri) - R(1));
+  R kappal = tdiv<TH>(R(1), get_gamma<R, NY>(th, wli) - R(1));
+  R kappar = tdiv<TH>(R(1), get_gamma<R, NY>(th, wri) - R(1));
   // (which product is fused into the sum is fixed here)
-  R hl = fma(qdiv(wli[ipr], wli[0]), kappal + R(1),
+  R hl = fma(tdiv<TH>(wli[ipr], wli[0]), kappal + R(1),
              R(0.5) * (wli[ivx] * wli[ivx] + wli[ivy] * wli[ivy] + wli[ivz] * wli[ivz]));
-  R hr = fma(qdiv(wri[ipr], wri[0]), kappar + R(1),
+  R hr = fma(tdiv<TH>(wri[ipr], wri[0]), kappar + R(1),
              R(0.5) * (wri[ivx] * wri[ivx] + wri[ivy] * wri[ivy] + wri[ivz] * wri[ivz]));
   R rhobar = R(0.5) * (wli[0] + wri[0]);
-  R cbar = qsqrt(qdiv(R(0.5) * (R(1) + (qdiv(R(1), kappar) + qdiv(R(1), kappal)) / R(2)) *
-                          (wli[ipr] + wri[ipr]),
-                      rhobar));
+  R cbar = tsqrt<TH>(
+      tdiv<TH>(R(0.5) * (R(1) + (tdiv<TH>(R(1), kappar) + tdiv<TH>(R(1), kappal)) / R(2)) *
+                   (wli[ipr] + wri[ipr]),
+               rhobar));
   R pbar = R(0.5) * (wli[ipr] + wri[ipr]) +
            R(0.5) * (rhobar * cbar) * (wli[ivx] - wri[ivx]);
   R ubar = R(0.5) * (wli[ivx] + wri[ivx]) +
-           qdiv(R(0.5), rhobar * cbar) * (wli[ipr] - wri[ipr]);
+           tdiv<TH>(R(0.5), rhobar * cbar) * (wli[ipr] - wri[ipr]);
   R rdl = R(1), rdr = R(1);
 #pragma unroll
   for (int n = 1; n <= NY; ++n) {
@@ -295,11 +322,11 @@ __device__ __forceinline__ void hllc(const TH &th, const R *wl,
   wri[IPR] = wr[IPR];
 
   R gammal = get_gamma<R, NY>(th, wli);
-  R kappal = qdiv(R(1), gammal - R(1));
+  R kappal = tdiv<TH>(R(1), gammal - R(1));
   R gammar = get_gamma<R, NY>(th, wri);
-  R kappar = qdiv(R(1), gammar - R(1));
-  R cl = qsqrt(qdiv(gammal * wli[IPR], wli[0]));
-  R cr = qsqrt(qdiv(gammar * wri[IPR], wri[0]));
+  R kappar = tdiv<TH>(R(1), gammar - R(1));
+  R cl = tsqrt<TH>(tdiv<TH>(gammal * wli[IPR], wli[0]));
+  R cr = tsqrt<TH>(tdiv<TH>(gammar * wri[IPR], wri[0]));
   R KE_l, KE_r;
   if constexpr (COVKE) {
     R vy = wli[IVY] + wli[IVZ] * ke_cth, vz = wli[IVZ] + wli[IVY] * ke_cth;
@@ -318,10 +345,10 @@ __device__ __forceinline__ void hllc(const TH &th, const R *wl,
   R pmid = R(.5) * (wli[IPR] + wri[IPR] + (wli[IVX] - wri[IVX]) * rhoa * ca);
   R ql = (pmid <= wli[IPR])
              ? R(1)
-             : qsqrt(R(1) + qdiv(gammal + R(1), R(2) * gammal) * (qdiv(pmid, wli[IPR]) - R(1)));
+             : tsqrt<TH>(R(1) + tdiv<TH>(gammal + R(1), R(2) * gammal) * (tdiv<TH>(pmid, wli[IPR]) - R(1)));
   R qr = (pmid <= wri[IPR])
              ? R(1)
-             : qsqrt(R(1) + qdiv(gammar + R(1), R(2) * gammar) * (qdiv(pmid, wri[IPR]) - R(1)));
+             : tsqrt<TH>(R(1) + tdiv<TH>(gammar + R(1), R(2) * gammar) * (tdiv<TH>(pmid, wri[IPR]) - R(1)));
   R al = wli[IVX] - cl * ql;
   R ar = wri[IVX] + cr * qr;
   R bp = ar > R(0) ? ar : R(TINY_NUMBER);
@@ -332,7 +359,7 @@ __device__ __forceinline__ void hllc(const TH &th, const R *wl,
   R tr = wri[IPR] + vxr * wri[0] * wri[IVX];
   R ml = wli[0] * vxl;
   R mr = -(wri[0] * vxr);
-  const Recip<R> im(ml + mr);
+  const TRecip<TH, R> im(ml + mr);
   R am = im.of(tl - tr);
   R cp = im.of(ml * tr + mr * tl);
   cp = cp > R(0) ? cp : R(0);
@@ -345,7 +372,7 @@ __device__ __forceinline__ void hllc(const TH &th, const R *wl,
     rdr -= wri[n];
   }
   const bool pos = am >= R(0);
-  const Recip<R> is(pos ? am - bm : bp - am);
+  const TRecip<TH, R> is(pos ? am - bm : bp - am);
   const R s = is.of(pos ? am : -am), sm = is.of(pos ? -bm : bp);
   const R sl = pos ? s : R(0), sr = pos ? R(0) : s;
   R f[S::NV];
