@@ -28,6 +28,15 @@ CB_DECL2(6)
 #undef CB_DECL2
 #undef CB_DECL
 
+// tiles of a march that shared memory lets an SM hold at once
+template <int NY, typename R, int N, int GEO>
+static int march_resident(int nc1, int per_sm, int reserved) {
+  const size_t b = nc1 % 2 ? MarchSmem<5 + NY, march_chunk<R>(NY, N, 1), R, GEO, N>::bytes(nc1)
+                           : MarchSmem<5 + NY, march_chunk<R>(NY, N, 0), R, GEO, N>::bytes(nc1);
+  constexpr int kStatic = 1024;  // the kernel's barriers and column table
+  return (int)(per_sm / (b + kStatic + reserved));
+}
+
 // whether the fused x1 stage of a block marches, its scratch granted
 static bool march_serves(const Geom &g, const canoe_thermo_t &th, int flag, int prec) {
   const int64_t ncol = (int64_t)g.nx2 * g.nx3 * (g.npanel > 1 ? g.npanel : 1);
@@ -36,9 +45,38 @@ static bool march_serves(const Geom &g, const canoe_thermo_t &th, int flag, int 
   // decomposition, with du initialised by an x2 pass
   if (!(flag & 1) || lines || g.bc[0] == CANOE_BC_PERIODIC || th.grav == 0. || !g.f2) return false;
   const int n = flag & 8 ? 5 : 3;
-  const int least = n == 5 ? kMarchMinCols5
-                           : (prec == CANOE_FP32_PERTURBATION ? kMarchMinCols32 : kMarchMinCols64);
+  const bool f32 = prec == CANOE_FP32_PERTURBATION;
+  const int least = n == 5 ? kMarchMinCols5 : (f32 ? kMarchMinCols32 : kMarchMinCols64);
   if (ncol < least || !march_available()) return false;
+  if (n == 3 && !g.shell) {
+    int dev = 0, sms = 0, per_sm = 0, reserved = 0, resident = 0;
+    if (cudaGetDevice(&dev) ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) ||
+        cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) ||
+        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev)) {
+      cudaGetLastError();
+      return false;
+    }
+#define CB_RES(NY)                                                               \
+  case NY:                                                                       \
+    resident = f32 ? march_resident<NY, float, 3, 0>(g.nc1, per_sm, reserved)    \
+                   : march_resident<NY, double, 3, 0>(g.nc1, per_sm, reserved);  \
+    break;
+    switch (th.ny) { CB_RES(0) CB_RES(1) CB_RES(2) CB_RES(3) CB_RES(6) }
+#undef CB_RES
+    if (resident < 1) return false;
+    const MarchTile t = march_tile(g.nx1, g.nx2, g.nx3);
+    const int64_t tiles = (int64_t)t.nj * t.nk;
+    if (resident == 1) {
+      const int64_t rounds = (tiles + sms - 1) / sms;
+      // (columns so long that eight variables fill an SM too are the other
+      // kernel's worst: 64x54 of 330 levels 2676 and 1265 us in FP32)
+      if (th.ny > 3 && ncol * 16 < least * rounds * march_round_16ths(g.nx1, f32)) return false;
+    } else if (!f32 && tiles > sms && g.nx1 >= kMarchPairsLo && g.nx1 <= kMarchPairsHi &&
+               ncol < kMarchMinCols64Pairs) {
+      return false;
+    }
+  }
   // columns too long for the CTA-per-column kernel stay refused there
   return sizeof(double) * col_smem(g.nv, g.nc1, g.nx1, n, 0, 1).total <= 227 * 1024;
 }

@@ -57,14 +57,29 @@ namespace cb {
 
 constexpr int kMarchCols = 32;  // columns per CTA
 constexpr int kMarchUp = 4;     // levels per chunk of the way back up
-// Fewest columns that march.  A tile takes the same time alone on an SM as
-// beside another, so up to 148 tiles (4736 columns) the march takes as long as
-// for one: 128 levels 121 us in FP32, 186 us in FP64, where the CTA-per-column
-// kernel takes 38 and 46 ns a column.
+// Fewest columns that march.  As long as every tile has an SM to itself (148
+// tiles, 4736 columns) the march takes as long as for one: 128 levels of eight
+// variables 121 us in FP32, 186 us in FP64, where the CTA-per-column kernel takes
+// 38 and 46 ns a column.
 constexpr int kMarchMinCols32 = 3400, kMarchMinCols64 = 4300;
 // with 5x5 blocks one tile fills an SM: 128 levels 227 us a round of 148 tiles
 // against 188 ns a column
 constexpr int kMarchMinCols5 = 1200;
+// Two tiles on an SM get in each other's way in FP64: 65x67 columns, 153 tiles,
+// of 128 levels take 1172 us a step marching, 1092 with a CTA per column, and
+// 69x70, 162 tiles, 1188 and 1171.  Outside these numbers of levels, where the
+// other kernel is the slower one (16: 375 and 276 us), the line stays.
+constexpr int kMarchMinCols64Pairs = 4800, kMarchPairsLo = 32, kMarchPairsHi = 150;
+// Where shared memory holds one tile on an SM (six species but for even columns
+// in FP32), 3x3 blocks march in rounds of 148 tiles, each of which has to pay
+// for itself: so many sixteenths of the least columns, by the number of levels.
+// Six species of 65 levels, 69x70 columns in two rounds: 893 us a step with a
+// CTA per column, 1229 marching in FP32, 1270 and 1635 in FP64; 64x74 columns in
+// one: 1043 and 858 in FP64.  Of 16 levels 69x70 columns take 492 and 434 us, of
+// 160 levels 64x100 columns, in two rounds too, 2563 and 2281.
+constexpr int march_round_16ths(int nx1, bool f32) {
+  return nx1 < 32 ? 8 : (nx1 <= 128 ? (f32 ? 16 : 15) : 11);
+}
 
 // scratch per level of a tile with N x N blocks: H and g (a tile's levels
 // contiguous); then du of the two transverse momenta (N = 3, whose solve

@@ -6,8 +6,8 @@ import ctypes
 import numpy as np
 import pytest
 
-from canoe_b200 import Batch, CanoeError, Mesh, MeshBlock, Shell, problems
-from canoe_b200._abi import check, load
+from canoe_b200 import Batch, CanoeError, Mesh, MeshBlock, Shell, problems, thermo
+from canoe_b200._abi import FP32_PERTURBATION, check, load
 from test_gpu_march import _perturbed, _rel
 
 pytestmark = pytest.mark.gpu
@@ -159,3 +159,19 @@ def test_autotuner_leaves_marching_blocks_alone():
     assert [t for t, _ in bt.shapes()] == list(choice)
     for b, r in zip(blocks, ref):
         assert np.array_equal(b.conserved(), r)
+
+
+# one tile on an SM (six species, FP64 and odd FP32 columns): rounds of 148 tiles; two: FP64 columns
+# of 32 to 150 levels in more than 148 tiles
+@pytest.mark.parametrize("ny,f32,nx1,nx2,nx3,marches", [
+    (6, 0, 65, 69, 70, False), (6, 0, 65, 64, 74, True), (6, 0, 16, 69, 70, True),
+    (6, 0, 160, 64, 100, True), (6, 1, 65, 69, 70, False), (6, 1, 64, 69, 70, True),
+    (3, 0, 128, 65, 67, False), (3, 0, 128, 69, 70, True), (3, 0, 16, 65, 67, True),
+    (3, 0, 160, 65, 67, True), (3, 1, 128, 58, 59, True), (3, 0, 330, 64, 100, True)])
+def test_rule(ny, f32, nx1, nx2, nx3, marches):
+    th = thermo.earth_water_ammonia() if ny == 6 else thermo.earth_moist()
+    p = problems.moist3d(nx1=nx1, nx2=nx2, nx3=nx3, x1max=100.0 * nx1, x2max=250.0 * nx2,
+                         x3max=250.0 * nx3, th=th, satadj=0)
+    if f32:
+        p.cfg.precision = FP32_PERTURBATION
+    assert MeshBlock(p).marches() == marches
