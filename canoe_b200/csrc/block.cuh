@@ -163,6 +163,8 @@ int validate_block_config(const canoe_block_config_t &c);
 
 // raise a kernel's dynamic shared-memory limit once per (kernel, size)
 int ensure_smem(const void *kernel, size_t bytes);
+// multiprocessors of the current device (0: no answer)
+int sm_count();
 
 
 }  // namespace cb

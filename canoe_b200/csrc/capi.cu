@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -40,6 +41,18 @@ int ensure_smem(const void *kernel, size_t bytes) {
                                  (int)bytes));
   done[kernel] = bytes;
   return 0;
+}
+
+int sm_count() {
+  static std::atomic<int> known[64];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev < 64 && (n = known[dev].load()) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (dev < 64) known[dev].store(n);
+  return n;
 }
 
 namespace {

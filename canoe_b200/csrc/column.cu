@@ -49,9 +49,9 @@ static bool march_serves(const Geom &g, const canoe_thermo_t &th, int flag, int 
   const int least = n == 5 ? kMarchMinCols5 : (f32 ? kMarchMinCols32 : kMarchMinCols64);
   if (ncol < least || !march_available()) return false;
   if (n == 3 && !g.shell) {
-    int dev = 0, sms = 0, per_sm = 0, reserved = 0, resident = 0;
-    if (cudaGetDevice(&dev) ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) ||
+    const int sms = sm_count();
+    int dev = 0, per_sm = 0, reserved = 0, resident = 0;
+    if (sms < 1 || cudaGetDevice(&dev) ||
         cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) ||
         cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev)) {
       cudaGetLastError();

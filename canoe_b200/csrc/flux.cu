@@ -294,8 +294,8 @@ __global__ void __launch_bounds__(32 * RBY)
   }
 }
 
-// warps below which the default runs get shorter: four per SM
-constexpr int kRunMinWarps = 4 * 148;
+// warps per SM below which the default runs get shorter
+constexpr int kRunMinWarps = 4;
 
 // 1: the x2 / x3 fluxes run as k_flux_x23_run, 0: as the tile kernel
 constexpr int kFluxRun = 1;
@@ -316,10 +316,12 @@ int run_x23(const Geom &g, const canoe_thermo_t &th, const double *w, double *du
   // its runs are halved, at two extra cells a run, until there are four warps
   // per SM or two cells per run (13 us)
   int RL = g.flux_run;
-  if (RL <= 0)
+  if (RL <= 0) {
+    const int least = kRunMinWarps * sm_count();
     for (RL = run_len<R>();
-         RL > 2 && (int64_t)((g.nx1 + 31) / 32) * no * ((nd + RL - 1) / RL) < kRunMinWarps;)
+         RL > 2 && (int64_t)((g.nx1 + 31) / 32) * no * ((nd + RL - 1) / RL) < least;)
       RL /= 2;
+  }
   // a 2-D block (one line across the flux direction) keeps the tile kernel:
   // its runs would fill one warp in four of each CTA, and the 150 x 100
   // bubble would march 20 warps in all (x2 pass 4 x slower than the tiles);
