@@ -46,9 +46,8 @@ struct Geom {
   // (the six panels of a cubed-sphere shell share one geometry)
   int npanel = 1;
   int64_t pstride = 0;
-  // scratch of the column march and its RK register u1 (march.cuh), from
-  // march_scratch(); null: the fused x1 stage runs one CTA per column
-  // (column.cuh)
+  // scratch of the column march and its RK register u1 (march.cuh), from a
+  // MarchClaim; null: the fused x1 stage runs one CTA per column (column.cuh)
   double *march = nullptr, *march_u1 = nullptr;
   // polls after which the march's bounded waits give up, on its way down and
   // back up (canoe_selftest_march_wait)
@@ -98,15 +97,30 @@ int launch_x1col(const Geom &g, const canoe_thermo_t &th, int recon, int rs,
                  int implicit_flag, int precision, int mode, const double *w, double *du, double *u,
                  double *u1, const double *dtp, const Stage &s, int stage,
                  double *flx_out, cudaStream_t st);
-// Decides whether a block's fused x1 stage marches down its columns (march.cuh):
-// sets g.march and g.march_u1 and returns the scratch for the owner to free, or
-// nulls when the block keeps the CTA-per-column kernel (too few columns, a form
-// the march does not provide, or no memory left).  u1: the block's register
-// array, which the march lays out in its own order
-double *march_scratch(Geom &g, const canoe_thermo_t &th, int implicit_flag, int precision,
-                      double *u1, size_t u1_doubles);
-// the device's memory that the march's scratch leaves free: one in so many
-constexpr int kMarchReserve = 32;
+// A block's (or shell's) claim to the column march of its fused x1 stage
+// (march.cuh), whose scratch g->march it owns.  The scratch (128x256x256 moist:
+// 1.21 GB beside a block's 2.15) is taken when the block is created, while half
+// of the device stays free; else at its first step, while one part in
+// kMarchReserve does.  Until that step it is given back to any block that finds
+// no memory for its own arrays (block_malloc), so that as many blocks fit a
+// device as without the march.  From the first step on the choice stands.
+struct MarchClaim {
+  Geom *g = nullptr;
+  const canoe_thermo_t *th = nullptr;
+  int flag = 0, dev = 0;
+  double *u1 = nullptr;  // the block's register array, which the march lays out in its own order
+  size_t u1_doubles = 0;
+  bool serves = false;   // the march provides the form and pays for the columns
+  bool allowed = true, decided = false;
+};
+constexpr int kMarchEager = 2, kMarchReserve = 32;
+void march_create(MarchClaim &c, Geom *g, const canoe_thermo_t *th, int implicit_flag,
+                  int precision, double *u1, size_t u1_doubles);
+bool march_allow(MarchClaim &c, bool on);  // false once decided
+bool march_decide(MarchClaim &c);          // whether the x1 stage marches
+void march_destroy(MarchClaim &c);
+// cudaMalloc for the arrays that a block cannot do without
+cudaError_t block_malloc(void **p, size_t bytes);
 // implicit solves along x2 (dir 1) and x3 (dir 2) of a dry block (lines.cu):
 // whether the flag asks for one in a direction the block has, the doubles
 // of each of the two line-major scratch arrays, and the solve of du in place

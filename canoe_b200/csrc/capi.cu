@@ -155,9 +155,7 @@ struct canoe_block {
   // x2 / x3 implicit solves: line-major scratch of w and du, line spacings
   // (nx2 + 2 NG entries of dx2, then nx3 + 2 NG of dx3)
   double *d_wt = nullptr, *d_dut = nullptr, *d_dxl = nullptr;
-  double *d_march = nullptr;  // scratch of the column march (Geom::march)
-  bool march = true;          // the x1 stage may march
-  bool stepped = false;       // whether it does is decided
+  MarchClaim march;  // of the x1 stage
   bool lines = false;
   cudaStream_t st = nullptr;
   bool own_stream = false;
@@ -248,12 +246,13 @@ int validate_block_config(const canoe_block_config_t &c) {
 
 static int block_free(canoe_block *b) {
   if (!b) return 0;
+  march_destroy(b->march);
   if (b->gexec) cudaGraphExecDestroy(b->gexec);
   for (void *p : {(void *)b->d_u, (void *)b->d_w, (void *)b->d_u1, (void *)b->d_du,
                   (void *)b->d_x1f, (void *)b->d_x1v, (void *)b->d_dx1f,
                   (void *)b->d_scr, (void *)b->d_dt, (void *)b->d_pref, (void *)b->d_dtacc,
                   (void *)b->d_err, (void *)b->d_sat, (void *)b->d_wt, (void *)b->d_dut,
-                  (void *)b->d_dxl, (void *)b->d_march})
+                  (void *)b->d_dxl})
     if (p) cudaFree(p);
   if (b->own_stream && b->st) cudaStreamDestroy(b->st);
   delete b;
@@ -286,21 +285,12 @@ static int line_solves(canoe_block *b, double *du, const double *dtp, const Stag
   return 0;
 }
 
-// whether the x1 stage of b marches, decided once: a step's stages share u1
-static void decide_march(canoe_block *b) {
-  if (b->stepped) return;
-  b->stepped = true;
-  if (b->march)
-    b->d_march = march_scratch(b->g, b->th, b->cfg.implicit_flag, b->cfg.precision, b->d_u1,
-                               b->nvals);
-}
-
 // one RK stage of block b on stream st (the per-stage task list up to
 // cons2prim with the physical boundaries); dtp: the step's device dt, acc:
 // the CFL accumulator fed at the last stage
 static int stage_launches(canoe_block *b, int s, double *dtp, unsigned long long *acc,
                           cudaStream_t st, StepTimer *tm = nullptr) {
-  decide_march(b);
+  march_decide(b->march);
   const Geom &g = b->g;
   const Stage &sg = kRK3[s];
   int rc;
@@ -473,19 +463,19 @@ int canoe_block_create(const canoe_block_config_t *cfg, canoe_block_t *out) {
     return rc;
   };
   cudaError_t e;
-  if ((e = cudaMalloc(&b->d_u, bytes))) return fail(e, "cudaMalloc u");
-  if ((e = cudaMalloc(&b->d_w, bytes))) return fail(e, "cudaMalloc w");
-  if ((e = cudaMalloc(&b->d_u1, bytes))) return fail(e, "cudaMalloc u1");
-  if ((e = cudaMalloc(&b->d_du, bytes))) return fail(e, "cudaMalloc du");
-  if ((e = cudaMalloc(&b->d_x1f, (g.nc1 + 1) * sizeof(double)))) return fail(e, "cudaMalloc x1f");
-  if ((e = cudaMalloc(&b->d_x1v, g.nc1 * sizeof(double)))) return fail(e, "cudaMalloc x1v");
-  if ((e = cudaMalloc(&b->d_dx1f, g.nc1 * sizeof(double)))) return fail(e, "cudaMalloc dx1f");
-  if ((e = cudaMalloc(&b->d_dt, 2 * sizeof(double)))) return fail(e, "cudaMalloc dt");
-  if ((e = cudaMalloc(&b->d_pref, g.nc1 * sizeof(double)))) return fail(e, "cudaMalloc pref");
+  if ((e = block_malloc((void **)&b->d_u, bytes))) return fail(e, "cudaMalloc u");
+  if ((e = block_malloc((void **)&b->d_w, bytes))) return fail(e, "cudaMalloc w");
+  if ((e = block_malloc((void **)&b->d_u1, bytes))) return fail(e, "cudaMalloc u1");
+  if ((e = block_malloc((void **)&b->d_du, bytes))) return fail(e, "cudaMalloc du");
+  if ((e = block_malloc((void **)&b->d_x1f, (g.nc1 + 1) * sizeof(double)))) return fail(e, "cudaMalloc x1f");
+  if ((e = block_malloc((void **)&b->d_x1v, g.nc1 * sizeof(double)))) return fail(e, "cudaMalloc x1v");
+  if ((e = block_malloc((void **)&b->d_dx1f, g.nc1 * sizeof(double)))) return fail(e, "cudaMalloc dx1f");
+  if ((e = block_malloc((void **)&b->d_dt, 2 * sizeof(double)))) return fail(e, "cudaMalloc dt");
+  if ((e = block_malloc((void **)&b->d_pref, g.nc1 * sizeof(double)))) return fail(e, "cudaMalloc pref");
   if ((e = cudaMemset(b->d_pref, 0, g.nc1 * sizeof(double)))) return fail(e, "cudaMemset pref");
-  if ((e = cudaMalloc(&b->d_dtacc, sizeof(unsigned long long)))) return fail(e, "cudaMalloc dtacc");
-  if ((e = cudaMalloc(&b->d_err, sizeof(uint32_t)))) return fail(e, "cudaMalloc err");
-  if ((e = cudaMalloc(&b->d_sat, 4 * sizeof(unsigned long long)))) return fail(e, "cudaMalloc sat");
+  if ((e = block_malloc((void **)&b->d_dtacc, sizeof(unsigned long long)))) return fail(e, "cudaMalloc dtacc");
+  if ((e = block_malloc((void **)&b->d_err, sizeof(uint32_t)))) return fail(e, "cudaMalloc err");
+  if ((e = block_malloc((void **)&b->d_sat, 4 * sizeof(unsigned long long)))) return fail(e, "cudaMalloc sat");
   if ((e = cudaMemset(b->d_sat, 0, 4 * sizeof(unsigned long long)))) return fail(e, "cudaMemset sat");
   if ((e = cudaMemset(b->d_u, 0, bytes))) return fail(e, "cudaMemset u");
   if ((e = cudaMemset(b->d_w, 0, bytes))) return fail(e, "cudaMemset w");
@@ -502,16 +492,17 @@ int canoe_block_create(const canoe_block_config_t *cfg, canoe_block_t *out) {
   b->lines = line_solve_on(g, cfg->implicit_flag, 1) || line_solve_on(g, cfg->implicit_flag, 2);
   if (b->lines) {
     const size_t nl = line_scratch_doubles(g, cfg->implicit_flag) * sizeof(double);
-    if ((e = cudaMalloc(&b->d_wt, nl))) return fail(e, "cudaMalloc line scratch");
-    if ((e = cudaMalloc(&b->d_dut, nl))) return fail(e, "cudaMalloc line scratch");
+    if ((e = block_malloc((void **)&b->d_wt, nl))) return fail(e, "cudaMalloc line scratch");
+    if ((e = block_malloc((void **)&b->d_dut, nl))) return fail(e, "cudaMalloc line scratch");
     const int n2 = g.nx2 + 2 * NG, n3 = g.nx3 + 2 * NG;
     std::vector<double> dl(n2 + n3);
     for (int q = 0; q < n2; ++q) dl[q] = g.dx2;
     for (int q = 0; q < n3; ++q) dl[n2 + q] = g.dx3;
-    if ((e = cudaMalloc(&b->d_dxl, dl.size() * sizeof(double)))) return fail(e, "cudaMalloc dxl");
+    if ((e = block_malloc((void **)&b->d_dxl, dl.size() * sizeof(double)))) return fail(e, "cudaMalloc dxl");
     if ((e = cudaMemcpy(b->d_dxl, dl.data(), dl.size() * sizeof(double), cudaMemcpyHostToDevice)))
       return fail(e, "copy");
   }
+  march_create(b->march, &b->g, &b->th, cfg->implicit_flag, cfg->precision, b->d_u1, b->nvals);
   if ((e = cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking))) return fail(e, "stream");
   b->own_stream = true;
   g.x1f = b->d_x1f;
@@ -805,18 +796,16 @@ int canoe_block_set_column_threads(canoe_block_t b, int threads) {
 
 int canoe_block_set_march(canoe_block_t b, int on) {
   if (!b) return CANOE_ERR_ARG;
-  if (b->stepped) {
+  if (!march_allow(b->march, on != 0)) {
     set_error("canoe_block_set_march: before the block's first step");
     return CANOE_ERR_ARG;
   }
-  b->march = on != 0;
   return 0;
 }
 
 int canoe_block_marches(canoe_block_t b, int *marches) {
   if (!b || !marches) return CANOE_ERR_ARG;
-  decide_march(b);
-  *marches = b->d_march != nullptr;
+  *marches = march_decide(b->march);
   return 0;
 }
 
@@ -1309,7 +1298,7 @@ int canoe_batch_autotune(canoe_batch_t q, int32_t *h_threads) {
   for (size_t n = 0; n < nb && !rc; ++n) {
     canoe_block *b = q->blocks[n];
     const size_t bytes = b->nvals * sizeof(double);
-    if (cudaMalloc(&su[n], bytes) || cudaMalloc(&sw[n], bytes)) {
+    if (block_malloc((void **)&su[n], bytes) || block_malloc((void **)&sw[n], bytes)) {
       rc = cuda_status(cudaErrorMemoryAllocation, "canoe_batch_autotune");
       break;
     }
@@ -1331,11 +1320,11 @@ int canoe_batch_autotune(canoe_batch_t q, int32_t *h_threads) {
   for (size_t n = 0; n < nb && !rc; ++n) {
     canoe_block *b = q->blocks[n];
     float best = 1e30f, ms = 0.f;
-    decide_march(b);
-    int pick = b->d_march ? 0 : kColThreads;
+    const bool march = march_decide(b->march);
+    int pick = march ? 0 : kColThreads;
     b->g.flux_run = 0;
     for (int c : cand) {
-      if (b->d_march) break;
+      if (march) break;
       b->g.col_threads = c;
       rc = step_launches(b, 0.);
       if (!rc) {

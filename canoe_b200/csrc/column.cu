@@ -1,5 +1,8 @@
 // column.cu -- dispatch of the x1 pencil kernel and of the column march over
 // the species count.
+#include <mutex>
+#include <set>
+
 #include "march.cuh"
 
 namespace cb {
@@ -81,18 +84,16 @@ static bool march_serves(const Geom &g, const canoe_thermo_t &th, int flag, int 
   return sizeof(double) * col_smem(g.nv, g.nc1, g.nx1, n, 0, 1).total <= 227 * 1024;
 }
 
-// Taken at a block's first step, not when it is created: a program makes its
-// blocks first, and as many fit the device as without the march (128x256x256
-// moist: 2.15 GB a block, and 1.21 GB of scratch).  A share of the device stays
-// free for what the program allocates later.
-double *march_scratch(Geom &g, const canoe_thermo_t &th, int flag, int prec, double *u1,
-                      size_t u1_doubles) {
-  g.march = g.march_u1 = nullptr;
-  if (!march_serves(g, th, flag, prec)) return nullptr;
-  const int n = flag & 8 ? 5 : 3;
+// claims with scratch whose block has not stepped, which may be given back
+static std::mutex claim_mu;
+static std::set<MarchClaim *> claims;
+
+static void claim_scratch(MarchClaim &c, size_t keep_free_one_in) {
+  Geom &g = *c.g;
+  const int n = c.flag & 8 ? 5 : 3;
   const size_t cells = march_cells(g.nx1, g.nx2, g.nx3, g.npanel > 1 ? g.npanel : 1);
-  const size_t scr = cells * (march_h(n) + march_nd(th.ny, n)), reg = cells * (5 + th.ny);
-  const bool own = reg > u1_doubles;  // ragged tiles of long columns: u1's array is too short
+  const size_t scr = cells * (march_h(n) + march_nd(c.th->ny, n)), reg = cells * (5 + c.th->ny);
+  const bool own = reg > c.u1_doubles;  // ragged tiles of long columns: u1's array is too short
   const size_t bytes = (scr + (own ? reg : 0)) * sizeof(double);
   // the first step may be captured into a graph, where other modes refuse an
   // allocation
@@ -100,7 +101,7 @@ double *march_scratch(Geom &g, const canoe_thermo_t &th, int flag, int prec, dou
   cudaThreadExchangeStreamCaptureMode(&mode);
   size_t left = 0, all = 0;
   double *p = nullptr;
-  if (cudaMemGetInfo(&left, &all) != cudaSuccess || left < bytes + all / kMarchReserve ||
+  if (cudaMemGetInfo(&left, &all) != cudaSuccess || left < bytes + all / keep_free_one_in ||
       cudaMalloc(&p, bytes) != cudaSuccess) {
     cudaGetLastError();
     p = nullptr;
@@ -108,9 +109,77 @@ double *march_scratch(Geom &g, const canoe_thermo_t &th, int flag, int prec, dou
   cudaThreadExchangeStreamCaptureMode(&mode);
   if (p) {
     g.march = p;
-    g.march_u1 = own ? p + scr : u1;
+    g.march_u1 = own ? p + scr : c.u1;
   }
-  return p;
+}
+
+static void drop_scratch(MarchClaim &c) {
+  if (c.g && c.g->march) cudaFree(c.g->march);
+  if (c.g) c.g->march = c.g->march_u1 = nullptr;
+}
+
+void march_create(MarchClaim &c, Geom *g, const canoe_thermo_t *th, int flag, int prec, double *u1,
+                  size_t u1_doubles) {
+  c.g = g;
+  c.th = th;
+  c.flag = flag;
+  c.u1 = u1;
+  c.u1_doubles = u1_doubles;
+  cudaGetDevice(&c.dev);
+  c.serves = march_serves(*g, *th, flag, prec);
+  if (!c.serves) return;
+  std::lock_guard<std::mutex> lk(claim_mu);
+  claim_scratch(c, kMarchEager);
+  if (g->march) claims.insert(&c);
+}
+
+bool march_allow(MarchClaim &c, bool on) {
+  std::lock_guard<std::mutex> lk(claim_mu);
+  if (c.decided) return false;
+  c.allowed = on;
+  if (!on) {
+    claims.erase(&c);
+    drop_scratch(c);
+  }
+  return true;
+}
+
+bool march_decide(MarchClaim &c) {
+  if (!c.decided) {
+    std::lock_guard<std::mutex> lk(claim_mu);
+    claims.erase(&c);
+    if (c.serves && c.allowed && !c.g->march) claim_scratch(c, kMarchReserve);
+    c.decided = true;
+  }
+  return c.g->march != nullptr;
+}
+
+void march_destroy(MarchClaim &c) {
+  std::lock_guard<std::mutex> lk(claim_mu);
+  claims.erase(&c);
+  drop_scratch(c);
+}
+
+cudaError_t block_malloc(void **p, size_t bytes) {
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  int dev = -1;
+  bool any = false;
+  cudaGetLastError();
+  cudaGetDevice(&dev);
+  {
+    std::lock_guard<std::mutex> lk(claim_mu);
+    for (auto it = claims.begin(); it != claims.end();) {
+      if ((*it)->dev == dev) {
+        drop_scratch(**it);
+        any = true;
+        it = claims.erase(it);
+      } else {
+        ++it;
+      }
+    }
+  }
+  return any ? cudaMalloc(p, bytes) : e;
 }
 
 template <int N>

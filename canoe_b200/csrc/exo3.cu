@@ -883,9 +883,8 @@ struct canoe_shell {
   canoe_thermo_t th;
   Geom g;
   int64_t pvals = 0;  // values per panel
-  double *d_march = nullptr;  // scratch of the column march (Geom::march)
-  bool march = true;          // the x1 stage may march
-  bool stepped = false;       // whether it does is decided
+  Geom g6;           // the six panels' x1 stage, one launch
+  MarchClaim march;  // of that stage
   double *d_u = nullptr, *d_w = nullptr, *d_u1 = nullptr, *d_du = nullptr;
   double *d_x1f = nullptr, *d_x1v = nullptr, *d_dx1f = nullptr, *d_dt = nullptr;
   double *d_tabs = nullptr, *d_lr = nullptr, *d_pref = nullptr;
@@ -900,7 +899,8 @@ struct canoe_shell {
 
 static int shell_free(canoe_shell *s) {
   if (!s) return 0;
-  for (void *p : {(void *)s->d_u, (void *)s->d_w, (void *)s->d_u1, (void *)s->d_du, (void *)s->d_march,
+  march_destroy(s->march);
+  for (void *p : {(void *)s->d_u, (void *)s->d_w, (void *)s->d_u1, (void *)s->d_du, 
                   (void *)s->d_x1f, (void *)s->d_x1v, (void *)s->d_dx1f, (void *)s->d_dt,
                   (void *)s->d_tabs, (void *)s->d_lr, (void *)s->d_pref, (void *)s->d_dtacc,
                   (void *)s->d_err,
@@ -1060,22 +1060,22 @@ int canoe_shell_create(const canoe_shell_config_t *cfg, canoe_shell_t *out) {
     shell_free(s);
     return rc;
   };
-  if ((e = cudaMalloc(&s->d_u, bytes))) return fail(e, "cudaMalloc u");
-  if ((e = cudaMalloc(&s->d_w, bytes))) return fail(e, "cudaMalloc w");
-  if ((e = cudaMalloc(&s->d_u1, bytes))) return fail(e, "cudaMalloc u1");
-  if ((e = cudaMalloc(&s->d_du, bytes))) return fail(e, "cudaMalloc du");
-  if ((e = cudaMalloc(&s->d_lr, lr_bytes))) return fail(e, "cudaMalloc lr");
-  if ((e = cudaMalloc(&s->d_x1f, xf.size() * sizeof(double)))) return fail(e, "cudaMalloc x1f");
-  if ((e = cudaMalloc(&s->d_x1v, xv.size() * sizeof(double)))) return fail(e, "cudaMalloc x1v");
-  if ((e = cudaMalloc(&s->d_dx1f, dx.size() * sizeof(double)))) return fail(e, "cudaMalloc dx1f");
-  if ((e = cudaMalloc(&s->d_dt, 2 * sizeof(double)))) return fail(e, "cudaMalloc dt");
-  if ((e = cudaMalloc(&s->d_pref, g.nc1 * sizeof(double)))) return fail(e, "cudaMalloc pref");
+  if ((e = block_malloc((void **)&s->d_u, bytes))) return fail(e, "cudaMalloc u");
+  if ((e = block_malloc((void **)&s->d_w, bytes))) return fail(e, "cudaMalloc w");
+  if ((e = block_malloc((void **)&s->d_u1, bytes))) return fail(e, "cudaMalloc u1");
+  if ((e = block_malloc((void **)&s->d_du, bytes))) return fail(e, "cudaMalloc du");
+  if ((e = block_malloc((void **)&s->d_lr, lr_bytes))) return fail(e, "cudaMalloc lr");
+  if ((e = block_malloc((void **)&s->d_x1f, xf.size() * sizeof(double)))) return fail(e, "cudaMalloc x1f");
+  if ((e = block_malloc((void **)&s->d_x1v, xv.size() * sizeof(double)))) return fail(e, "cudaMalloc x1v");
+  if ((e = block_malloc((void **)&s->d_dx1f, dx.size() * sizeof(double)))) return fail(e, "cudaMalloc dx1f");
+  if ((e = block_malloc((void **)&s->d_dt, 2 * sizeof(double)))) return fail(e, "cudaMalloc dt");
+  if ((e = block_malloc((void **)&s->d_pref, g.nc1 * sizeof(double)))) return fail(e, "cudaMalloc pref");
   if ((e = cudaMemset(s->d_pref, 0, g.nc1 * sizeof(double)))) return fail(e, "cudaMemset pref");
-  if ((e = cudaMalloc(&s->d_dtacc, sizeof(unsigned long long)))) return fail(e, "cudaMalloc acc");
-  if ((e = cudaMalloc(&s->d_err, sizeof(uint32_t)))) return fail(e, "cudaMalloc err");
-  if ((e = cudaMalloc(&s->d_tabs, tabs.size() * sizeof(double)))) return fail(e, "cudaMalloc tabs");
-  if ((e = cudaMalloc(&s->d_ghost, gr.size() * sizeof(GhostRow)))) return fail(e, "cudaMalloc ghost");
-  if ((e = cudaMalloc(&s->d_edge, er.size() * sizeof(EdgeRow)))) return fail(e, "cudaMalloc edge");
+  if ((e = block_malloc((void **)&s->d_dtacc, sizeof(unsigned long long)))) return fail(e, "cudaMalloc acc");
+  if ((e = block_malloc((void **)&s->d_err, sizeof(uint32_t)))) return fail(e, "cudaMalloc err");
+  if ((e = block_malloc((void **)&s->d_tabs, tabs.size() * sizeof(double)))) return fail(e, "cudaMalloc tabs");
+  if ((e = block_malloc((void **)&s->d_ghost, gr.size() * sizeof(GhostRow)))) return fail(e, "cudaMalloc ghost");
+  if ((e = block_malloc((void **)&s->d_edge, er.size() * sizeof(EdgeRow)))) return fail(e, "cudaMalloc edge");
   for (double *p : {s->d_u, s->d_w, s->d_u1, s->d_du})
     if ((e = cudaMemset(p, 0, bytes))) return fail(e, "cudaMemset state");
   if ((e = cudaMemset(s->d_lr, 0, lr_bytes))) return fail(e, "cudaMemset lr");
@@ -1101,6 +1101,11 @@ int canoe_shell_create(const canoe_shell_config_t *cfg, canoe_shell_t *out) {
   g.pref = s->d_pref;
   g.err = s->d_err;
   g.shell = s->d_tabs;
+  s->g6 = g;
+  s->g6.npanel = 6;
+  s->g6.pstride = s->pvals;
+  march_create(s->march, &s->g6, &s->th, cfg->implicit_flag, cfg->precision, s->d_u1,
+               6 * (size_t)s->pvals);
   *out = s;
   return 0;
 }
@@ -1181,34 +1186,18 @@ int canoe_shell_calculate_fluxes(canoe_shell_t s, double *d_f1, double *d_f2, do
   return 0;
 }
 
-// whether the x1 stage marches, its six panels in one launch, decided once: a
-// step's stages share u1
-static void decide_march(canoe_shell *s) {
-  if (s->stepped) return;
-  s->stepped = true;
-  if (!s->march) return;
-  Geom g6 = s->g;
-  g6.npanel = 6;
-  s->d_march = march_scratch(g6, s->th, s->cfg.implicit_flag, s->cfg.precision, s->d_u1,
-                             6 * (size_t)s->pvals);
-  s->g.march = g6.march;
-  s->g.march_u1 = g6.march_u1;
-}
-
 int canoe_shell_set_march(canoe_shell_t s, int on) {
   if (!s) return CANOE_ERR_ARG;
-  if (s->stepped) {
+  if (!march_allow(s->march, on != 0)) {
     set_error("canoe_shell_set_march: before the shell's first step");
     return CANOE_ERR_ARG;
   }
-  s->march = on != 0;
   return 0;
 }
 
 int canoe_shell_marches(canoe_shell_t s, int *marches) {
   if (!s || !marches) return CANOE_ERR_ARG;
-  decide_march(s);
-  *marches = s->d_march != nullptr;
+  *marches = march_decide(s->march);
   return 0;
 }
 
@@ -1217,7 +1206,7 @@ int canoe_shell_step(canoe_shell_t s, double dt) {
     set_error("canoe_shell_step: dt must be positive");
     return CANOE_ERR_ARG;
   }
-  decide_march(s);
+  march_decide(s->march);
   int rc;
   if ((rc = launch_dt_finalize(s->d_dt, s->d_dtacc, s->cfg.cfl, dt, s->st))) return rc;
   for (int stage = 0; stage < 3; ++stage) {
@@ -1226,10 +1215,7 @@ int canoe_shell_step(canoe_shell_t s, double dt) {
     if ((rc = shell_x23(s, 1, sg.beta, nullptr))) return rc;
     if ((rc = shell_x23(s, 2, sg.beta, nullptr))) return rc;
     {  // the six panels' x1 pencils in one launch
-      Geom g6 = s->g;
-      g6.npanel = 6;
-      g6.pstride = s->pvals;
-      if ((rc = launch_x1col(g6, s->th, s->cfg.recon, s->cfg.rsolver, s->cfg.implicit_flag,
+      if ((rc = launch_x1col(s->g6, s->th, s->cfg.recon, s->cfg.rsolver, s->cfg.implicit_flag,
                              s->cfg.precision, kColStep, s->d_w, s->d_du, s->d_u, s->d_u1,
                              s->d_dt, sg, stage, nullptr, s->st)))
         return rc;

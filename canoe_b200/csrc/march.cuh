@@ -18,11 +18,11 @@
 //   warps C and C + 1 eliminate the rows of the previous chunk downwards
 //     (forward_backward.hpp:15-91 with the sweep reversed), a row each in
 //     turn, so that one forms its row while the other finishes the row above:
-//     with the rows
-//     scaled by twice the cell's volume over its lower face area,
+//     with the rows scaled by twice the cell's volume over its lower face area,
 //     b' = A_i + J_{i-1} = -b, c' = A_{i+1} - J_{i+1} = -c,
 //     D_i = a_i - c'_i H_{i+1}, H_i = D_i^-1 b'_i,
-//     g_i = D_i^-1 (r_i + c'_i g_{i+1}).
+//     g_i = D_i^-1 (r_i + c'_i g_{i+1}); 5x5 blocks by LU, with pivoting where
+//     a pivot cancels
 // H, g and what the update needs of du go to a scratch array laid out
 // [tile][level][component][lane]; on the way up x_i = g_i + H_i x_{i-1}, then
 // the species correction and the register update (forward_backward.hpp:93-137,
@@ -42,8 +42,8 @@
 // blocks FP32 12.3 -> 3.1 ms.  What bounds it: a chunk is a chain of four
 // barrier-separated phases of dependent FP64 and FP32 arithmetic (about 10k
 // cycles for eight levels) that two CTAs per SM (shared memory) overlap: issue
-// 45 %, DRAM 44 % busy; its traffic is the algorithmic bytes and 2 x 136 B per
-// cell of scratch.
+// 46 %, DRAM 47 % busy; its traffic is the algorithmic bytes and 2 x 144 B per
+// cell of scratch (18 doubles with three species).
 #pragma once
 
 #include <cuda.h>

@@ -410,11 +410,12 @@ int canoe_block_set_column_threads(canoe_block_t b, int threads);
 
 /* Whether the fused x1 stage of a block of many columns may march down them, a
  * column per thread (on != 0, the default), or runs a CTA per column as small
- * blocks do.  Decided once, at the block's first step, where a block that
- * marches allocates its scratch (14 doubles a cell with the 3x3 solve, 15 + ny
- * with ny species; 30 or 31 + ny with the 5x5 solve) unless that would leave
- * less than a thirty-second of the device's memory free: CANOE_ERR_ARG
- * afterwards.
+ * blocks do.  Decided for good at the block's first step: CANOE_ERR_ARG
+ * afterwards.  Scratch (14 doubles a cell with the 3x3 solve, 15 + ny with ny
+ * species; 30 or 31 + ny with the 5x5 solve) is taken when the block is created
+ * if half of the device's memory stays free, else at the first step if a
+ * thirty-second does; before that step it is given back to any block or shell
+ * that finds no memory for its own arrays.
  * canoe_block_marches tells, and decides where no step has.  The two forms
  * eliminate in different orders: the same state to roundoff, not the same
  * bits.  So blocks that cut one domain give the bits of its single block where

@@ -1,5 +1,5 @@
 """Which blocks march down their columns (csrc/march.cuh) and what that costs and changes: scratch
-taken at the first step alone, the setting and the query, the kernel without scratch, equal bits
+that gives way to other blocks, the setting and the query, the kernel without scratch, equal bits
 among blocks of one route and roundoff across."""
 import ctypes
 
@@ -25,18 +25,50 @@ def _free():
     return torch.cuda.mem_get_info()[0]
 
 
-def test_scratch_is_taken_at_the_first_step():
-    p = _p(60, 100, 100)
+def _ballast(nbytes):
+    import torch
+    return torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+
+
+def _drop():
+    import torch
+    torch.cuda.empty_cache()
+
+
+def test_scratch_gives_way_to_a_block_until_the_first_step():
     MeshBlock(_p(8, 8, 8)).step(0.1)  # the library's own memory
-    f0 = _free()
-    b = MeshBlock(p)
-    f1 = _free()
+    p = _p(60, 100, 100)
     arrays = 4 * p.u.nbytes  # u, w, u1, du
-    assert f0 - f1 <= arrays + (16 << 20)
-    assert b.marches()
-    assert f1 - _free() >= 60 * 100 * 100 * 18 * 8
+    scratch = 60 * 100 * 100 * 18 * 8
+    f0 = _free()
+    a = MeshBlock(p)
+    assert f0 - _free() >= arrays + scratch
+    ballast = _ballast(_free() - arrays + scratch // 2)
+    b = MeshBlock(p)  # fits without a's scratch
+    assert not a.marches() and not b.marches()
+    del ballast
+    _drop()
+    a.step(0.2)
+    b.step(0.2)
+    assert np.array_equal(a.conserved(), b.conserved())
+    a.close()
     b.close()
     assert abs(f0 - _free()) <= 16 << 20
+
+
+def test_scratch_waits_for_the_first_step_where_memory_is_scarce():
+    p = _p(60, 100, 100)
+    a = MeshBlock(p)
+    ballast = _ballast(int(0.7 * _free()))
+    f0 = _free()
+    b = MeshBlock(p)
+    assert f0 - _free() <= 4 * p.u.nbytes + (16 << 20)
+    assert b.marches()
+    a.step(0.2)
+    b.step(0.2)
+    del ballast
+    _drop()
+    assert np.array_equal(a.conserved(), b.conserved())
 
 
 def test_setting_and_query():
@@ -78,13 +110,14 @@ def test_shell_setting_and_query():
 def test_block_without_room_for_scratch():
     import torch
     p = _p()
-    a, b = MeshBlock(p), MeshBlock(p)
+    b = MeshBlock(p)
     b.set_march(False)
     free, total = torch.cuda.mem_get_info()
-    ballast = torch.empty(free - total // 32, dtype=torch.uint8, device="cuda")
+    ballast = _ballast(free - total // 32)
+    a = MeshBlock(p)
     assert not a.marches()
     del ballast
-    torch.cuda.empty_cache()
+    _drop()
     a.step(0.2)
     b.step(0.2)
     assert not a.marches()
