@@ -489,17 +489,23 @@ __device__ __forceinline__ double mlp_features(const canoe_thermo_t &th, const S
   return tdiv<TH>(ev, sc.cvd * cvs);
 }
 
+// such a cell from load to store; evaluations, and flags from bit 28 on
 template <int NY>
 __device__ __noinline__ int sat_cell_any(const canoe_thermo_t &th, const SatConst &sc,
-                                         const canoe_satadj_opts_t &o, double *uc, double t_guess,
-                                         double &t_out, int &flags) {
-  return sat_cell<NY, ExactThermo>(th, sc, o, uc, t_guess, t_out, flags);
-}
-
-template <int NY>
-__device__ __noinline__ double mlp_features_any(const canoe_thermo_t &th, const SatConst &sc,
-                                                const double *uc, float *x) {
-  return mlp_features<NY, ExactThermo>(th, sc, uc, x);
+                                         const canoe_satadj_opts_t &o, double *u, int64_t stride,
+                                         double t_guess, double *t_out, int32_t *iters) {
+  double uc[Slots<NY>::NV], T;
+  int fl = 0;
+#pragma unroll
+  for (int n = 0; n < Slots<NY>::NV; ++n) uc[n] = u[n * stride];
+  const int it = sat_cell<NY, ExactThermo>(th, sc, o, uc, t_guess, T, fl);
+  if (!(fl & 4)) {
+#pragma unroll
+    for (int n = 1; n <= NY; ++n) u[n * stride] = uc[n];
+  }
+  if (t_out) *t_out = T;
+  if (iters) *iters = it;
+  return it | fl << 28;
 }
 
 // true when a condensable family of the cell is at or above saturation at
@@ -605,17 +611,8 @@ __device__ __forceinline__ void satadj_chunk(
     // stay unsaturated
     float x[kMlpIn] = {0.f, 0.f, 0.f, 0.f};
     if (active) {
-      if (ordinary) {
-        tdry = mlp_features<NY, canoe_thermo_t>(th, sc, uc, x);
-      } else {
-        double ua[S::NV];
-        float xa[kMlpIn];
-#pragma unroll
-        for (int n = 0; n < S::NV; ++n) ua[n] = uc[n];
-        tdry = mlp_features_any<NY>(th, sc, ua, xa);
-#pragma unroll
-        for (int n = 0; n < kMlpIn; ++n) x[n] = xa[n];
-      }
+      tdry = ordinary ? mlp_features<NY, canoe_thermo_t>(th, sc, uc, x)
+                      : mlp_features<NY, ExactThermo>(th, sc, uc, x);
       need = may_condense<NY>(th, uc, tdry);
     }
     tg = __longlong_as_double(0x7ff8000000000000LL);  // no guess: cold start
@@ -649,26 +646,21 @@ __device__ __forceinline__ void satadj_chunk(
     if (active && t_out) t_out[t] = tdry;
     if (active && iters) iters[t] = 0;
   } else if (active) {
-    double T;
     if (ordinary) {
+      double T;
       it = sat_cell<NY, canoe_thermo_t>(th, sc, o, uc, tg, T, fl);
+      if (!(fl & 4)) {
+#pragma unroll
+        for (int n = 1; n <= NY; ++n) u[n * stride + off] = uc[n];
+      }
+      if (t_out) t_out[t] = T;
+      if (iters) iters[t] = it;
     } else {
-      double ua[S::NV], Ta;
-      int fa = 0;
-#pragma unroll
-      for (int n = 0; n < S::NV; ++n) ua[n] = uc[n];
-      it = sat_cell_any<NY>(th, sc, o, ua, tg, Ta, fa);
-#pragma unroll
-      for (int n = 0; n < S::NV; ++n) uc[n] = ua[n];
-      T = Ta;
-      fl = fa;
+      const int r = sat_cell_any<NY>(th, sc, o, u + off, stride, tg, t_out ? t_out + t : nullptr,
+                                     iters ? iters + t : nullptr);
+      it = r & 0xfffffff;
+      fl = r >> 28;
     }
-    if (!(fl & 4)) {
-#pragma unroll
-      for (int n = 1; n <= NY; ++n) u[n * stride + off] = uc[n];
-    }
-    if (t_out) t_out[t] = T;
-    if (iters) iters[t] = it;
   }
   if (stats) {
     uint32_t a = active ? 1u : 0u, b = (uint32_t)it, c = (fl & 1) ? 1u : 0u,
