@@ -38,7 +38,7 @@
 // the chunk's first level, two levels more than the chunk.
 //
 // Measured against the CTA-per-column kernel (one launch, 128x256x256 moist,
-// PPM + HLLC): FP32 fluxes 2.52 -> 1.14 ms, FP64 3.05 -> 1.63 ms; with 5x5
+// PPM + HLLC): FP32 fluxes 2.52 -> 1.16 ms, FP64 3.05 -> 1.63 ms; with 5x5
 // blocks FP32 12.3 -> 3.1 ms.  What bounds it: a chunk is a chain of four
 // barrier-separated phases of dependent FP64 and FP32 arithmetic (about 10k
 // cycles for eight levels) that two CTAs per SM (shared memory) overlap: issue
