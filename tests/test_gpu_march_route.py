@@ -20,8 +20,11 @@ def _p(nx1=12, nx2=72, nx3=62, **kw):
 
 
 def _free():
+    import gc
     import torch
+    gc.collect()
     torch.cuda.synchronize()
+    torch.cuda.empty_cache()  # what earlier tests left in torch's pool
     return torch.cuda.mem_get_info()[0]
 
 
