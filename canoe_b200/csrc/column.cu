@@ -84,9 +84,10 @@ static bool march_serves(const Geom &g, const canoe_thermo_t &th, int flag, int 
   return sizeof(double) * col_smem(g.nv, g.nc1, g.nx1, n, 0, 1).total <= 227 * 1024;
 }
 
-// claims with scratch whose block has not stepped, which may be given back
+// claims with scratch whose block has not stepped, which may be given back (not
+// destroyed at exit: a host's blocks may go later than the library's statics)
 static std::mutex claim_mu;
-static std::set<MarchClaim *> claims;
+static std::set<MarchClaim *> &claims = *new std::set<MarchClaim *>;
 
 static void claim_scratch(MarchClaim &c, size_t keep_free_one_in) {
   Geom &g = *c.g;
